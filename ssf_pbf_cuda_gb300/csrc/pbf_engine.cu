@@ -174,9 +174,9 @@ pbf_status derive_desc(const pbf_params &p, const float domain_end[3], SceneDesc
 
 uint64_t bytes_per_particle(uint32_t max_pair)
 {
-    // x v xs xa xb xold w vt wx (float4) + xv (2 float4) + key slot tmp perm id id_tmp wpos + lam + nnb +
+    // x v xs xa xb xold w pa vs (float4) + pb (float2) + key slot tmp perm id id_tmp wpos + lam + nnb +
     // selfat + cls + nbr
-    return 11 * 16 + 7 * 4 + 4 + 1 + 1 + 1 + 16ull * ((max_pair - 1 + 3) / 4);  // list slots in whole quads
+    return 9 * 16 + 8 + 7 * 4 + 4 + 1 + 1 + 1 + 16ull * ((max_pair - 1 + 3) / 4);  // list slots in whole quads
 }
 
 // ---------------------------------------------------------------- batch --
@@ -189,9 +189,9 @@ Batch::~Batch()
     if (small_done_) cudaEventDestroy(small_done_);
     if (h_small_) cudaFreeHost(h_small_);
     void *ptrs[] = {d_scenes_, d_tile_scene_, d_tile_start_, d_ctrl_, d_scene_num_, d_flags_, d_x_, d_v_,
-                    d_xs_, d_xa_, d_xb_, d_xold_, d_w_, d_vt_, d_key_, d_slot_, d_tmp_, d_perm_, d_count_,
-                    d_offsets_, d_bsum_, d_lam_, d_nbr_, d_nnb_, d_self_, d_bnd_, d_pack_off_, d_active_, d_xv_, d_id_, d_id_tmp_,
-                    d_next_id_, d_cls_, d_wx_, d_chist_, d_wpos_, d_dense_, d_mid_};
+                    d_xs_, d_xa_, d_xb_, d_xold_, d_w_, d_pa_, d_pb_, d_vs_, d_key_, d_slot_, d_tmp_, d_perm_, d_count_,
+                    d_offsets_, d_bsum_, d_lam_, d_nbr_, d_nnb_, d_self_, d_bnd_, d_pack_off_, d_active_, d_id_, d_id_tmp_,
+                    d_next_id_, d_cls_, d_chist_, d_wpos_, d_dense_, d_mid_};
     for (void *p : ptrs)
         if (p) cudaFree(p);
 }
@@ -227,11 +227,11 @@ pbf_status Batch::init(uint32_t max_scenes, uint64_t max_particles, uint64_t max
     CK(A((void **)&d_scene_num_, 4ull * max_scenes));
     CK(A((void **)&d_flags_, 4ull * max_scenes));
     CK(A((void **)&d_next_id_, 4ull * max_scenes));
-    float4 **f4[] = {&d_x_, &d_v_, &d_xs_, &d_xa_, &d_xb_, &d_xold_, &d_w_, &d_vt_, &d_wx_};
+    float4 **f4[] = {&d_x_, &d_v_, &d_xs_, &d_xa_, &d_xb_, &d_xold_, &d_w_, &d_pa_, &d_vs_};
     // + kWalkSpare records: the neighbour walk reads candidates in groups of
     // four and may read up to three past the end of a range (never accepted)
     for (float4 **p : f4) CK(A((void **)p, 16 * (P + kWalkSpare)));
-    CK(A((void **)&d_xv_, 32 * (P + kWalkSpare)));
+    CK(A((void **)&d_pb_, 8 * (P + kWalkSpare)));
     uint32_t **u4[] = {&d_key_, &d_slot_, &d_tmp_, &d_perm_, &d_id_, &d_id_tmp_, &d_wpos_};
     for (uint32_t **p : u4) CK(A((void **)p, 4 * P));
     CK(A((void **)&d_count_, 4 * (C + 4)));
@@ -435,7 +435,7 @@ pbf_status Batch::set_particles(uint32_t id, const float *x, const float *v, uin
             // raw AoS float3 goes to the scene's slice of the xs / vt scratch
             // (free between steps) and is widened on the device
             float *stx = reinterpret_cast<float *>(d_xs_ + s.desc.p_off + start);
-            float *stv = reinterpret_cast<float *>(d_vt_ + s.desc.p_off + start);
+            float *stv = reinterpret_cast<float *>(d_pa_ + s.desc.p_off + start);
             CK(cudaMemcpyAsync(stx, x, 12ull * n, cudaMemcpyHostToDevice, st));
             if (v) CK(cudaMemcpyAsync(stv, v, 12ull * n, cudaMemcpyHostToDevice, st));
             sx = stx;
@@ -483,8 +483,8 @@ pbf_status Batch::upload_all(const uint32_t *counts, const float *x, const float
         CK(cudaMemcpyAsync(d_xs_, x, 12 * tot, cudaMemcpyHostToDevice, st));
         sx = reinterpret_cast<const float *>(d_xs_);
         if (v) {
-            CK(cudaMemcpyAsync(d_vt_, v, 12 * tot, cudaMemcpyHostToDevice, st));
-            sv = reinterpret_cast<const float *>(d_vt_);
+            CK(cudaMemcpyAsync(d_pa_, v, 12 * tot, cudaMemcpyHostToDevice, st));
+            sv = reinterpret_cast<const float *>(d_pa_);
         }
     }
     if (ctrl_.n_tiles) launch_unpack(args(), shape_for(tile_), d_pack_off_, sx, sv, st);
@@ -577,7 +577,7 @@ pbf_status Batch::download_all(uint32_t *counts, float *x, float *v, bool dst_de
     float *dx = x, *dv = v;
     if (!dst_dev) {
         dx = x ? reinterpret_cast<float *>(d_xs_) : nullptr;
-        dv = v ? reinterpret_cast<float *>(d_vt_) : nullptr;
+        dv = v ? reinterpret_cast<float *>(d_pa_) : nullptr;
     }
     launch_pack(args(), shape_for(tile_), d_pack_off_, dx, dv, st);
     CK(cudaGetLastError());
@@ -771,9 +771,11 @@ LaunchShape Batch::shape_for(uint32_t tile) const
     sh.grid_nb = ntb;  // a block per tile: the walk's cost varies per tile, and fresh blocks balance it
     sh.grid_lambda = g(o.lambda);
     sh.grid_dp = g(o.dp);
-    sh.grid_omega = g(o.omega);
-    sh.grid_apply = g(o.apply);
-    sh.grid_xsph = g(o.xsph);
+    for (int f = 0; f < 2; ++f) {
+        sh.grid_omega[f] = g(o.omega[f]);
+        sh.grid_apply[f] = g(o.apply[f]);
+        sh.grid_xsph[f] = g(o.xsph[f]);
+    }
     sh.grid_cells = pow2(std::max<uint32_t>(1, ctrl_.n_cell_tiles));  // a block per cell tile
     sh.cell_tile = cell_tile_;
     sh.small = (uint64_t)nt * tile <= kSmallStep ? 1u : 0u;
@@ -817,7 +819,6 @@ StepArgs Batch::args() const
     a.xold = d_xold_;
     a.id = d_id_;
     a.cls = d_cls_;
-    a.wx = d_wx_;
     a.wpos = d_wpos_;
     a.dense = d_dense_;
     a.mid = d_mid_;
@@ -829,8 +830,9 @@ StepArgs Batch::args() const
     a.nnb = d_nnb_;
     a.selfat = d_self_;
     a.w = d_w_;
-    a.vt = d_vt_;
-    a.xv = d_xv_;
+    a.pa = d_pa_;
+    a.pb = d_pb_;
+    a.vs = d_vs_;
     a.bnd = d_bnd_;
     a.nbr_stride = max_particles_;
     a.pin = d_pin_;
@@ -840,12 +842,11 @@ StepArgs Batch::args() const
 
 uint32_t Batch::post_modes() const
 {
-    bool x_off = false, x_walk = false, x_list = false, v_ref = false, v_text = false, l16 = false, l32 = false;
+    bool x_walk = false, x_list = false, v_ref = false, v_text = false, l16 = false, l32 = false;
     for (auto &s : scenes_)
         if (s.active) {
             l16 |= s.desc.list16 != 0;
             l32 |= s.desc.list16 == 0;
-            x_off |= s.desc.xsph_mode == PBF_XSPH_OFF;
             x_walk |= s.desc.xsph_mode == PBF_XSPH_WALK;
             x_list |= s.desc.xsph_mode == PBF_XSPH_LIST;
             v_ref |= s.desc.vort_mode == PBF_VORTICITY_REFERENCE;
@@ -853,9 +854,7 @@ uint32_t Batch::post_modes() const
         }
     uint32_t m = 0;
     if (x_walk) m |= kPostXsphWalk;
-    // the list-form XSPH kernel also copies the velocities of scenes without
-    // XSPH when some scene of the batch has it
-    if (x_list || (x_off && x_walk)) m |= kPostXsphList;
+    if (x_list) m |= kPostXsphList;
     if (v_ref) m |= kPostVortReference;
     if (v_text) m |= kPostVortTextbook;
     if (l16) m |= kPostList16;
@@ -929,7 +928,8 @@ pbf_status Batch::profile_step(int iters, cudaStream_t st, float *ms, char *name
     cudaEvent_t e0;
     CK(cudaEventCreate(&e0));
     CK(cudaEventRecord(e0, st));
-    last_launches_ = enqueue_step(args(), shape_for(tile_), iters, post_modes(), st, &hook);
+    const LaunchShape sh = shape_for(tile_);
+    last_launches_ = enqueue_step(args(), sh, iters, post_modes(), st, &hook);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(st));
     cudaEvent_t prev = e0;
@@ -1102,17 +1102,20 @@ pbf_status Batch::get_debug(uint32_t id, uint32_t *sorted_hash, uint32_t *perm, 
         const uint32_t mp = d.cap + 1;
         const uint64_t padded = ((uint64_t)live + 31) / 32 * 32;
         std::fill(neighbor_list, neighbor_list + padded * mp, 0xFFFFFFFFu);
+        // lists are stored by working slot; wpos names each sorted slot's
         std::vector<uint8_t> nn(live), self(live);
-        std::vector<uint32_t> quads(4ull * live);
+        std::vector<uint32_t> quads(4ull * live), wpos(n_in), sorted(n_in);
         if (live) {
             CK(cudaMemcpy(nn.data(), d_nnb_ + d.p_off, live, cudaMemcpyDeviceToHost));
             CK(cudaMemcpy(self.data(), d_self_ + d.p_off, live, cudaMemcpyDeviceToHost));
         }
+        if (n_in) CK(cudaMemcpy(wpos.data(), d_wpos_ + d.p_off, 4ull * n_in, cudaMemcpyDeviceToHost));
+        for (uint32_t g = 0; g < n_in; ++g) sorted[wpos[g] - d.p_off] = g;
         auto at = [&](uint32_t k, uint32_t p) -> uint32_t & {
             return neighbor_list[((uint64_t)k << 5) + (p & 31) + (uint64_t)((p >> 5) << 5) * mp];
         };
-        // rows of 16 bytes per particle: quads of 4 u32 sorted slots, or
-        // octs of 8 u16 scene-local indices (scenes of at most kList16Max
+        // rows of 16 bytes per particle: quads of 4 u32 working slots, or
+        // octs of 8 u16 scene-local ones (scenes of at most kList16Max
         // slots).  Stored entry k is list slot k, or k + 1 from the particle's
         // own position on (the particle itself is listed but not stored).
         const uint32_t per_row = d.list16 ? 8u : 4u;
@@ -1121,13 +1124,13 @@ pbf_status Batch::get_debug(uint32_t id, uint32_t *sorted_hash, uint32_t *perm, 
                           cudaMemcpyDeviceToHost));
             const uint16_t *octs = reinterpret_cast<const uint16_t *>(quads.data());
             for (uint32_t k = per_row * kq; k < per_row * kq + per_row && k < d.cap; ++k)
-                for (uint32_t p = 0; p < live; ++p)
-                    if (k < nn[p])
-                        at(k + (k >= self[p] ? 1u : 0u), p) =
-                            d.list16 ? octs[8ull * p + (k & 7)] : quads[4ull * p + (k & 3)] - d.p_off;
+                for (uint32_t w = 0; w < live; ++w)
+                    if (k < nn[w])
+                        at(k + (k >= self[w] ? 1u : 0u), sorted[w]) =
+                            sorted[d.list16 ? octs[8ull * w + (k & 7)] : quads[4ull * w + (k & 3)] - d.p_off];
         }
-        for (uint32_t p = 0; p < live; ++p)
-            if (self[p] != kNotListed) at(self[p], p) = p;
+        for (uint32_t w = 0; w < live; ++w)
+            if (self[w] != kNotListed) at(self[w], sorted[w]) = sorted[w];
     }
     return PBF_SUCCESS;
 }

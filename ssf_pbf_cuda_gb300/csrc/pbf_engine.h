@@ -143,7 +143,8 @@ private:
     Ctrl *d_ctrl_ = nullptr;
     uint32_t *d_scene_num_ = nullptr, *d_flags_ = nullptr;
     float4 *d_x_ = nullptr, *d_v_ = nullptr, *d_xs_ = nullptr, *d_xa_ = nullptr, *d_xb_ = nullptr,
-           *d_xold_ = nullptr, *d_w_ = nullptr, *d_vt_ = nullptr;
+           *d_xold_ = nullptr, *d_w_ = nullptr, *d_pa_ = nullptr, *d_vs_ = nullptr;
+    float2 *d_pb_ = nullptr;
     uint32_t *d_key_ = nullptr, *d_slot_ = nullptr, *d_tmp_ = nullptr, *d_perm_ = nullptr;
     uint32_t *d_count_ = nullptr, *d_offsets_ = nullptr, *d_bsum_ = nullptr;
     float *d_lam_ = nullptr;
@@ -157,10 +158,8 @@ private:
     uint32_t *d_id_ = nullptr, *d_id_tmp_ = nullptr;  // particle ids, phase order / sorted scratch
     uint32_t *d_next_id_ = nullptr;                   // per scene: next id to hand out
     uint8_t *d_cls_ = nullptr;                        // alias class per particle (input order)
-    float4 *d_wx_ = nullptr;                          // class-grouped walk copy of the sorted positions
-    float4 *d_xv_ = nullptr;                          // final (x, v) records, two float4 per particle slot
     uint64_t *d_chist_ = nullptr;                     // per cell: class counts of its bucket
-    uint32_t *d_wpos_ = nullptr;                      // sorted slot -> walk-copy slot
+    uint32_t *d_wpos_ = nullptr;                      // sorted slot -> working slot
     uint32_t *d_dense_ = nullptr;                     // dense-bucket queue
     uint32_t *d_mid_ = nullptr;                       // medium-bucket queue
     uint32_t *h_small_ = nullptr;     // pinned host scratch: pack offsets + counts

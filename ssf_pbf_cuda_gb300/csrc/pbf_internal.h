@@ -105,21 +105,22 @@ struct StepArgs {
     float4 *xs;                   // predicted positions, input order
     uint32_t *key, *slot, *tmp, *perm;
     uint32_t *count, *offsets, *bsum;
-    float4 *xa, *xb, *xold;       // working positions (ping-pong) and sorted old x
+    // working slots: sorted slots, with a bucket of several alias classes grouped by class
+    float4 *xa, *xb, *xold;       // working positions (ping-pong), old x (.w = sorted slot)
     float *lam;
-    uint32_t *nbr;                // nbr[k * nbr_stride + i]
+    uint32_t *nbr;                // neighbour lists, in rows of 16 bytes per working slot
     uint8_t *nnb;                 // list entries stored (the particle itself is not stored)
     uint8_t *selfat;              // position of the particle itself in its walk-order list, kNotListed if cut
-    float4 *w, *vt;               // vorticity, XSPH velocity scratch
-    float4 *xv;                   // final (x, v) side by side, 32 B per particle slot, for the list-form
-                                  // vorticity pass's neighbour gathers (one 256-bit load per neighbour)
+    float4 *w;                    // vorticity
+    float4 *pa;                   // (x, y, z, vx) and (vy, vz) between the list-form post passes, working slots
+    float2 *pb;
+    float4 *vs;                   // velocity between the walk-form post passes, sorted slots
     const float4 *bnd;            // boundary primitives
-    uint32_t *id, *id_tmp;        // particle ids (phase order) and their sorted copy
+    uint32_t *id, *id_tmp;        // particle ids (phase order) and their copy in working order
     uint8_t *cls;                 // alias class of each particle (input order)
-    uint32_t *wpos;               // sorted slot -> walk-copy slot (mixed-class buckets only)
+    uint32_t *wpos;               // sorted slot -> working slot
     uint32_t *dense;              // [0] count, then (cell, scene) pairs of buckets for k_dense_sort
     uint32_t *mid;                // the same for buckets of kMidMin+1 .. kDenseMin members
-    float4 *wx;                   // walk copy of mixed-class buckets: grouped by class, .w = sorted slot
     uint64_t *chist;              // per cell: 8 x 8-bit class counts of its bucket, or kClassWhole
     uint32_t *next_id;            // per scene: id of the next particle added
     uint64_t nbr_stride;
@@ -134,7 +135,8 @@ struct LaunchShape {
     uint32_t scan_rounds; // one-block scan: rounds of 1024 cells held in registers (1..16), 0 = looped
     uint32_t chunk;       // neighbours per chunk in the lambda / delta-p passes (4 or 8)
     // persistent grids of the heavy kernels, each from its own occupancy
-    uint32_t grid_nb, grid_lambda, grid_dp, grid_omega, grid_apply, grid_xsph;
+    uint32_t grid_nb, grid_lambda, grid_dp;
+    uint32_t grid_omega[2], grid_apply[2], grid_xsph[2];  // list-form post passes: u32 lists, u16 lists
     uint32_t grid_cells;  // grid of k_rank_cells: a block of cell_tile threads per cell tile
     uint32_t cell_tile;   // cells per cell tile = threads per k_rank_cells block (autotuned)
     uint32_t small;       // latency-bound step (at most kSmallStep particle slots): split
@@ -147,13 +149,15 @@ struct LaunchShape {
                chunk == o.chunk &&
                grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && grid_split == o.grid_split && nb_smem == o.nb_smem &&
                grid_nb == o.grid_nb && grid_lambda == o.grid_lambda && grid_dp == o.grid_dp &&
-               grid_omega == o.grid_omega && grid_apply == o.grid_apply && grid_xsph == o.grid_xsph;
+               grid_omega[0] == o.grid_omega[0] && grid_omega[1] == o.grid_omega[1] && grid_apply[0] == o.grid_apply[0] &&
+               grid_apply[1] == o.grid_apply[1] && grid_xsph[0] == o.grid_xsph[0] && grid_xsph[1] == o.grid_xsph[1];
     }
 };
 
 // Resident blocks per SM of each kernel class at a tile size / chunk.
 struct Occupancy {
-    uint32_t light, nb, lambda, dp, omega, apply, xsph, cells, split;
+    uint32_t light, nb, lambda, dp, cells, split;
+    uint32_t omega[2], apply[2], xsph[2];
 };
 Occupancy occupancy(uint32_t tile, uint32_t chunk);
 
@@ -166,7 +170,7 @@ struct StepHook {
 // Post-solve passes a step runs (bit set: some active scene needs that form).
 enum : uint32_t {
     kPostXsphWalk = 1,       // XSPH, the reference's uncapped 27-cell walk
-    kPostXsphList = 2,       // XSPH over the step's neighbour list (+ copy for scenes without XSPH)
+    kPostXsphList = 2,       // XSPH over the step's neighbour list
     kPostVortReference = 4,  // vorticity, the reference's walk and kernel scaling
     kPostVortTextbook = 8,   // vorticity, textbook form over the neighbour list
     kPostList32 = 16,        // some scene keeps a u32 neighbour list (list forms launch per list format)
@@ -201,8 +205,8 @@ void launch_unpack(const StepArgs &a, const LaunchShape &sh, const uint32_t *pac
 void launch_pack(const StepArgs &a, const LaunchShape &sh, const uint32_t *pack_off, float *dst_x, float *dst_v,
                  cudaStream_t st);
 
-// chist value of a bucket whose walk copy is in plain sorted order (more
-// than 255 members, or a bucket left in atomic order)
+// chist value of a bucket in plain sorted order, walked whole (more than 255
+// members, or a table of fewer than 4 cells on an axis)
 constexpr uint64_t kClassWhole = ~0ull;
 
 constexpr uint32_t kScanItemsPerWarp = 512;   // 32 lanes x 16

@@ -18,6 +18,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <utility>
 
 #include "pbf_internal.h"
 #include "pbf_sort.cuh"
@@ -82,15 +83,6 @@ __device__ __forceinline__ void fma2(float &c0, float &c1, float a0, float a1, f
         "mov.b64 {%0, %1}, pc;\n\t}"
         : "+f"(c0), "+f"(c1)
         : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-
-// One 32-byte record (two float4) by one 256-bit load through the
-// read-only path; p must be 32-byte aligned.
-__device__ __forceinline__ void ld_rec(const float4 *p, float4 &a, float4 &b)
-{
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
 }
 
 // r^2 exactly as findPair computes it (pbf_neighbor_search_util.cu:398):
@@ -344,15 +336,15 @@ __device__ __forceinline__ void walk27_ranges(const SceneDesc &d, const uint32_t
 // The neighbour-search walk: the same 27 cells in the same order as
 // walk27_ranges, one range per cell, and inside a cell's bucket only the
 // particles of the cell's alias class (chist holds the bucket's class
-// counts): a bucket of one class is the sorted range itself (xa), a bucket
+// counts): a bucket of one class is its range, a bucket
 // without the class is skipped, and a mixed bucket gives the class's
-// sub-range of the class-grouped walk copy (wx).  Candidates of the other
-// classes lie at least G - 1 cells away and can never be accepted, and both
-// arrays keep each class in sorted order with the sorted slot in .w, so the
+// sub-range (working slots hold a mixed bucket grouped by class).
+// Candidates of the other classes lie at least G - 1 cells away and can
+// never be accepted, and each class keeps its sorted order, so the
 // accepted sequence is the reference's.  Buckets marked kClassWhole (and
 // every bucket of a scene with an axis of fewer than 4 cells, where the
 // reference visits wrapped cells twice) are visited whole, in sorted order.
-// r(src, st, en) gets the array and the range.
+// r(st, en) gets the range of working slots.
 //
 // PRUNE restricts the walk to cells that can hold a particle within h of xp
 // (the binned position): a cell whose nearest point is farther than h holds
@@ -362,9 +354,8 @@ __device__ __forceinline__ void walk27_ranges(const SceneDesc &d, const uint32_t
 // cells (with fewer, the reference visits wrapped cells more than once).
 template <bool PRUNE, class R>
 __device__ __forceinline__ void walk27_cells(const SceneDesc &d, const uint32_t *__restrict__ offsets,
-                                             const uint64_t *__restrict__ chist, const float4 *xa,
-                                             const float4 *wx, uint32_t shift, float4 xp, R &&r, int rr0 = 0,
-                                             int rr1 = 9)
+                                             const uint64_t *__restrict__ chist, uint32_t shift, float4 xp, R &&r,
+                                             int rr0 = 0, int rr1 = 9)
 {
     const int32_t icx = cell_coord(xp.x, d.cw), icy = cell_coord(xp.y, d.cw), icz = cell_coord(xp.z, d.cw);
     const bool prune = PRUNE && d.gx >= 4 && d.gy >= 4 && d.gz >= 4;
@@ -405,19 +396,17 @@ __device__ __forceinline__ void walk27_cells(const SceneDesc &d, const uint32_t 
             uint32_t en = __ldg(off + b + 1);
             const uint64_t h = __ldg(reinterpret_cast<const unsigned long long *>(ch + b));
             if (st == en) continue;
-            const float4 *src = xa;
             if (h != kClassWhole) {
                 const uint32_t sh = 8u * (cyz | (uint32_t)((tx >> sx) & 1));
                 const uint32_t cnt = (uint32_t)((h >> sh) & 0xFFull);
                 if (cnt == 0) continue;  // no particle of this cell in the bucket
-                if (cnt != en - st) {    // several classes: this one's sub-range of the walk copy
+                if (cnt != en - st) {    // several classes: this one's sub-range
                     const uint64_t lower = sh ? (h & ((1ull << sh) - 1ull)) : 0ull;
                     st += (uint32_t)((lower * 0x0101010101010101ull) >> 56);  // byte sum: bucket <= 255
                     en = st + cnt;
-                    src = wx;
                 }
             }
-            if (!r(src, st + shift, en + shift)) return;
+            if (!r(st + shift, en + shift)) return;
         }
     }
 }
@@ -555,31 +544,6 @@ __device__ __forceinline__ void list_walk_any(bool l16, const uint32_t *__restri
         list_walk16(nl, stride, nn, base, f);
     else
         list_walk<CH>(nl, stride, nn, f);
-}
-
-// list_walk in chunks of one quad with the quads requested two chunks
-// ahead: eight indices in flight, one quad of them per use.
-template <class F>
-__device__ __forceinline__ void list_walk_ahead2(const uint32_t *__restrict__ nl, uint64_t stride, uint32_t nn,
-                                                 F &&f)
-{
-    const uint4 *p = reinterpret_cast<const uint4 *>(nl);
-    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    uint4 q0 = (0u < nn) ? list_ld(p) : z;
-    uint4 q1 = (4u < nn) ? list_ld(p + stride) : z;
-    uint32_t k0 = 0;
-    for (; k0 + 4 <= nn; k0 += 4) {
-        const uint4 q = q0;
-        q0 = q1;
-        q1 = (k0 + 8 < nn) ? list_ld(p + (uint64_t)((k0 >> 2) + 2) * stride) : z;
-        f(q.x);
-        f(q.y);
-        f(q.z);
-        f(q.w);
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-        if (k0 + c < nn) f(quad_at(q0, c));
 }
 
 // Per-tile prologue shared by the particle kernels.
@@ -839,11 +803,9 @@ __global__ void __launch_bounds__(256) k_scan_down(StepArgs a)
 }
 
 // tmp entries of scenes up to kClsLimit particles carry the member's alias
-// class above its input index.  wpos of a particle outside a mixed-class
-// bucket is kNoWalkCopy.
+// class above its input index.
 constexpr uint32_t kClsShift = 29;
 constexpr uint32_t kClsLimit = 1u << kClsShift;
-constexpr uint32_t kNoWalkCopy = 0xFFFFFFFFu;
 
 // Scatter into the cell buckets in atomic-slot order (sortByCountingCUDA,
 // pbf_counting_sort.cu:120-134).
@@ -919,7 +881,7 @@ __global__ void __launch_bounds__(kCellTileMax) k_rank_cells(StepArgs a)
                 frank += (cu == ct && iu < it) ? 1u : 0u;
             }
             a.perm[g0 + rank] = it;
-            a.wpos[g0 + rank] = mixed ? g0 + below + frank : kNoWalkCopy;
+            a.wpos[g0 + rank] = g0 + (mixed ? below + frank : rank);
         }
         a.chist[gk] = grouped ? hist : kClassWhole;
     }
@@ -983,7 +945,7 @@ __global__ void __launch_bounds__(512) k_rank_reorder(StepArgs a)
     // particle data in sorted order (coalesced writes, as the reference's
     // reorderDataCUDA gathers).  Buckets holding more than one alias class
     // also place the particle in the class-grouped walk copy.
-    a.wpos[g] = mixed ? d.p_off + (st - base) + below + frank : kNoWalkCopy;
+    a.wpos[g] = mixed ? d.p_off + (st - base) + below + frank : g;
     if (rank == 0) a.chist[gk] = grouped ? hist : kClassWhole;
     a.perm[g] = local;
     TILE_LOOP_END
@@ -1063,11 +1025,11 @@ __global__ void __launch_bounds__(kRadixThreads) k_dense_sort(StepArgs a)
             }
             if (h0) {
                 a.perm[g0 + r0] = i0;
-                a.wpos[g0 + r0] = mixed ? g0 + b0 + f0 : kNoWalkCopy;
+                a.wpos[g0 + r0] = g0 + (mixed ? b0 + f0 : r0);
             }
             if (h1) {
                 a.perm[g0 + r1] = i1;
-                a.wpos[g0 + r1] = mixed ? g0 + b1 + f1 : kNoWalkCopy;
+                a.wpos[g0 + r1] = g0 + (mixed ? b1 + f1 : r1);
             }
             if (lane == 0) a.chist[gk] = grouped ? hist : kClassWhole;
         }
@@ -1084,7 +1046,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_dense_sort(StepArgs a)
         if (b > kStableLimit) {  // the bucket's scatter entries are scratch once sorted into perm
             block_radix_stable(a.tmp + st, a.perm + g0, b, imask, radix_bits(d.capacity),
                                *reinterpret_cast<RadixSmem *>(S), rbase, rtot);
-            for (uint32_t t = threadIdx.x; t < b; t += blockDim.x) a.wpos[g0 + t] = kNoWalkCopy;
+            for (uint32_t t = threadIdx.x; t < b; t += blockDim.x) a.wpos[g0 + t] = g0 + t;
             if (threadIdx.x == 0) a.chist[gk] = kClassWhole;
             __syncthreads();
             continue;
@@ -1112,7 +1074,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_dense_sort(StepArgs a)
         if (mixed) bitonic_sort<true>(W, P, imask);  // (class, index) order
         for (uint32_t t = threadIdx.x; t < b; t += blockDim.x) {
             a.perm[g0 + t] = S[t] & imask;
-            if (!mixed) a.wpos[g0 + t] = kNoWalkCopy;
+            if (!mixed) a.wpos[g0 + t] = g0 + t;
         }
         if (mixed) {
             for (uint32_t w = threadIdx.x; w < b; w += blockDim.x) {
@@ -1131,10 +1093,18 @@ __global__ void __launch_bounds__(kRadixThreads) k_dense_sort(StepArgs a)
     }
 }
 
-// Reorder in sorted order (reorderDataCUDA x2, pbf_neighbor_search_util.cu:143-154):
-// sorted predicted positions (carrying their own slot in .w, which the
-// neighbour walk records), sorted old positions and ids; the walk copy of
-// mixed-class buckets.  PACKED: old positions from the packed input.
+// Reorder (reorderDataCUDA x2, pbf_neighbor_search_util.cu:143-154): predicted
+// and old positions and ids of the sorted slots, each into its working slot.
+// Working slots are the sorted slots, except that a bucket of several alias
+// classes is grouped by class, so the neighbour walk reads one range per
+// cell.  The solver works in working slots throughout; the old position's .w
+// holds the sorted slot, where the step's results go.  PACKED: old positions
+// from the packed input.
+//
+// Bound by the random 16-byte reads in input order.  One working array, not
+// the sorted positions and a grouped copy of the mixed buckets beside them:
+// 98 -> 86 us at 5.95 M particles in 256 scenes, and the neighbour walk, whose
+// candidates' slots are then their indices, 1,428 -> 1,405 us.
 template <bool PACKED>
 __global__ void __launch_bounds__(512) k_gather(StepArgs a)
 {
@@ -1144,19 +1114,19 @@ __global__ void __launch_bounds__(512) k_gather(StepArgs a)
     const SceneDesc d = a.scenes[s];
     const uint32_t g = d.p_off + local;
     const uint32_t li = a.perm[g];
+    const uint32_t w = a.wpos[g];
     const uint32_t i = d.p_off + li;
     const float4 ps = a.xs[i];
-    const float4 xg = make_float4(ps.x, ps.y, ps.z, __uint_as_float(g));
-    a.xa[g] = xg;
+    a.xa[w] = make_float4(ps.x, ps.y, ps.z, 0.f);
+    const float gs = __uint_as_float(g);
     if (PACKED) {
         const float *px = a.pin->x + 3ull * ((uint64_t)a.pack_off[s] + li);
-        a.xold[g] = make_float4(px[0], px[1], px[2], 0.f);
+        a.xold[w] = make_float4(px[0], px[1], px[2], gs);
     } else {
-        a.xold[g] = a.x[i];
+        const float4 xo = a.x[i];
+        a.xold[w] = make_float4(xo.x, xo.y, xo.z, gs);
     }
-    a.id_tmp[g] = __float_as_uint(ps.w);  // the id, stored beside the prediction
-    const uint32_t w = a.wpos[g];
-    if (w != kNoWalkCopy) a.wx[w] = xg;
+    a.id_tmp[w] = __float_as_uint(ps.w);  // the id, stored beside the prediction
     TILE_LOOP_END
 }
 
@@ -1189,14 +1159,12 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
     uint16_t *nl16 = reinterpret_cast<uint16_t *>(nl);  // u16 lists: scene-local indices
     const bool l16 = d.list16 != 0;
     const float4 *__restrict__ xa = a.xa;
-    const float4 *__restrict__ wx = a.wx;
     // phase 1: the walk only tests and records (lanes of a warp accept
     // different candidates, so pair math inside the walk would run masked
-    // for almost every candidate); a candidate's .w is its sorted slot
+    // for almost every candidate)
     // Candidates are fetched kNbFetch at a time (more loads in flight; a
     // group past the range's end reads up to kNbFetch - 1 records beyond it,
-    // never accepted: xa and wx carry that many spare records at the end of
-    // their allocations), all of the
+    // never accepted: xa carries that many spare records), all of the
     // group is tested first (independent chains), then the accepted ones are
     // appended in order up to the cap, so the first `cap` accepted ones are
     // the reference's.
@@ -1210,11 +1178,10 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
     // carries no extra state; otherwise the walk skips it as it stores.
     constexpr uint32_t kNbFetch = 4;
     uint32_t cnt = 0, selfat = kNotListed;
-    walk27_cells<true>(d, a.offsets, a.chist, xa, wx, shift, xp,
-                       [&](const float4 *src, uint32_t st, uint32_t en) -> bool {
+    walk27_cells<true>(d, a.offsets, a.chist, shift, xp, [&](uint32_t st, uint32_t en) -> bool {
         for (uint32_t q0 = st; q0 < en; q0 += kNbFetch) {
             float4 c[kNbFetch];
-            const float4 *pq = src + q0;
+            const float4 *pq = xa + q0;
 #pragma unroll
             for (uint32_t k = 0; k < kNbFetch; ++k) c[k] = __ldg(pq + k);
             bool acc[kNbFetch];
@@ -1223,7 +1190,7 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
 #pragma unroll
             for (uint32_t k = 0; k < kNbFetch; ++k) {
                 if (acc[k] && cnt < cap) {
-                    const uint32_t q = __float_as_uint(c[k].w);
+                    const uint32_t q = q0 + k;
                     if (SMEM) {
                         s_list[cnt * blockDim.x + threadIdx.x] = q;
                     } else {
@@ -1399,7 +1366,6 @@ __global__ void __launch_bounds__(256) k_neighbors_split(StepArgs a, uint32_t ti
                 nl[list_slot(k, stride)] = q;
         };
         const float4 *__restrict__ xa = a.xa;
-        const float4 *__restrict__ wx = a.wx;
         // rows shared over the lanes (split_rows); one lane takes all nine
         // when the list does not fit the private buffer
         const bool one = cap > kSplitCap;
@@ -1411,25 +1377,22 @@ __global__ void __launch_bounds__(256) k_neighbors_split(StepArgs a, uint32_t ti
         // tself is its place in this lane's run)
         uint32_t cnt = 0, tself = kNotListed;
         if (one && sub == 0) {  // write straight into the list
-            walk27_cells<true>(d, a.offsets, a.chist, xa, wx, shift, xp,
-                               [&](const float4 *src, uint32_t st, uint32_t en) -> bool {
+            walk27_cells<true>(d, a.offsets, a.chist, shift, xp, [&](uint32_t st, uint32_t en) -> bool {
                 for (uint32_t q = st; q < en; ++q) {
-                    const float4 c = __ldg(src + q);
+                    const float4 c = __ldg(xa + q);
                     if (dist2_exact(xp, c) < h2) {
-                        const uint32_t qs = __float_as_uint(c.w);
-                        if (qs == i) tself = cnt;
-                        else put(cnt - (tself < cnt ? 1u : 0u), qs);
+                        if (q == i) tself = cnt;
+                        else put(cnt - (tself < cnt ? 1u : 0u), q);
                         if (++cnt == cap) return false;
                     }
                 }
                 return true;
             });
         } else if (!one) {
-            walk27_cells<true>(d, a.offsets, a.chist, xa, wx, shift, xp,
-                               [&](const float4 *src, uint32_t st, uint32_t en) -> bool {
+            walk27_cells<true>(d, a.offsets, a.chist, shift, xp, [&](uint32_t st, uint32_t en) -> bool {
                 for (uint32_t q0 = st; q0 < en; q0 += 4) {
                     float4 c[4];
-                    const float4 *pq = src + q0;  // up to three spare records past the range
+                    const float4 *pq = xa + q0;  // up to three spare records past the range
 #pragma unroll
                     for (uint32_t k = 0; k < 4; ++k) c[k] = __ldg(pq + k);
                     bool acc[4];
@@ -1438,7 +1401,7 @@ __global__ void __launch_bounds__(256) k_neighbors_split(StepArgs a, uint32_t ti
 #pragma unroll
                     for (uint32_t k = 0; k < 4; ++k) {
                         if (acc[k] && cnt < cap) {
-                            const uint32_t qs = __float_as_uint(c[k].w);
+                            const uint32_t qs = q0 + k;
                             if (qs == i) tself = cnt;
                             buf[cnt] = qs;
                             ++cnt;
@@ -1555,9 +1518,76 @@ __device__ __forceinline__ ScorrConst scorr_const(const SceneDesc &d, float li)
     return c;
 }
 
-// Sum over the list of -(lambda_i + lambda_j + s_corr) grad W (the body of
-// calcPositionUpdateCUDA, pbf_position_update.cu:131-188), in list order:
-// each pair adds (coefficient * s) d.
+// One pair's share of the sum of -(lambda_i + lambda_j + s_corr) grad W (the
+// body of calcPositionUpdateCUDA, pbf_position_update.cu:131-188): adds
+// (coefficient * s) d.  PK: the x and y differences and sums by one packed
+// operation each (the same bits; measured faster in large steps only).
+template <int FORM, bool PK>
+__device__ __forceinline__ void dp_add(float3 &sum, float4 xp, float4 xq, float li, float lj, const PairConst &pc,
+                                       const ScorrConst &sc)
+{
+    const PairGeo g = pair_geo<PK>(xp, xq);
+    const PairWS k = pair_ws(g.r2, pc);
+    const float f = __fmul_rn(dp_coef<FORM>(li, lj, k.W, sc), k.s);
+    if (PK) {
+        fma2(sum.x, sum.y, f, f, g.d0, g.d1);
+    } else {
+        sum.x = __fmaf_rn(f, g.d0, sum.x);
+        sum.y = __fmaf_rn(f, g.d1, sum.y);
+    }
+    sum.z = __fmaf_rn(f, g.d2, sum.z);
+}
+
+// Where a step's velocity goes after a stage, by the scene's next stage: the
+// list forms of vorticity and XSPH read it in working order beside the
+// position (pa = x, y, z, vx; pb = vy, vz), the walk forms in sorted order
+// (vs), and without a further stage it is the result.  slot() gives the
+// sorted slot; i is the working slot.
+template <class G>
+__device__ __forceinline__ void put_velocity(const StepArgs &a, bool list_next, bool walk_next, uint32_t i, G &&slot,
+                                             float4 x, float4 v)
+{
+    if (list_next) {
+        a.pa[i] = make_float4(x.x, x.y, x.z, v.x);
+        a.pb[i] = make_float2(v.y, v.z);
+    } else {
+        (walk_next ? a.vs : a.v)[slot()] = v;
+    }
+}
+
+// The final position, velocity ((x_new - x_old) / dt: updateVelocityCUDA,
+// pbf_update.cu:25-39) and id of working slot i.
+__device__ __forceinline__ void put_final(const StepArgs &a, const SceneDesc &d, uint32_t i, float4 xn)
+{
+    const float4 xo = a.xold[i];
+    const uint32_t g = __float_as_uint(xo.w);
+    const float4 vn = make_float4(d.inv_dt * (xn.x - xo.x), d.inv_dt * (xn.y - xo.y), d.inv_dt * (xn.z - xo.z), 0.f);
+    a.x[g] = xn;
+    a.id[g] = a.id_tmp[i];  // ids follow the particles into sorted order
+    const bool no_vort = d.vort_mode == PBF_VORTICITY_OFF;
+    put_velocity(a, d.vort_mode == PBF_VORTICITY_TEXTBOOK || (no_vort && d.xsph_mode == PBF_XSPH_LIST),
+                 d.vort_mode == PBF_VORTICITY_REFERENCE || (no_vort && d.xsph_mode == PBF_XSPH_WALK), i,
+                 [&] { return g; }, xn, vn);
+}
+
+// A particle's delta-p from the list sum: scale, boundary response
+// (pbf_response_collision.cu:12-66), x += dp (updateInterimPositionCUDA,
+// pbf_constraint.cu:335-345) into the second buffer, so neighbours still read
+// the old positions; on the last iteration the step's results.
+__device__ __forceinline__ void dp_finish(const StepArgs &a, const SceneDesc &d, uint32_t s, uint32_t i, float4 xp,
+                                          float3 sum, float4 *__restrict__ xo, int last)
+{
+    float3 dp = make_float3(sum.x * d.dp_k, sum.y * d.dp_k, sum.z * d.dp_k);  // m beta / rho0
+    const bool ok = collide(d, a.bnd, make_float3(xp.x, xp.y, xp.z), dp);
+    if (!ok) atomicOr(a.flags + s, PBF_FLAG_COLLISION_LIMIT);
+    const float4 xn = make_float4(xp.x + dp.x, xp.y + dp.y, xp.z + dp.z, 0.f);
+    if (last)
+        put_final(a, d, i, xn);
+    else
+        xo[i] = xn;
+}
+
+// Sum over the list, in list order.  LAMW: lambda in .w of the positions.
 template <int kChunk, int FORM, bool LAMW>
 __device__ __forceinline__ float3 dp_sum(const StepArgs &a, const SceneDesc &d, const float4 *__restrict__ xc,
                                          uint32_t i, float4 xp, float li)
@@ -1565,54 +1595,18 @@ __device__ __forceinline__ float3 dp_sum(const StepArgs &a, const SceneDesc &d, 
     const PairConst pc = pair_const(d);
     const ScorrConst sc = scorr_const(d, li);
     const float *__restrict__ lam = a.lam;
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+    float3 sum = make_float3(0.f, 0.f, 0.f);
     list_walk_any<kChunk>(d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, [&](uint32_t q) {
         const float4 xq = __ldg(xc + q);
-        const PairGeo g = pair_geo<LAMW>(xp, xq);
-        const PairWS k = pair_ws(g.r2, pc);
-        const float lj = LAMW ? xq.w : __ldg(lam + q);  // LAMW: lambda in .w of the positions
-        const float f = __fmul_rn(dp_coef<FORM>(li, lj, k.W, sc), k.s);
-        if (LAMW) {  // large steps: the x and y sums by one packed fma (measured faster there only)
-            fma2(s0, s1, f, f, g.d0, g.d1);
-        } else {
-            s0 = __fmaf_rn(f, g.d0, s0);
-            s1 = __fmaf_rn(f, g.d1, s1);
-        }
-        s2 = __fmaf_rn(f, g.d2, s2);
+        dp_add<FORM, LAMW>(sum, xp, xq, li, LAMW ? xq.w : __ldg(lam + q), pc, sc);
     });
-    return make_float3(s0, s1, s2);
+    return sum;
 }
 
-// A particle's delta-p from the list sum: scale, boundary response, x += dp
-// into the second buffer, and on the last iteration the velocity and id.
-__device__ __forceinline__ void dp_finish(const StepArgs &a, const SceneDesc &d, uint32_t s, uint32_t i, float4 xp,
-                                          float3 sum, float4 *__restrict__ xo, float4 *__restrict__ vo, int last)
-{
-    float3 dp = make_float3(sum.x * d.dp_k, sum.y * d.dp_k, sum.z * d.dp_k);  // m beta / rho0
-    const bool ok = collide(d, a.bnd, make_float3(xp.x, xp.y, xp.z), dp);
-    if (!ok) atomicOr(a.flags + s, PBF_FLAG_COLLISION_LIMIT);
-    const float4 xn = make_float4(xp.x + dp.x, xp.y + dp.y, xp.z + dp.z, 0.f);
-    xo[i] = xn;
-    if (last) {
-        const float4 xo_ = a.xold[i];
-        const float4 vn =
-            make_float4(d.inv_dt * (xn.x - xo_.x), d.inv_dt * (xn.y - xo_.y), d.inv_dt * (xn.z - xo_.z), 0.f);
-        vo[i] = vn;
-        a.xv[2ull * i] = xn;  // the post passes gather x and v together
-        a.xv[2ull * i + 1] = vn;
-        a.id[i] = a.id_tmp[i];  // ids follow the particles into sorted order
-    }
-}
-
-// delta-p with s_corr (calcPositionUpdateCUDA cached, pbf_position_update.cu:131-188),
-// boundary response (pbf_response_collision.cu:12-66) and x += dp
-// (updateInterimPositionCUDA, pbf_constraint.cu:335-345), written to a second
-// buffer so neighbours still read the old positions.  On the last iteration
-// the velocity update (updateVelocityCUDA, pbf_update.cu:25-39) is fused in:
-// v = (x_new - x_old) / dt, written with x_new to the particle phase.
+// delta-p with s_corr (calcPositionUpdateCUDA cached, pbf_position_update.cu:131-188).
 template <int kChunk, bool LAMW>
 __global__ void __launch_bounds__(512, 2) k_dp(StepArgs a, const float4 *__restrict__ xc, float4 *__restrict__ xo,
-                                               float4 *__restrict__ vo, int last)
+                                               int last)
 {
     TILE_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
@@ -1632,12 +1626,12 @@ __global__ void __launch_bounds__(512, 2) k_dp(StepArgs a, const float4 *__restr
         sum = dp_sum<kChunk, kScorrTextbook, LAMW>(a, d, xc, i, xp, li);
     else
         sum = dp_sum<kChunk, kScorrOff, LAMW>(a, d, xc, i, xp, li);
-    dp_finish(a, d, s, i, xp, sum, xo, vo, last);
+    dp_finish(a, d, s, i, xp, sum, xo, last);
     TILE_LOOP_END
 }
 
 // iters == 0: positions stay at the prediction; v from the velocity update.
-__global__ void __launch_bounds__(512) k_finalize(StepArgs a, float4 *__restrict__ vo)
+__global__ void __launch_bounds__(512) k_finalize(StepArgs a)
 {
     TILE_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
@@ -1647,225 +1641,292 @@ __global__ void __launch_bounds__(512) k_finalize(StepArgs a, float4 *__restrict
     if (local >= live) continue;
     const uint32_t i = d.p_off + local;
     const float4 xn = a.xa[i];
-    const float4 xo_ = a.xold[i];
-    a.x[i] = xn;
-    const float4 vn = make_float4(d.inv_dt * (xn.x - xo_.x), d.inv_dt * (xn.y - xo_.y), d.inv_dt * (xn.z - xo_.z), 0.f);
-    vo[i] = vn;
-    a.xv[2ull * i] = xn;
-    a.xv[2ull * i + 1] = vn;
-    a.id[i] = a.id_tmp[i];
+    put_final(a, d, i, make_float4(xn.x, xn.y, xn.z, 0.f));
     TILE_LOOP_END
 }
 
 // Vorticity, pass 1 (calcVorticityCUDA, pbf_vorticity_confinement.cu:87-115):
-// omega_i = m/rho0 * sum_j (v_j - v_i) x r_hat * W'(r).  REF: the reference's
-// uncapped 27-cell walk, with h passed where 1/h is expected
-// (pbf_vorticity_confinement.cu:28); otherwise the textbook kernel over the
-// step's neighbour list.  Each form is its own kernel (scenes of the other
-// forms are skipped) so the list form keeps a lean register allocation.
-template <bool REF, bool L16>
-__global__ void __launch_bounds__(512) k_vort_omega(StepArgs a, const float4 *__restrict__ vs)
-{
-    TILE_LOOP_BEGIN
-    const SceneDesc d = a.scenes[s];
-    if (d.vort_mode != (REF ? PBF_VORTICITY_REFERENCE : PBF_VORTICITY_TEXTBOOK)) continue;
-    if (!REF && (d.list16 != 0) != L16) continue;  // the other list format's instance
-    const uint32_t base = a.offsets[d.c_off];
-    const uint32_t live = a.offsets[d.c_off + d.ncell] - base;
-    if (local >= live) continue;
-    const uint32_t i = d.p_off + local;
-    const float4 xi = a.x[i], vi = vs[i];
-    const float kh = REF ? d.h : d.inv_h;
-    const float4 *__restrict__ x = a.x;
-    float w0 = 0.f, w1 = 0.f, w2 = 0.f;
-    auto pair = [&](const float4 &xj, const float4 &vj) {
+// omega_i = m/rho0 * sum_j (v_j - v_i) x r_hat * W'(r).
+struct OmegaSum {
+    float4 xi, vi;
+    float kh, w0 = 0.f, w1 = 0.f, w2 = 0.f;
+    __device__ __forceinline__ OmegaSum(float4 x, float4 v, float k) : xi(x), vi(v), kh(k) {}
+    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz)
+    {
         const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
         const float r2 = p0 * p0 + p1 * p1 + p2 * p2;
         if (r2 > 0.f) {
             const float inv_r = rsqrtf(r2);
-            const float v0 = vj.x - vi.x, v1 = vj.y - vi.y, v2 = vj.z - vi.z;
+            const float v0 = vx - vi.x, v1 = vy - vi.y, v2 = vz - vi.z;
             const float wd = wspiky_d(r2 * inv_r, kh) * inv_r;
             w0 += (v1 * p2 - v2 * p1) * wd;
             w1 += (v2 * p0 - v0 * p2) * wd;
             w2 += (v0 * p1 - v1 * p0) * wd;
         }
-    };
-    // the walk form gathers x and then, for a pair at r > 0, v
-    auto use = [&](uint32_t j) {
-        const float4 xj = __ldg(x + j);
-        const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
-        if (p0 * p0 + p1 * p1 + p2 * p2 > 0.f) pair(xj, __ldg(vs + j));
-    };
-    // the list form gathers both with one 256-bit load of the (x, v) record
-    auto use_rec = [&](uint32_t j) {
-        float4 xj, vj;
-        ld_rec(a.xv + 2ull * j, xj, vj);
-        pair(xj, vj);
-    };
-    if (REF) {  // the kernel scaled by h reaches the whole 27-cell block
-        walk27_batched(
-            d, a.offsets, d.p_off - base, xi,
-            [&](uint32_t j) -> bool {
-                const float4 xj = __ldg(x + j);
-                const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
-                return p0 * p0 + p1 * p1 + p2 * p2 > 0.f;
-            },
-            use);
-    } else {
-        list_walk_any<4>(L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, use_rec);
     }
+};
+
+// omega, and |omega| once per particle beside the position (xs is free after
+// the reorder): pass 2 gathers both with one load per neighbour
+__device__ __forceinline__ void put_omega(const StepArgs &a, const SceneDesc &d, uint32_t i, const OmegaSum &o)
+{
     const float mr = d.m * d.inv_rho0;
-    const float4 wi = make_float4(mr * w0, mr * w1, mr * w2, 0.f);
+    const float4 wi = make_float4(mr * o.w0, mr * o.w1, mr * o.w2, 0.f);
     a.w[i] = wi;
-    // |omega| once per particle, beside the position (xs is free after the
-    // reorder): pass 2 gathers both with one load per neighbour
-    a.xs[i] = make_float4(xi.x, xi.y, xi.z, sqrtf(wi.x * wi.x + wi.y * wi.y + wi.z * wi.z));
-    TILE_LOOP_END
+    a.xs[i] = make_float4(o.xi.x, o.xi.y, o.xi.z, sqrtf(wi.x * wi.x + wi.y * wi.y + wi.z * wi.z));
 }
 
-// Vorticity, pass 2 (addVorticityConfinementCUDA, pbf_vorticity_confinement.cu:192-222).
-template <bool REF, bool L16>
-__global__ void __launch_bounds__(512) k_vort_apply(StepArgs a, float4 *__restrict__ vs)
+// The list form: the textbook kernel over the step's neighbour list, working
+// slots, neighbours' (x, v) in pa and pb.  One instance per list format (each
+// skips the other format's scenes) keeps its registers, and so its
+// occupancy, to that format's loop.
+template <bool L16>
+__global__ void __launch_bounds__(512) k_vort_omega(StepArgs a)
 {
     TILE_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
-    if (d.vort_mode != (REF ? PBF_VORTICITY_REFERENCE : PBF_VORTICITY_TEXTBOOK)) continue;
-    if (!REF && (d.list16 != 0) != L16) continue;  // the other list format's instance
+    if (d.vort_mode != PBF_VORTICITY_TEXTBOOK || (d.list16 != 0) != L16) continue;
     const uint32_t base = a.offsets[d.c_off];
     const uint32_t live = a.offsets[d.c_off + d.ncell] - base;
     if (local >= live) continue;
     const uint32_t i = d.p_off + local;
-    const float4 xi = a.x[i];
-    const float kh = REF ? d.h : d.inv_h;
-    const float sgn = REF ? 1.f : -1.f;
+    const float4 A = a.pa[i];
+    const float2 B = a.pb[i];
+    OmegaSum o(A, make_float4(A.w, B.x, B.y, 0.f), d.inv_h);
+    const float4 *__restrict__ pa = a.pa;
+    const float2 *__restrict__ pb = a.pb;
+    list_walk_any<4>(L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, [&](uint32_t q) {
+        const float4 xj = __ldg(pa + q);
+        const float2 vj = __ldg(pb + q);
+        o.add(xj, xj.w, vj.x, vj.y);
+    });
+    put_omega(a, d, i, o);
+    TILE_LOOP_END
+}
+
+// The reference's uncapped 27-cell walk over final positions in sorted order,
+// with h passed where 1/h is expected (pbf_vorticity_confinement.cu:28).
+__global__ void __launch_bounds__(512) k_vort_omega_walk(StepArgs a)
+{
+    TILE_LOOP_BEGIN
+    const SceneDesc d = a.scenes[s];
+    if (d.vort_mode != PBF_VORTICITY_REFERENCE) continue;
+    const uint32_t base = a.offsets[d.c_off];
+    const uint32_t live = a.offsets[d.c_off + d.ncell] - base;
+    if (local >= live) continue;
+    const uint32_t i = d.p_off + local;
     const float4 *__restrict__ x = a.x;
-    const float4 *__restrict__ w = a.w;
-    const uint32_t lb = (!REF && L16) ? d.p_off : 0u;  // use(j): j counts from lb
-    const float4 *__restrict__ xw = a.xs + lb;          // (x_j, |omega_j|), stored by pass 1
-    float n0 = 0.f, n1 = 0.f, n2 = 0.f;
-    auto use = [&](uint32_t j) {
-        const float4 xj = __ldg(xw + j);
+    const float4 *__restrict__ vs = a.vs;
+    const float4 xi = x[i];
+    OmegaSum o(xi, vs[i], d.h);
+    // the kernel scaled by h reaches the whole 27-cell block
+    walk27_batched(
+        d, a.offsets, d.p_off - base, xi,
+        [&](uint32_t j) -> bool {
+            const float4 xj = __ldg(x + j);
+            const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
+            return p0 * p0 + p1 * p1 + p2 * p2 > 0.f;
+        },
+        [&](uint32_t j) {
+            const float4 vj = __ldg(vs + j);
+            o.add(__ldg(x + j), vj.x, vj.y, vj.z);
+        });
+    put_omega(a, d, i, o);
+    TILE_LOOP_END
+}
+
+// Vorticity, pass 2 (addVorticityConfinementCUDA, pbf_vorticity_confinement.cu:192-222):
+// the sum of |omega_j| grad W.
+struct EtaSum {
+    float4 xi;
+    float kh, sgn, n0 = 0.f, n1 = 0.f, n2 = 0.f;
+    __device__ __forceinline__ EtaSum(float4 x, float k, float sg) : xi(x), kh(k), sgn(sg) {}
+    __device__ __forceinline__ void add(float4 xj)  // (x_j, |omega_j|)
+    {
         const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
         const float r2 = p0 * p0 + p1 * p1 + p2 * p2;
         if (r2 > 0.f) {
             const float inv_r = rsqrtf(r2);
-            const float wl = xj.w;
-            const float f = sgn * wl * wspiky_d(r2 * inv_r, kh) * inv_r;
+            const float f = sgn * xj.w * wspiky_d(r2 * inv_r, kh) * inv_r;
             n0 += f * p0;
             n1 += f * p1;
             n2 += f * p2;
         }
-    };
-    if (REF) {
-        walk27_batched(
-            d, a.offsets, d.p_off - base, xi,
-            [&](uint32_t j) -> bool {
-                const float4 xj = __ldg(x + j);
-                const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
-                return p0 * p0 + p1 * p1 + p2 * p2 > 0.f;
-            },
-            use);
-    } else {
-        // quads of 4: fewer registers, more warps (measured)
-        list_walk_any<4>(L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], 0u, use);
     }
-    const float4 wi = w[i];
+};
+
+// The list form's velocity change, and where the velocity goes next.
+__device__ __forceinline__ void put_confinement(const StepArgs &a, const SceneDesc &d, uint32_t i, const EtaSum &e)
+{
+    const float4 wi = a.w[i];
     const float mr = d.m * d.inv_rho0;
-    float4 v = vs[i];
-    if (REF) {
-        if (sqrtf(n0 * n0 + n1 * n1 + n2 * n2) > 0.f) {
-            n0 = n0 * d.m * d.inv_rho0;
-            n1 = n1 * d.m * d.inv_rho0;
-            n2 = n2 * d.m * d.inv_rho0;
-            const float ln = sqrtf(n0 * n0 + n1 * n1 + n2 * n2);
-            n0 /= ln; n1 /= ln; n2 /= ln;
-            const float c0 = n1 * wi.z - n2 * wi.y, c1 = n2 * wi.x - n0 * wi.z, c2 = n0 * wi.y - n1 * wi.x;
-            v.x = v.x + d.vort_eps * c0 / d.inv_rho0 * d.dt;
-            v.y = v.y + d.vort_eps * c1 / d.inv_rho0 * d.dt;
-            v.z = v.z + d.vort_eps * c2 / d.inv_rho0 * d.dt;
-        }
-    } else {
-        n0 *= mr; n1 *= mr; n2 *= mr;
-        const float ln = sqrtf(n0 * n0 + n1 * n1 + n2 * n2);
-        if (ln > 0.f) {
-            n0 /= ln; n1 /= ln; n2 /= ln;
-            const float c0 = n1 * wi.z - n2 * wi.y, c1 = n2 * wi.x - n0 * wi.z, c2 = n0 * wi.y - n1 * wi.x;
-            v.x = v.x + d.dt * d.vort_eps * c0;
-            v.y = v.y + d.dt * d.vort_eps * c1;
-            v.z = v.z + d.dt * d.vort_eps * c2;
-        }
+    const float4 A = a.pa[i];
+    const float2 B = a.pb[i];
+    float4 v = make_float4(A.w, B.x, B.y, 0.f);
+    float n0 = e.n0 * mr, n1 = e.n1 * mr, n2 = e.n2 * mr;
+    const float ln = sqrtf(n0 * n0 + n1 * n1 + n2 * n2);
+    if (ln > 0.f) {
+        n0 /= ln; n1 /= ln; n2 /= ln;
+        const float c0 = n1 * wi.z - n2 * wi.y, c1 = n2 * wi.x - n0 * wi.z, c2 = n0 * wi.y - n1 * wi.x;
+        v.x = v.x + d.dt * d.vort_eps * c0;
+        v.y = v.y + d.dt * d.vort_eps * c1;
+        v.z = v.z + d.dt * d.vort_eps * c2;
     }
-    vs[i] = v;
-    TILE_LOOP_END
+    put_velocity(a, d.xsph_mode == PBF_XSPH_LIST, d.xsph_mode == PBF_XSPH_WALK, i,
+                 [&] { return __float_as_uint(a.xold[i].w); }, A, v);
 }
 
-// XSPH (calcXSPHCUDA, pbf_xsph.cu:84-113): v_i += c m/rho0 sum_j (v_j - v_i) W(r_ij),
-// NaN guard.  WALK: the reference's uncapped 27-cell walk (scenes with
-// PBF_XSPH_WALK); otherwise over the step's neighbour list (scenes with
-// PBF_XSPH_LIST), also copying vs to vo for scenes without XSPH.
-template <bool WALK, bool L16>
-__global__ void __launch_bounds__(512) k_xsph(StepArgs a, const float4 *__restrict__ vs, float4 *__restrict__ vo)
+template <bool L16>
+__global__ void __launch_bounds__(512) k_vort_apply(StepArgs a)
 {
     TILE_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
-    if ((d.xsph_mode == PBF_XSPH_WALK) != WALK) continue;
-    if (!WALK && (d.list16 != 0) != L16) continue;  // the other list format's instance
+    if (d.vort_mode != PBF_VORTICITY_TEXTBOOK || (d.list16 != 0) != L16) continue;
     const uint32_t base = a.offsets[d.c_off];
     const uint32_t live = a.offsets[d.c_off + d.ncell] - base;
     if (local >= live) continue;
     const uint32_t i = d.p_off + local;
-    const float4 xi = a.x[i], vi = vs[i];
-    if (!WALK && d.xsph_mode == PBF_XSPH_OFF) {  // scene without XSPH in a batch that has some
-        vo[i] = vi;
-        continue;
-    }
-    const float inv_h = d.inv_h, alpha6 = d.alpha6;
+    // u16 lists index the array offset by the scene's first slot (no add per slot)
+    const float4 *__restrict__ xw = a.xs + (L16 ? d.p_off : 0u);
+    EtaSum e(a.xs[i], d.inv_h, -1.f);
+    list_walk_any<4>(L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], 0u, [&](uint32_t q) { e.add(__ldg(xw + q)); });
+    put_confinement(a, d, i, e);
+    TILE_LOOP_END
+}
+
+// The reference's form (sorted order throughout; the XSPH list form that may
+// follow reads working order).
+__global__ void __launch_bounds__(512) k_vort_apply_walk(StepArgs a)
+{
+    TILE_LOOP_BEGIN
+    const SceneDesc d = a.scenes[s];
+    if (d.vort_mode != PBF_VORTICITY_REFERENCE) continue;
+    const uint32_t base = a.offsets[d.c_off];
+    const uint32_t live = a.offsets[d.c_off + d.ncell] - base;
+    if (local >= live) continue;
+    const uint32_t i = d.p_off + local;
     const float4 *__restrict__ x = a.x;
-    const uint32_t lb = (!WALK && L16) ? d.p_off : 0u;  // use(j): j counts from lb
-    const float4 *__restrict__ xb = x + lb;
-    const float4 *__restrict__ vb = vs + lb;
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-    const float ih2 = inv_h * inv_h;
-    auto use = [&](uint32_t j) {
-        const float4 xj = __ldg(xb + j);
+    const float4 *__restrict__ xw = a.xs;
+    const float4 xi = x[i];
+    EtaSum e(xi, d.h, 1.f);
+    walk27_batched(
+        d, a.offsets, d.p_off - base, xi,
+        [&](uint32_t j) -> bool {
+            const float4 xj = __ldg(x + j);
+            const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
+            return p0 * p0 + p1 * p1 + p2 * p2 > 0.f;
+        },
+        [&](uint32_t j) { e.add(__ldg(xw + j)); });
+    const float4 wi = a.w[i];
+    float4 v = a.vs[i];
+    float n0 = e.n0, n1 = e.n1, n2 = e.n2;
+    if (sqrtf(n0 * n0 + n1 * n1 + n2 * n2) > 0.f) {
+        n0 = n0 * d.m * d.inv_rho0;
+        n1 = n1 * d.m * d.inv_rho0;
+        n2 = n2 * d.m * d.inv_rho0;
+        const float ln = sqrtf(n0 * n0 + n1 * n1 + n2 * n2);
+        n0 /= ln; n1 /= ln; n2 /= ln;
+        const float c0 = n1 * wi.z - n2 * wi.y, c1 = n2 * wi.x - n0 * wi.z, c2 = n0 * wi.y - n1 * wi.x;
+        v.x = v.x + d.vort_eps * c0 / d.inv_rho0 * d.dt;
+        v.y = v.y + d.vort_eps * c1 / d.inv_rho0 * d.dt;
+        v.z = v.z + d.vort_eps * c2 / d.inv_rho0 * d.dt;
+    }
+    put_velocity(a, d.xsph_mode == PBF_XSPH_LIST, d.xsph_mode == PBF_XSPH_WALK, a.wpos[i], [&] { return i; }, xi, v);
+    TILE_LOOP_END
+}
+
+// XSPH (calcXSPHCUDA, pbf_xsph.cu:84-113): v_i += c m/rho0 sum_j (v_j - v_i) W(r_ij),
+// NaN guard.  Bound by the L1 wavefronts of its gathers: a neighbour's
+// position and velocity as 16 + 8 bytes instead of two float4 took the list
+// form from 446 to 355 us at 5.95 M particles (u16 lists), 96 to 77 us at
+// 1,048,576 (u32 lists).
+struct XsphSum {
+    float4 xi, vi;
+    float ih2, alpha6, s0 = 0.f, s1 = 0.f, s2 = 0.f;
+    __device__ __forceinline__ XsphSum(float4 x, float4 v, const SceneDesc &d)
+        : xi(x), vi(v), ih2(d.inv_h * d.inv_h), alpha6(d.alpha6)
+    {
+    }
+    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz)
+    {
         const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
         // Wpoly6 from r^2 (q^2 = r^2 / h^2 instead of (|r| / h)^2: no square
         // root per pair; the two differ by rounding only)
         const float q2 = (p0 * p0 + p1 * p1 + p2 * p2) * ih2;
         const float t = 1.f - q2;
         const float W = (q2 <= 1.f) ? alpha6 * t * t * t : 0.f;
-        const float4 vj = __ldg(vb + j);
-        s0 += (vj.x - vi.x) * W;
-        s1 += (vj.y - vi.y) * W;
-        s2 += (vj.z - vi.z) * W;
-    };
-    if (WALK) {
-        // W = 0 beyond h: those candidates add nothing (a non-finite velocity
-        // of a non-neighbour is no longer folded into the sum; such particles
-        // raise PBF_FLAG_NONFINITE in the next step's prediction)
-        const float rcut2 = d.h2 * 1.0001f;
-        walk27_batched(
-            d, a.offsets, d.p_off - base, xi,
-            [&](uint32_t j) -> bool {
-                const float4 xj = __ldg(x + j);
-                const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
-                return p0 * p0 + p1 * p1 + p2 * p2 <= rcut2;
-            },
-            use);
-    } else {
-        if (L16)
-            list_walk16(list_of(a.nbr, i), a.nbr_stride, a.nnb[i], 0u, use);
-        else
-            list_walk_ahead2(list_of(a.nbr, i), a.nbr_stride, a.nnb[i], use);
+        s0 += (vx - vi.x) * W;
+        s1 += (vy - vi.y) * W;
+        s2 += (vz - vi.z) * W;
     }
-    float4 out = vi;
-    if (!(isnan(s0) || isnan(s1) || isnan(s2))) {
-        const float c = d.xsph_c * d.m * d.inv_rho0;
-        out.x = vi.x + c * s0;
-        out.y = vi.y + c * s1;
-        out.z = vi.z + c * s2;
+    __device__ __forceinline__ float4 result(const SceneDesc &d) const
+    {
+        float4 out = vi;
+        if (!(isnan(s0) || isnan(s1) || isnan(s2))) {
+            const float c = d.xsph_c * d.m * d.inv_rho0;
+            out.x = vi.x + c * s0;
+            out.y = vi.y + c * s1;
+            out.z = vi.z + c * s2;
+        }
+        return out;
     }
-    vo[i] = out;
+};
+
+template <bool L16>
+__global__ void __launch_bounds__(512) k_xsph(StepArgs a)
+{
+    TILE_LOOP_BEGIN
+    const SceneDesc d = a.scenes[s];
+    if (d.xsph_mode != PBF_XSPH_LIST || (d.list16 != 0) != L16) continue;
+    const uint32_t base = a.offsets[d.c_off];
+    const uint32_t live = a.offsets[d.c_off + d.ncell] - base;
+    if (local >= live) continue;
+    const uint32_t i = d.p_off + local;
+    const float4 *__restrict__ pa = a.pa;
+    const float2 *__restrict__ pb = a.pb;
+    const float4 A = a.pa[i];
+    const float2 B = a.pb[i];
+    XsphSum o(A, make_float4(A.w, B.x, B.y, 0.f), d);
+    list_walk_any<4>(L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, [&](uint32_t q) {
+        const float4 xj = __ldg(pa + q);
+        const float2 vj = __ldg(pb + q);
+        o.add(xj, xj.w, vj.x, vj.y);
+    });
+    a.v[__float_as_uint(a.xold[i].w)] = o.result(d);
+    TILE_LOOP_END
+}
+
+// The reference's uncapped 27-cell walk (scenes with PBF_XSPH_WALK), sorted
+// order.
+__global__ void __launch_bounds__(512) k_xsph_walk(StepArgs a)
+{
+    TILE_LOOP_BEGIN
+    const SceneDesc d = a.scenes[s];
+    if (d.xsph_mode != PBF_XSPH_WALK) continue;
+    const uint32_t base = a.offsets[d.c_off];
+    const uint32_t live = a.offsets[d.c_off + d.ncell] - base;
+    if (local >= live) continue;
+    const uint32_t i = d.p_off + local;
+    const float4 *__restrict__ x = a.x;
+    const float4 *__restrict__ vs = a.vs;
+    const float4 xi = x[i];
+    XsphSum o(xi, vs[i], d);
+    // W = 0 beyond h: those candidates add nothing (a non-finite velocity
+    // of a non-neighbour is no longer folded into the sum; such particles
+    // raise PBF_FLAG_NONFINITE in the next step's prediction)
+    const float rcut2 = d.h2 * 1.0001f;
+    walk27_batched(
+        d, a.offsets, d.p_off - base, xi,
+        [&](uint32_t j) -> bool {
+            const float4 xj = __ldg(x + j);
+            const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
+            return p0 * p0 + p1 * p1 + p2 * p2 <= rcut2;
+        },
+        [&](uint32_t j) {
+            const float4 vj = __ldg(vs + j);
+            o.add(__ldg(x + j), vj.x, vj.y, vj.z);
+        });
+    a.v[i] = o.result(d);
     TILE_LOOP_END
 }
 
@@ -1973,13 +2034,13 @@ struct PassFns {
             k_lambda<CH, false><<<sh.grid_lambda, sh.tile, 0, st>>>(a, cur);
     }
     // lamw: lambda in .w of cur (iterations >= 1); iteration 0 reads it from lam
-    static void launch_dp(const StepArgs &a, const LaunchShape &sh, const float4 *cur, float4 *out, float4 *vo,
-                          int last, bool lamw, cudaStream_t st)
+    static void launch_dp(const StepArgs &a, const LaunchShape &sh, const float4 *cur, float4 *out, int last,
+                          bool lamw, cudaStream_t st)
     {
         if (lamw)
-            k_dp<CH, true><<<sh.grid_dp, sh.tile, 0, st>>>(a, cur, out, vo, last);
+            k_dp<CH, true><<<sh.grid_dp, sh.tile, 0, st>>>(a, cur, out, last);
         else
-            k_dp<CH, false><<<sh.grid_dp, sh.tile, 0, st>>>(a, cur, out, vo, last);
+            k_dp<CH, false><<<sh.grid_dp, sh.tile, 0, st>>>(a, cur, out, last);
     }
 };
 
@@ -2022,9 +2083,12 @@ Occupancy occupancy(uint32_t tile, uint32_t chunk)
     const bool c4 = chunk == 4;
     o.lambda = occ(c4 ? PassFns<4>::lambda() : PassFns<8>::lambda());
     o.dp = occ(c4 ? PassFns<4>::dp() : PassFns<8>::dp());
-    o.omega = mn(occ((const void *)k_vort_omega<false, false>), occ((const void *)k_vort_omega<false, true>));
-    o.apply = mn(occ((const void *)k_vort_apply<false, false>), occ((const void *)k_vort_apply<false, true>));
-    o.xsph = mn(occ((const void *)k_xsph<false, false>), occ((const void *)k_xsph<false, true>));
+    o.omega[0] = occ((const void *)k_vort_omega<false>);
+    o.omega[1] = occ((const void *)k_vort_omega<true>);
+    o.apply[0] = occ((const void *)k_vort_apply<false>);
+    o.apply[1] = occ((const void *)k_vort_apply<true>);
+    o.xsph[0] = occ((const void *)k_xsph<false>);
+    o.xsph[1] = occ((const void *)k_xsph<true>);
     std::lock_guard<std::mutex> lk(mu);
     cache[key] = o;
     return o;
@@ -2128,73 +2192,47 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
             k_neighbors_lambda<false><<<sh.grid_nb, b, 0, st>>>(a);
         PBF_LAUNCHED("k_neighbors_lambda");
     }
-    const bool xsph = (post & (kPostXsphWalk | kPostXsphList)) != 0;
-    float4 *vfinal = xsph ? a.vt : a.v;
     float4 *cur = a.xa, *nxt = a.xb;
     for (int it = 0; it < iters; ++it) {
         if (it > 0) {
             PBF_PASS_DISPATCH(sh.chunk, launch_lambda(a, sh, cur, !sh.small, st));
             PBF_LAUNCHED("k_lambda");
         }
-        const bool last = (it == iters - 1);
-        float4 *out = last ? a.x : nxt;
-        PBF_PASS_DISPATCH(sh.chunk,
-                          launch_dp(a, sh, cur, out, last ? vfinal : nullptr, last ? 1 : 0, it > 0 && !sh.small, st));
+        PBF_PASS_DISPATCH(sh.chunk, launch_dp(a, sh, cur, nxt, it == iters - 1 ? 1 : 0, it > 0 && !sh.small, st));
         PBF_LAUNCHED("k_dp");
-        float4 *t = cur;
-        cur = nxt;
-        nxt = t;
+        std::swap(cur, nxt);
     }
     if (iters <= 0) {
-        k_finalize<<<g, b, 0, st>>>(a, vfinal);
+        k_finalize<<<g, b, 0, st>>>(a);
         PBF_LAUNCHED("k_finalize");
     }
-    // omega of every form before any apply: both forms read final positions
-    // and velocities only
-    // the list forms run one instance per list format present (each skips
-    // the other format's scenes): one instance per format keeps its
-    // registers, and so its occupancy, to that format's loop
+    // the list forms run one instance per list format present
     const bool l16 = (post & kPostList16) != 0, l32 = (post & kPostList32) != 0;
+#define PBF_POST(kernel, grid)                   \
+    if (l32) {                                   \
+        kernel<false><<<grid[0], b, 0, st>>>(a); \
+        PBF_LAUNCHED(#kernel);                   \
+    }                                            \
+    if (l16) {                                   \
+        kernel<true><<<grid[1], b, 0, st>>>(a);  \
+        PBF_LAUNCHED(#kernel);                   \
+    }
     if (post & kPostVortTextbook) {
-        if (l32) {
-            k_vort_omega<false, false><<<sh.grid_omega, b, 0, st>>>(a, vfinal);
-            PBF_LAUNCHED("k_vort_omega");
-        }
-        if (l16) {
-            k_vort_omega<false, true><<<sh.grid_omega, b, 0, st>>>(a, vfinal);
-            PBF_LAUNCHED("k_vort_omega");
-        }
+        PBF_POST(k_vort_omega, sh.grid_omega)
+        PBF_POST(k_vort_apply, sh.grid_apply)
     }
     if (post & kPostVortReference) {
-        k_vort_omega<true, false><<<sh.grid_omega, b, 0, st>>>(a, vfinal);
+        k_vort_omega_walk<<<g, b, 0, st>>>(a);
         PBF_LAUNCHED("k_vort_omega_walk");
-    }
-    if (post & kPostVortTextbook) {
-        if (l32) {
-            k_vort_apply<false, false><<<sh.grid_apply, b, 0, st>>>(a, vfinal);
-            PBF_LAUNCHED("k_vort_apply");
-        }
-        if (l16) {
-            k_vort_apply<false, true><<<sh.grid_apply, b, 0, st>>>(a, vfinal);
-            PBF_LAUNCHED("k_vort_apply");
-        }
-    }
-    if (post & kPostVortReference) {
-        k_vort_apply<true, false><<<sh.grid_apply, b, 0, st>>>(a, vfinal);
+        k_vort_apply_walk<<<g, b, 0, st>>>(a);
         PBF_LAUNCHED("k_vort_apply_walk");
     }
     if (post & kPostXsphList) {
-        if (l32) {
-            k_xsph<false, false><<<sh.grid_xsph, b, 0, st>>>(a, a.vt, a.v);
-            PBF_LAUNCHED("k_xsph");
-        }
-        if (l16) {
-            k_xsph<false, true><<<sh.grid_xsph, b, 0, st>>>(a, a.vt, a.v);
-            PBF_LAUNCHED("k_xsph");
-        }
+        PBF_POST(k_xsph, sh.grid_xsph)
     }
+#undef PBF_POST
     if (post & kPostXsphWalk) {
-        k_xsph<true, false><<<sh.grid_xsph, b, 0, st>>>(a, a.vt, a.v);
+        k_xsph_walk<<<g, b, 0, st>>>(a);
         PBF_LAUNCHED("k_xsph_walk");
     }
 #undef PBF_LAUNCHED
