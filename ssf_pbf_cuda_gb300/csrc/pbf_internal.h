@@ -121,7 +121,7 @@ struct StepArgs {
     uint32_t *wpos;               // sorted slot -> working slot
     uint32_t *dense;              // [0] count, then (cell, scene) pairs of buckets for k_dense_sort
     uint32_t *mid;                // the same for buckets of kMidMin+1 .. kDenseMin members
-    uint64_t *chist;              // per cell: 8 x 8-bit class counts of its bucket, or kClassWhole
+    uint64_t *chist;              // per cell: 8 x 8-bit class ends of its bucket, or kClassWhole
     uint32_t *next_id;            // per scene: id of the next particle added
     uint64_t nbr_stride;
     const PackedIn *pin;          // packed-input steps: the input buffers
@@ -205,7 +205,7 @@ void launch_unpack(const StepArgs &a, const LaunchShape &sh, const uint32_t *pac
 void launch_pack(const StepArgs &a, const LaunchShape &sh, const uint32_t *pack_off, float *dst_x, float *dst_v,
                  cudaStream_t st);
 
-// chist value of a bucket in plain sorted order, walked whole (more than 255
+// chist value of a bucket in plain sorted order, walked whole (more than 254
 // members, or a table of fewer than 4 cells on an axis)
 constexpr uint64_t kClassWhole = ~0ull;
 
