@@ -782,15 +782,20 @@ LaunchShape Batch::shape_for(uint32_t tile) const
     sh.grid_split = std::min<uint32_t>((uint32_t)sms_ * std::max<uint32_t>(1, o.split), ntb * (tile / (256 / kSplit)));
     const uint32_t scan_tiles = std::max<uint32_t>(1, (ctrl_.n_cells + kScanTile - 1) / kScanTile);
     sh.scan_grid = std::min<uint32_t>(pow2(scan_tiles), (uint32_t)sms_ * 8);
-    if (ctrl_.n_cells <= kSingleScanMax) sh.scan_grid = 0;  // one-block scan
     {  // the block's lists in shared memory when they fit
         const uint64_t b = (uint64_t)tile * (max_pair_ - 1u) * 4u;
         sh.nb_smem = b <= kNbSmemMax ? (uint32_t)b : 0u;
     }
-    sh.scan_rounds = 0;
-    if (sh.scan_grid == 0) {  // the table's rounds of 1024 cells, if they fit in registers
-        const uint32_t r = std::max<uint32_t>(1, (ctrl_.n_cells + 1023u) / 1024u);
-        if (r <= 16) sh.scan_rounds = r;
+    // one kernel while the table fits in registers: one block, then a cluster
+    sh.scan_cluster = sh.scan_rounds = 0;
+    const uint32_t cells = std::max<uint32_t>(1, ctrl_.n_cells), lim = scan_cluster_limit();
+    if (cells <= kBlockScanMax) {
+        sh.scan_grid = 0;
+        sh.scan_rounds = (cells + 1023u) / 1024u;
+    } else if (cells <= lim * 1024u * kScanRoundsMax) {
+        sh.scan_grid = 0;
+        sh.scan_cluster = lim;
+        sh.scan_rounds = std::min(pow2((cells + lim * 1024u - 1u) / (lim * 1024u)), kScanRoundsMax);
     }
     return sh;
 }

@@ -131,8 +131,9 @@ struct StepArgs {
 struct LaunchShape {
     uint32_t tile;        // particles per tile = threads per block
     uint32_t grid;        // persistent grid (blocks) for the light tile kernels
-    uint32_t scan_grid;   // grid for the scan kernels; 0 = the one-block scan
-    uint32_t scan_rounds; // one-block scan: rounds of 1024 cells held in registers (1..16), 0 = looped
+    uint32_t scan_grid;   // grid for the three scan kernels; 0 = one kernel
+    uint32_t scan_cluster; // one kernel: blocks of its cluster, 0 = one block
+    uint32_t scan_rounds; // one kernel: rounds of 1024 cells a block holds in registers
     uint32_t chunk;       // neighbours per chunk in the lambda / delta-p passes (4 or 8)
     // persistent grids of the heavy kernels, each from its own occupancy
     uint32_t grid_nb, grid_lambda, grid_dp;
@@ -145,7 +146,7 @@ struct LaunchShape {
     uint32_t nb_smem;     // k_neighbors_lambda: bytes of shared memory for the block's lists (0 = stored directly)
     bool operator==(const LaunchShape &o) const
     {
-        return tile == o.tile && grid == o.grid && scan_grid == o.scan_grid && scan_rounds == o.scan_rounds &&
+        return tile == o.tile && grid == o.grid && scan_grid == o.scan_grid && scan_rounds == o.scan_rounds && scan_cluster == o.scan_cluster &&
                chunk == o.chunk &&
                grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && grid_split == o.grid_split && nb_smem == o.nb_smem &&
                grid_nb == o.grid_nb && grid_lambda == o.grid_lambda && grid_dp == o.grid_dp &&
@@ -160,6 +161,7 @@ struct Occupancy {
     uint32_t omega[2], apply[2], xsph[2];
 };
 Occupancy occupancy(uint32_t tile, uint32_t chunk);
+uint32_t scan_cluster_limit();  // blocks the scan's cluster may have on the current device
 
 // Called after every kernel launch of a step (per-kernel event timing).
 struct StepHook {
@@ -212,7 +214,9 @@ constexpr uint64_t kClassWhole = ~0ull;
 constexpr uint32_t kScanItemsPerWarp = 512;   // 32 lanes x 16
 constexpr uint32_t kScanWarps = 8;
 constexpr uint32_t kScanTile = kScanItemsPerWarp * kScanWarps;  // 4096 cells per scan tile
-constexpr uint32_t kSingleScanMax = 65536;  // cells up to which one block scans the whole table
+constexpr uint32_t kBlockScanMax = 8192;      // cells up to which one block scans the whole table
+constexpr uint32_t kScanClusterMax = 16;      // blocks of the scan's cluster (1024 threads each)
+constexpr uint32_t kScanRoundsMax = 18;       // cells a thread of it may hold: tables are 2^k + 1 cells, up to 2^18 + 1
 constexpr uint32_t kNbSmemMax = 96 * 1024;  // shared-memory budget for a k_neighbors_lambda block's lists
 constexpr uint32_t kSplit = 4;  // small steps: lanes per particle in the split neighbour walk (blocks of 256)
 constexpr uint32_t kCellTile = 256;         // default cells per cell tile = threads per k_rank_cells block

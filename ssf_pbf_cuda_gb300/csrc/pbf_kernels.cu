@@ -15,6 +15,8 @@
 // acceptance) uses explicitly rounded intrinsics so that it is bit-exact
 // against the CPU oracle.  Floating-point solver math follows the reference's
 // operation order but uses rsqrtf (as the reference does).
+#include <cooperative_groups.h>
+
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -734,41 +736,65 @@ __global__ void __launch_bounds__(1024) k_scan_single_reg(StepArgs a)
     }
 }
 
-// The whole scan in one block, for tables of at most kSingleScanMax cells
-// (small scenes: one launch instead of three).
-__global__ void __launch_bounds__(1024) k_scan_single(StepArgs a)
+// The whole scan in one thread-block cluster, for the tables between the
+// one-block scan and the three-kernel one: each block holds a run of 1024 * R
+// cells in registers as k_scan_single_reg does, its total goes into every
+// other block's shared memory, and after the cluster's barrier each block
+// adds the totals before it.  Bound by the latency of the one launch: 32,769
+// cells (event-timed, launch included) took 27.7 us in one block looping over
+// rounds of 1024 cells and take 8.4 here (9.3 in a cluster of 8), 65,537
+// cells 20.2 us in three kernels and 9.3 here.
+template <uint32_t R>
+__global__ void __launch_bounds__(1024) k_scan_cluster(StepArgs a)
 {
-    __shared__ uint32_t ws[32];
-    __shared__ uint32_t carry;
-    const uint32_t n = a.ctrl->n_cells;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        carry = 0;
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cluster = cg::this_cluster();
+    __shared__ uint32_t ws[R][32], tot[kScanClusterMax];
+    const uint32_t n = a.ctrl->n_cells, rank = cluster.block_rank(), blocks = cluster.num_blocks();
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, base = rank * (1024u * R);
+    if (rank == 0 && t == 0) {
         *a.dense = 0;  // the bucket queues of this step's rank kernel
         *a.mid = 0;
     }
+    uint32_t v[R], inc[R];
+#pragma unroll
+    for (uint32_t k = 0; k < R; ++k) {
+        const uint32_t idx = base + k * 1024u + t;
+        v[k] = idx < n ? a.count[idx] : 0u;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < R; ++k) {
+        inc[k] = warp_incl_scan(v[k]);
+        if (lane == 31) ws[k][warp] = inc[k];
+    }
     __syncthreads();
-    for (uint32_t base = 0; base < n; base += 1024) {
-        const uint32_t idx = base + threadIdx.x;
-        const uint32_t v = idx < n ? a.count[idx] : 0u;
-        const uint32_t inc = warp_incl_scan(v);
-        if (lane == 31) ws[warp] = inc;
-        __syncthreads();
-        if (warp == 0) {
-            const uint32_t wv = ws[lane];
-            ws[lane] = warp_incl_scan(wv) - wv;
+    if (warp == 0) {
+        uint32_t carry = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < R; ++k) {
+            const uint32_t wv = ws[k][lane];
+            const uint32_t wi = warp_incl_scan(wv);
+            ws[k][lane] = carry + wi - wv;
+            carry += __shfl_sync(0xffffffffu, wi, 31);
         }
-        __syncthreads();
-        const uint32_t c = carry;
+        if (lane < blocks) *cluster.map_shared_rank(&tot[rank], lane) = carry;
+    }
+    cluster.sync();  // every block's totals are in; no block writes another's memory after it
+    uint32_t before = 0, all = 0;
+    for (uint32_t k = 0; k < blocks; ++k) {
+        const uint32_t x = tot[k];
+        before += k < rank ? x : 0u;
+        all += x;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < R; ++k) {
+        const uint32_t idx = base + k * 1024u + t;
         if (idx < n) {
-            a.offsets[idx] = c + ws[warp] + inc - v;
+            a.offsets[idx] = before + ws[k][warp] + inc[k] - v[k];
             a.count[idx] = 0u;  // ready for the next step's histogram
         }
-        __syncthreads();
-        if (threadIdx.x == 1023) carry = c + ws[warp] + inc;
-        __syncthreads();
     }
-    if (threadIdx.x == 0) a.offsets[n] = carry;
+    if (rank == 0 && t == 0) a.offsets[n] = all;
 }
 
 __global__ void __launch_bounds__(256) k_scan_down(StepArgs a)
@@ -2144,6 +2170,52 @@ void launch_set_packed_in(PackedIn *dst, const float *x, const float *v, cudaStr
     k_set_packed_in<<<1, 1, 0, st>>>(dst, x, v);
 }
 
+using ScanFn = void (*)(StepArgs);
+static ScanFn scan_cluster_fn(uint32_t rounds)
+{
+    switch (rounds) {
+    case 1: return k_scan_cluster<1>;
+    case 2: return k_scan_cluster<2>;
+    case 4: return k_scan_cluster<4>;
+    case 8: return k_scan_cluster<8>;
+    case 16: return k_scan_cluster<16>;
+    default: return k_scan_cluster<kScanRoundsMax>;
+    }
+}
+
+// The largest cluster the scan may use on the current device (16 blocks of
+// 1024 threads are beyond the portable size; a device without room for one
+// such cluster takes 8), asked once per device.
+uint32_t scan_cluster_limit()
+{
+    static std::mutex mu;
+    static std::map<int, uint32_t> cache;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    const auto it = cache.find(dev);
+    if (it != cache.end()) return it->second;
+    bool ok = true;
+    for (uint32_t r : {1u, 2u, 4u, 8u, 16u, kScanRoundsMax}) {
+        const ScanFn fn = scan_cluster_fn(r);
+        ok = ok && cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kScanClusterMax);
+        cfg.blockDim = dim3(1024);
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kScanClusterMax;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        ok = ok && cudaOccupancyMaxActiveClusters(&n, (const void *)fn, &cfg) == cudaSuccess && n > 0;
+    }
+    cudaGetLastError();  // a refused attribute is an answer, not an error
+    cache[dev] = ok ? kScanClusterMax : 8u;
+    return cache[dev];
+}
+
 uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint32_t post,
                       cudaStream_t st, StepHook *hook, bool packed)
 {
@@ -2159,16 +2231,27 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
     else
         k_predict_hash<false><<<g, b, 0, st>>>(a);
     PBF_LAUNCHED("k_predict_hash");
-    if (sh.scan_grid == 0) {  // small table: one block
+    if (sh.scan_grid == 0 && sh.scan_cluster) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(sh.scan_cluster);
+        cfg.blockDim = dim3(1024);
+        cfg.stream = st;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = sh.scan_cluster;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, scan_cluster_fn(sh.scan_rounds), a);
+        PBF_LAUNCHED("k_scan_single");  // the profile's name for the scan in one launch
+    } else if (sh.scan_grid == 0) {  // small table: one block
         switch (sh.scan_rounds) {  // rounds of 1024 cells held in registers
 #define PBF_SCAN_ROUNDS(r) \
     case r: k_scan_single_reg<r><<<1, 1024, 0, st>>>(a); break;
         PBF_SCAN_ROUNDS(1) PBF_SCAN_ROUNDS(2) PBF_SCAN_ROUNDS(3) PBF_SCAN_ROUNDS(4)
-        PBF_SCAN_ROUNDS(5) PBF_SCAN_ROUNDS(6) PBF_SCAN_ROUNDS(7) PBF_SCAN_ROUNDS(8)
-        PBF_SCAN_ROUNDS(9) PBF_SCAN_ROUNDS(10) PBF_SCAN_ROUNDS(11) PBF_SCAN_ROUNDS(12)
-        PBF_SCAN_ROUNDS(13) PBF_SCAN_ROUNDS(14) PBF_SCAN_ROUNDS(15) PBF_SCAN_ROUNDS(16)
+        PBF_SCAN_ROUNDS(5) PBF_SCAN_ROUNDS(6) PBF_SCAN_ROUNDS(7)
 #undef PBF_SCAN_ROUNDS
-        default: k_scan_single<<<1, 1024, 0, st>>>(a); break;
+        default: k_scan_single_reg<8><<<1, 1024, 0, st>>>(a); break;
         }
         PBF_LAUNCHED("k_scan_single");
     } else {
