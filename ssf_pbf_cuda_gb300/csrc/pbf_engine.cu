@@ -429,31 +429,25 @@ pbf_status Batch::set_particles(uint32_t id, const float *x, const float *v, uin
     if ((uint64_t)start + n > s.desc.capacity) return PBF_ERROR_CAPACITY;
     float4 *dx = d_x_ + s.desc.p_off + start;
     float4 *dv = d_v_ + s.desc.p_off + start;
-    if (n) {
-        const float *sx = x, *sv = v;
-        if (!src_dev) {
-            // raw AoS float3 goes to the scene's slice of the xs / vt scratch
-            // (free between steps) and is widened on the device
-            float *stx = reinterpret_cast<float *>(d_xs_ + s.desc.p_off + start);
-            float *stv = reinterpret_cast<float *>(d_pa_ + s.desc.p_off + start);
-            CK(cudaMemcpyAsync(stx, x, 12ull * n, cudaMemcpyHostToDevice, st));
-            if (v) CK(cudaMemcpyAsync(stv, v, 12ull * n, cudaMemcpyHostToDevice, st));
-            sx = stx;
-            sv = v ? stv : nullptr;
-        }
-        launch_aos3_to_f4(sx, dx, n, st);
-        if (sv) launch_aos3_to_f4(sv, dv, n, st);
-        else CK(cudaMemsetAsync(dv, 0, 16ull * n, st));
-        CK(cudaGetLastError());
+    const float *sx = x, *sv = v;
+    if (n && !src_dev) {
+        // raw AoS float3 goes to the scene's slice of the xs / pa scratch
+        // (free between steps) and is widened on the device
+        float *stx = reinterpret_cast<float *>(d_xs_ + s.desc.p_off + start);
+        float *stv = reinterpret_cast<float *>(d_pa_ + s.desc.p_off + start);
+        CK(cudaMemcpyAsync(stx, x, 12ull * n, cudaMemcpyHostToDevice, st));
+        if (v) CK(cudaMemcpyAsync(stv, v, 12ull * n, cudaMemcpyHostToDevice, st));
+        sx = stx;
+        sv = v ? stv : nullptr;
     }
     // ids: a fresh set numbers the particles 0..n-1; an append continues
     // from the scene's device-side counter
-    launch_assign_ids(d_id_ + s.desc.p_off + start, d_next_id_ + id, n, append, st);
+    const uint32_t total = start + n;
+    launch_load_phase(sx, sv, dx, dv, d_id_ + s.desc.p_off + start, d_next_id_ + id, d_scene_num_ + id, n, total, append,
+                      st);
+    if (append) launch_bump_next_id(d_next_id_ + id, n, st);
     CK(cudaGetLastError());
     s.perm_valid = false;
-    const uint32_t total = start + n;
-    launch_set_u32(d_scene_num_ + id, total, st);
-    CK(cudaGetLastError());
     if (s.num_upper != total) dirty_tiles_ = true;
     s.num_upper = total;
     return PBF_SUCCESS;
@@ -780,6 +774,7 @@ LaunchShape Batch::shape_for(uint32_t tile) const
     sh.cell_tile = cell_tile_;
     sh.small = (uint64_t)nt * tile <= kSmallStep ? 1u : 0u;
     sh.grid_split = std::min<uint32_t>((uint32_t)sms_ * std::max<uint32_t>(1, o.split), ntb * (tile / (256 / kSplit)));
+    sh.grid_small = ntb * (tile / kSmallBlock);
     const uint32_t scan_tiles = std::max<uint32_t>(1, (ctrl_.n_cells + kScanTile - 1) / kScanTile);
     sh.scan_grid = std::min<uint32_t>(pow2(scan_tiles), (uint32_t)sms_ * 8);
     {  // the block's lists in shared memory when they fit
@@ -1025,21 +1020,19 @@ pbf_status Batch::get_particles(uint32_t id, float *x, float *v, uint32_t *num, 
     if (num) *num = n;
     if (!n) return PBF_SUCCESS;
     const SceneHost &s = scenes_[id];
-    float *stage = reinterpret_cast<float *>(d_xs_ + s.desc.p_off);  // xs is free between steps
-    float4 *srcs[2] = {d_x_ + s.desc.p_off, d_v_ + s.desc.p_off};
-    float *dsts[2] = {x, v};
-    for (int k = 0; k < 2; ++k) {
-        if (!dsts[k]) continue;
-        if (dst_dev) {
-            launch_f4_to_aos3(srcs[k], dsts[k], n, st);
-            CK(cudaGetLastError());
-        } else {
-            launch_f4_to_aos3(srcs[k], stage, n, st);
-            CK(cudaGetLastError());
-            CK(cudaMemcpyAsync(dsts[k], stage, 12ull * n, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-        }
+    const float4 *sx = d_x_ + s.desc.p_off, *sv = d_v_ + s.desc.p_off;
+    if (dst_dev) {
+        launch_store_phase(sx, sv, x, v, n, st);
+        CK(cudaGetLastError());
+        return PBF_SUCCESS;
     }
+    // the scene's slices of xs and pa are free between steps
+    float *stx = reinterpret_cast<float *>(d_xs_ + s.desc.p_off), *stv = reinterpret_cast<float *>(d_pa_ + s.desc.p_off);
+    launch_store_phase(sx, sv, x ? stx : nullptr, v ? stv : nullptr, n, st);
+    CK(cudaGetLastError());
+    if (x) CK(cudaMemcpyAsync(x, stx, 12ull * n, cudaMemcpyDeviceToHost, st));
+    if (v) CK(cudaMemcpyAsync(v, stv, 12ull * n, cudaMemcpyDeviceToHost, st));
+    if (x || v) CK(cudaStreamSynchronize(st));
     return PBF_SUCCESS;
 }
 
@@ -1154,7 +1147,7 @@ pbf_status Batch::export_x_device(uint32_t id, float *x_dev, cudaStream_t st)
     uint32_t n = 0;
     pbf_status rc = get_num(id, &n, st);
     if (rc != PBF_SUCCESS) return rc;
-    launch_f4_to_aos3(d_x_ + scenes_[id].desc.p_off, x_dev, n, st);
+    launch_store_phase(d_x_ + scenes_[id].desc.p_off, nullptr, x_dev, nullptr, n, st);
     CK(cudaGetLastError());
     return PBF_SUCCESS;
 }

@@ -141,14 +141,15 @@ struct LaunchShape {
     uint32_t grid_cells;  // grid of k_rank_cells: a block of cell_tile threads per cell tile
     uint32_t cell_tile;   // cells per cell tile = threads per k_rank_cells block (autotuned)
     uint32_t small;       // latency-bound step (at most kSmallStep particle slots): split
-                          // neighbour walk, per-particle rank, lambda kept in its own array
+                          // neighbour walk, per-particle rank, wide list reads
     uint32_t grid_split;  // grid of k_neighbors_split (blocks of 256 threads, 256 / kSplit particles each)
+    uint32_t grid_small;  // grid of the small steps' list passes (blocks of kSmallBlock particles)
     uint32_t nb_smem;     // k_neighbors_lambda: bytes of shared memory for the block's lists (0 = stored directly)
     bool operator==(const LaunchShape &o) const
     {
         return tile == o.tile && grid == o.grid && scan_grid == o.scan_grid && scan_rounds == o.scan_rounds && scan_cluster == o.scan_cluster &&
                chunk == o.chunk &&
-               grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && grid_split == o.grid_split && nb_smem == o.nb_smem &&
+               grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && grid_split == o.grid_split && grid_small == o.grid_small && nb_smem == o.nb_smem &&
                grid_nb == o.grid_nb && grid_lambda == o.grid_lambda && grid_dp == o.grid_dp &&
                grid_omega[0] == o.grid_omega[0] && grid_omega[1] == o.grid_omega[1] && grid_apply[0] == o.grid_apply[0] &&
                grid_apply[1] == o.grid_apply[1] && grid_xsph[0] == o.grid_xsph[0] && grid_xsph[1] == o.grid_xsph[1];
@@ -190,14 +191,18 @@ void launch_set_packed_in(PackedIn *dst, const float *x, const float *v, cudaStr
 
 // Edge conversions between the ABI's AoS float3 and the internal float4.
 void launch_aos3_to_f4(const float *src, float4 *dst, uint32_t n, cudaStream_t st);
-void launch_f4_to_aos3(const float4 *src, float *dst, uint32_t n, cudaStream_t st);
+// A scene's upload: n particles widened at x, v and numbered (append: from
+// *next_id on, which the caller then bumps), *scene_num = total.
+void launch_load_phase(const float *sx, const float *sv, float4 *x, float4 *v, uint32_t *id, uint32_t *next_id,
+                       uint32_t *scene_num, uint32_t n, uint32_t total, bool append, cudaStream_t st);
+void launch_store_phase(const float4 *x, const float4 *v, float *dx, float *dv, uint32_t n, cudaStream_t st);
 void launch_set_u32(uint32_t *dst, uint32_t value, cudaStream_t st);
 // pack_off[active[k]] = sum of the live counts of active[0..k), counts[k] =
 // the live count of active[k], computed on the device (one block)
 void launch_pack_offsets(const uint32_t *active, uint32_t n_active, const uint32_t *scene_num, uint32_t *pack_off,
                          uint32_t *counts, cudaStream_t st);
-// ids of n particles added at dst: append ? *next_id + k : k; *next_id += / = n.
-void launch_assign_ids(uint32_t *dst, uint32_t *next_id, uint32_t n, bool append, cudaStream_t st);
+// *next_id += n (an append's ids are handed out)
+void launch_bump_next_id(uint32_t *next_id, uint32_t n, cudaStream_t st);
 // Whole-batch moves between a packed AoS float3 buffer (active scenes in
 // slot order, pack_off[s] = first packed particle of scene s) and the
 // scene-sliced float4 phase arrays.  unpack uses the tile list (counts must
@@ -218,6 +223,7 @@ constexpr uint32_t kBlockScanMax = 8192;      // cells up to which one block sca
 constexpr uint32_t kScanClusterMax = 16;      // blocks of the scan's cluster (1024 threads each)
 constexpr uint32_t kScanRoundsMax = 18;       // cells a thread of it may hold: tables are 2^k + 1 cells, up to 2^18 + 1
 constexpr uint32_t kNbSmemMax = 96 * 1024;  // shared-memory budget for a k_neighbors_lambda block's lists
+constexpr uint32_t kSmallBlock = 64;        // threads of a block of the small steps' list passes
 constexpr uint32_t kSplit = 4;  // small steps: lanes per particle in the split neighbour walk (blocks of 256)
 constexpr uint32_t kCellTile = 256;         // default cells per cell tile = threads per k_rank_cells block
 constexpr uint32_t kCellTileMin = 64, kCellTileMax = 512;  // the autotuner's range

@@ -185,6 +185,14 @@ struct LamSum {
     }
 };
 
+// A pair past the list's end adds exactly nothing: its W, s and s r are 0
+// (its difference is finite: small steps pad with the particle itself, whose
+// difference is 0 or, for a non-finite position, NaN, as all its sums are).
+__device__ __forceinline__ PairWS masked(const PairWS &k, bool on)
+{
+    return PairWS{on ? k.W : 0.f, on ? k.s : 0.f, on ? k.sr : 0.f};
+}
+
 // one listed pair's terms of the lambda sums
 __device__ __forceinline__ void lam_add(LamSum &ls, float4 xi, float4 xj, const PairConst &c)
 {
@@ -553,6 +561,57 @@ __device__ __forceinline__ void list_walk_any(bool l16, const uint32_t *__restri
     else
         list_walk<CH>(nl, stride, nn, f);
 }
+
+// Small, latency-bound steps: a pass's time is one thread's chain of dependent
+// loads, so the list is read 32 slots at a time (all their rows at once) and
+// the neighbours' records 16 at a time, instead of one row and 8 (and the
+// last, partial row's one by one): lambda at 4,096 particles SMOLD us, SMNEW
+// (both alone, cold).  ld(q) loads the record of slot base + q, use(record, on)
+// adds it in list order; slots past the count load the particle's own record
+// (self, as q) and are used with on = false.
+template <class LD, class USE>
+__device__ __forceinline__ void list_walk_wide(bool l16, const uint32_t *__restrict__ nl, uint64_t stride, uint32_t nn,
+                                               uint32_t base, uint32_t self, LD &&ld, USE &&use)
+{
+    const uint4 *p = reinterpret_cast<const uint4 *>(nl);
+    for (uint32_t k0 = 0; k0 < nn; k0 += 32) {
+        uint32_t q[32];
+        if (l16) {
+            uint4 r[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) r[j] = k0 + 8 * j < nn ? list_ld(p + (uint64_t)(k0 / 8 + j) * stride) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (uint32_t c = 0; c < 32; ++c) q[c] = base + oct_at(r[c / 8], c % 8);
+        } else {
+            uint4 r[8];
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) r[j] = k0 + 4 * j < nn ? list_ld(p + (uint64_t)(k0 / 4 + j) * stride) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (uint32_t c = 0; c < 32; ++c) q[c] = quad_at(r[c / 4], c % 4);
+        }
+#pragma unroll
+        for (uint32_t h = 0; h < 32; h += 16) {
+            if (k0 + h < nn) {
+                decltype(ld(0u)) rec[16];
+#pragma unroll
+                for (uint32_t c = 0; c < 16; ++c) rec[c] = ld(k0 + h + c < nn ? q[h + c] : self);
+#pragma unroll
+                for (uint32_t c = 0; c < 16; ++c) use(rec[c], k0 + h + c < nn);
+            }
+        }
+    }
+}
+
+// Small steps' blocks: kSmallBlock threads, tile / kSmallBlock of them a tile,
+// so that few particles spread over many SMs.
+#define SMALL_LOOP_BEGIN                                                      \
+    const uint32_t parts_ = tile / kSmallBlock;                               \
+    const uint32_t n_work_ = a.ctrl->n_tiles * parts_;                        \
+    for (uint32_t u_ = blockIdx.x; u_ < n_work_; u_ += gridDim.x) {           \
+        const uint32_t t_ = u_ / parts_;                                      \
+        const uint32_t s = __ldg(a.tile_scene + t_);                          \
+        const uint32_t local = __ldg(a.tile_start + t_) + (u_ % parts_) * kSmallBlock + threadIdx.x;
+#define SMALL_LOOP_END }
 
 // Per-tile prologue shared by the particle kernels.
 #define TILE_LOOP_BEGIN                                                   \
@@ -1478,7 +1537,7 @@ __global__ void __launch_bounds__(256) k_neighbors_split(StepArgs a, uint32_t ti
         if (sub == 0) {
             a.nnb[i] = (uint8_t)nn;
             a.selfat[i] = listed ? (uint8_t)gself : kNotListed;
-            a.lam[i] = ls.lambda(d);
+            a.xb[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));  // the first delta-p pass gathers both
         }
     }
 }
@@ -1487,7 +1546,7 @@ __global__ void __launch_bounds__(256) k_neighbors_split(StepArgs a, uint32_t ti
 // pbf_kernel_memorization.cu:93-134 and pbf_constraint.cu:168-209, without the
 // per-pair cache: W and grad W are recomputed from positions).  One thread
 // per particle; the neighbour sums run in list order.
-template <int kChunk, bool LAMW>
+template <int kChunk>
 __global__ void __launch_bounds__(512, 2) k_lambda(StepArgs a, float4 *__restrict__ xc)
 {
     TILE_LOOP_BEGIN
@@ -1502,16 +1561,36 @@ __global__ void __launch_bounds__(512, 2) k_lambda(StepArgs a, float4 *__restric
     if (a.selfat[i] != kNotListed) ls.ks = 1.f;  // the particle's own w(0), not stored in the list
     list_walk_any<kChunk>(d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off,
                           [&](uint32_t q) { lam_add(ls, xp, __ldg(xc + q), pc); });
-    // LAMW: lambda rides in .w of the positions this pass reads and the
-    // delta-p pass gathers next (neighbours here use only .xyz); small,
-    // latency-bound steps keep it in its own array, as the store into the
-    // gathered array slows this pass's neighbour reads there
-    const float lam = ls.lambda(d);
-    if (LAMW)
-        reinterpret_cast<float *>(xc + i)[3] = lam;
-    else
-        a.lam[i] = lam;
+    // lambda rides in .w of the positions this pass reads and the delta-p
+    // pass gathers next (neighbours here use only .xyz)
+    reinterpret_cast<float *>(xc + i)[3] = ls.lambda(d);
     TILE_LOOP_END
+}
+
+// Small steps: (position, lambda) into the other buffer, which the delta-p
+// pass gathers.
+__global__ void __launch_bounds__(kSmallBlock, 8) k_lambda_small(StepArgs a, uint32_t tile,
+                                                                 const float4 *__restrict__ xc,
+                                                                 float4 *__restrict__ xo)
+{
+    SMALL_LOOP_BEGIN
+    const SceneDesc d = a.scenes[s];
+    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
+    if (local >= live) continue;
+    const uint32_t i = d.p_off + local;
+    const PairConst pc = pair_const(d);
+    const float4 xp = xc[i];
+    LamSum ls;
+    if (a.selfat[i] != kNotListed) ls.ks = 1.f;
+    list_walk_wide(
+        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        [&](uint32_t q) -> float4 { return __ldg(xc + q); },
+        [&](const float4 &xj, bool on) {
+            const PairGeo g = pair_geo(xp, xj);
+            ls.add(g, masked(pair_ws(g.r2, pc), on));
+        });
+    xo[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));
+    SMALL_LOOP_END
 }
 
 // s_corr forms, selected once per tile (a tile belongs to one scene).
@@ -1555,26 +1634,6 @@ __device__ __forceinline__ ScorrConst scorr_const(const SceneDesc &d, float li)
     c.c = d.tensile_mode == PBF_TENSILE_REFERENCE ? d.tens_c : d.scorr_c;
     c.sn = d.scorr_n;
     return c;
-}
-
-// One pair's share of the sum of -(lambda_i + lambda_j + s_corr) grad W (the
-// body of calcPositionUpdateCUDA, pbf_position_update.cu:131-188): adds
-// (coefficient * s) d.  PK: the x and y differences and sums by one packed
-// operation each (the same bits; measured faster in large steps only).
-template <int FORM, bool PK>
-__device__ __forceinline__ void dp_add(float3 &sum, float4 xp, float4 xq, float li, float lj, const PairConst &pc,
-                                       const ScorrConst &sc)
-{
-    const PairGeo g = pair_geo<PK>(xp, xq);
-    const PairWS k = pair_ws(g.r2, pc);
-    const float f = __fmul_rn(dp_coef<FORM>(li, lj, k.W, sc), k.s);
-    if (PK) {
-        fma2(sum.x, sum.y, f, f, g.d0, g.d1);
-    } else {
-        sum.x = __fmaf_rn(f, g.d0, sum.x);
-        sum.y = __fmaf_rn(f, g.d1, sum.y);
-    }
-    sum.z = __fmaf_rn(f, g.d2, sum.z);
 }
 
 // Where a step's velocity goes after a stage, by the scene's next stage: the
@@ -1626,7 +1685,12 @@ __device__ __forceinline__ void dp_finish(const StepArgs &a, const SceneDesc &d,
         xo[i] = xn;
 }
 
-// Sum over the list, in list order.  LAMW: lambda in .w of the positions.
+// Sum over the list of -(lambda_i + lambda_j + s_corr) grad W (the body of
+// calcPositionUpdateCUDA, pbf_position_update.cu:131-188), in list order:
+// each pair adds (coefficient * s) d.  LAMW: lambda in .w of the positions
+// (iterations >= 1 of large steps; their iteration 0 reads it from lam), and
+// the x and y differences and sums by one packed operation each (the same
+// bits; measured faster there only).
 template <int kChunk, int FORM, bool LAMW>
 __device__ __forceinline__ float3 dp_sum(const StepArgs &a, const SceneDesc &d, const float4 *__restrict__ xc,
                                          uint32_t i, float4 xp, float li)
@@ -1634,12 +1698,32 @@ __device__ __forceinline__ float3 dp_sum(const StepArgs &a, const SceneDesc &d, 
     const PairConst pc = pair_const(d);
     const ScorrConst sc = scorr_const(d, li);
     const float *__restrict__ lam = a.lam;
-    float3 sum = make_float3(0.f, 0.f, 0.f);
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
     list_walk_any<kChunk>(d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, [&](uint32_t q) {
         const float4 xq = __ldg(xc + q);
-        dp_add<FORM, LAMW>(sum, xp, xq, li, LAMW ? xq.w : __ldg(lam + q), pc, sc);
+        const PairGeo g = pair_geo<LAMW>(xp, xq);
+        const PairWS k = pair_ws(g.r2, pc);
+        const float lj = LAMW ? xq.w : __ldg(lam + q);
+        const float f = __fmul_rn(dp_coef<FORM>(li, lj, k.W, sc), k.s);
+        if (LAMW) {
+            fma2(s0, s1, f, f, g.d0, g.d1);
+        } else {
+            s0 = __fmaf_rn(f, g.d0, s0);
+            s1 = __fmaf_rn(f, g.d1, s1);
+        }
+        s2 = __fmaf_rn(f, g.d2, s2);
     });
-    return sum;
+    return make_float3(s0, s1, s2);
+}
+
+// The s_corr form once per tile (a tile belongs to one scene): f<FORM>().
+template <class F>
+__device__ __forceinline__ float3 by_scorr(const SceneDesc &d, F &&f)
+{
+    if (d.tensile_mode == PBF_TENSILE_REFERENCE) return f(std::integral_constant<int, kScorrReference>());
+    if (d.tensile_mode == PBF_TENSILE_TEXTBOOK && d.scorr_n == 4) return f(std::integral_constant<int, kScorrTextbook4>());
+    if (d.tensile_mode == PBF_TENSILE_TEXTBOOK) return f(std::integral_constant<int, kScorrTextbook>());
+    return f(std::integral_constant<int, kScorrOff>());
 }
 
 // delta-p with s_corr (calcPositionUpdateCUDA cached, pbf_position_update.cu:131-188).
@@ -1656,17 +1740,42 @@ __global__ void __launch_bounds__(512, 2) k_dp(StepArgs a, const float4 *__restr
     const uint32_t i = d.p_off + local;
     const float4 xp = xc[i];
     const float li = LAMW ? xp.w : a.lam[i];
-    float3 sum;
-    if (d.tensile_mode == PBF_TENSILE_REFERENCE)
-        sum = dp_sum<kChunk, kScorrReference, LAMW>(a, d, xc, i, xp, li);
-    else if (d.tensile_mode == PBF_TENSILE_TEXTBOOK && d.scorr_n == 4)
-        sum = dp_sum<kChunk, kScorrTextbook4, LAMW>(a, d, xc, i, xp, li);
-    else if (d.tensile_mode == PBF_TENSILE_TEXTBOOK)
-        sum = dp_sum<kChunk, kScorrTextbook, LAMW>(a, d, xc, i, xp, li);
-    else
-        sum = dp_sum<kChunk, kScorrOff, LAMW>(a, d, xc, i, xp, li);
+    const float3 sum = by_scorr(d, [&](auto form) { return dp_sum<kChunk, decltype(form)::value, LAMW>(a, d, xc, i, xp, li); });
     dp_finish(a, d, s, i, xp, sum, xo, last);
     TILE_LOOP_END
+}
+
+// Small steps: (position, lambda) gathered together.
+__global__ void __launch_bounds__(kSmallBlock, 8) k_dp_small(StepArgs a, uint32_t tile, const float4 *__restrict__ xc,
+                                                             float4 *__restrict__ xo, int last)
+{
+    SMALL_LOOP_BEGIN
+    const SceneDesc d = a.scenes[s];
+    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
+    if (last && local == 0) a.scene_num[s] = live;
+    if (local >= live) continue;
+    const uint32_t i = d.p_off + local;
+    const float4 xp = xc[i];
+    const PairConst pc = pair_const(d);
+    const ScorrConst sc = scorr_const(d, xp.w);
+    const float3 sum = by_scorr(d, [&](auto form) {
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+        list_walk_wide(
+            d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+            [&](uint32_t q) -> float4 { return __ldg(xc + q); },
+            [&](const float4 &xq, bool on) {
+                const PairGeo g = pair_geo(xp, xq);
+                const PairWS k = pair_ws(g.r2, pc);
+                const float f0 = __fmul_rn(dp_coef<decltype(form)::value>(xp.w, xq.w, k.W, sc), k.s);
+                const float f = on ? f0 : 0.f;
+                s0 = __fmaf_rn(f, g.d0, s0);
+                s1 = __fmaf_rn(f, g.d1, s1);
+                s2 = __fmaf_rn(f, g.d2, s2);
+            });
+        return make_float3(s0, s1, s2);
+    });
+    dp_finish(a, d, s, i, xp, sum, xo, last);
+    SMALL_LOOP_END
 }
 
 // iters == 0: positions stay at the prediction; v from the velocity update.
@@ -1690,11 +1799,11 @@ struct OmegaSum {
     float4 xi, vi;
     float kh, w0 = 0.f, w1 = 0.f, w2 = 0.f;
     __device__ __forceinline__ OmegaSum(float4 x, float4 v, float k) : xi(x), vi(v), kh(k) {}
-    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz)
+    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz, bool on = true)
     {
         const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
         const float r2 = p0 * p0 + p1 * p1 + p2 * p2;
-        if (r2 > 0.f) {
+        if (on && r2 > 0.f) {
             const float inv_r = rsqrtf(r2);
             const float v0 = vx - vi.x, v1 = vy - vi.y, v2 = vz - vi.z;
             const float wd = wspiky_d(r2 * inv_r, kh) * inv_r;
@@ -1743,6 +1852,33 @@ __global__ void __launch_bounds__(512) k_vort_omega(StepArgs a)
     TILE_LOOP_END
 }
 
+// A neighbour's (x, v) as the small steps' passes load it.
+struct PhaseRec {
+    float4 A;
+    float2 B;
+};
+
+__global__ void __launch_bounds__(kSmallBlock, 8) k_vort_omega_small(StepArgs a, uint32_t tile)
+{
+    SMALL_LOOP_BEGIN
+    const SceneDesc d = a.scenes[s];
+    if (d.vort_mode != PBF_VORTICITY_TEXTBOOK) continue;
+    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
+    if (local >= live) continue;
+    const uint32_t i = d.p_off + local;
+    const float4 *__restrict__ pa = a.pa;
+    const float2 *__restrict__ pb = a.pb;
+    const float4 A = pa[i];
+    const float2 B = pb[i];
+    OmegaSum o(A, make_float4(A.w, B.x, B.y, 0.f), d.inv_h);
+    list_walk_wide(
+        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; },
+        [&](const PhaseRec &r, bool on) { o.add(r.A, r.A.w, r.B.x, r.B.y, on); });
+    put_omega(a, d, i, o);
+    SMALL_LOOP_END
+}
+
 // The reference's uncapped 27-cell walk over final positions in sorted order,
 // with h passed where 1/h is expected (pbf_vorticity_confinement.cu:28).
 __global__ void __launch_bounds__(512) k_vort_omega_walk(StepArgs a)
@@ -1780,11 +1916,11 @@ struct EtaSum {
     float4 xi;
     float kh, sgn, n0 = 0.f, n1 = 0.f, n2 = 0.f;
     __device__ __forceinline__ EtaSum(float4 x, float k, float sg) : xi(x), kh(k), sgn(sg) {}
-    __device__ __forceinline__ void add(float4 xj)  // (x_j, |omega_j|)
+    __device__ __forceinline__ void add(float4 xj, bool on = true)  // (x_j, |omega_j|)
     {
         const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
         const float r2 = p0 * p0 + p1 * p1 + p2 * p2;
-        if (r2 > 0.f) {
+        if (on && r2 > 0.f) {
             const float inv_r = rsqrtf(r2);
             const float f = sgn * xj.w * wspiky_d(r2 * inv_r, kh) * inv_r;
             n0 += f * p0;
@@ -1831,6 +1967,23 @@ __global__ void __launch_bounds__(512) k_vort_apply(StepArgs a)
     list_walk_any<4>(L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], 0u, [&](uint32_t q) { e.add(__ldg(xw + q)); });
     put_confinement(a, d, i, e);
     TILE_LOOP_END
+}
+
+__global__ void __launch_bounds__(kSmallBlock, 8) k_vort_apply_small(StepArgs a, uint32_t tile)
+{
+    SMALL_LOOP_BEGIN
+    const SceneDesc d = a.scenes[s];
+    if (d.vort_mode != PBF_VORTICITY_TEXTBOOK) continue;
+    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
+    if (local >= live) continue;
+    const uint32_t i = d.p_off + local;
+    const float4 *__restrict__ xw = a.xs;
+    EtaSum e(xw[i], d.inv_h, -1.f);
+    list_walk_wide(
+        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        [&](uint32_t q) -> float4 { return __ldg(xw + q); }, [&](const float4 &xj, bool on) { e.add(xj, on); });
+    put_confinement(a, d, i, e);
+    SMALL_LOOP_END
 }
 
 // The reference's form (sorted order throughout; the XSPH list form that may
@@ -1886,14 +2039,14 @@ struct XsphSum {
         : xi(x), vi(v), ih2(d.inv_h * d.inv_h), alpha6(d.alpha6)
     {
     }
-    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz)
+    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz, bool on = true)
     {
         const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
         // Wpoly6 from r^2 (q^2 = r^2 / h^2 instead of (|r| / h)^2: no square
         // root per pair; the two differ by rounding only)
         const float q2 = (p0 * p0 + p1 * p1 + p2 * p2) * ih2;
         const float t = 1.f - q2;
-        const float W = (q2 <= 1.f) ? alpha6 * t * t * t : 0.f;
+        const float W = (on && q2 <= 1.f) ? alpha6 * t * t * t : 0.f;
         s0 += (vx - vi.x) * W;
         s1 += (vy - vi.y) * W;
         s2 += (vz - vi.z) * W;
@@ -1933,6 +2086,27 @@ __global__ void __launch_bounds__(512) k_xsph(StepArgs a)
     });
     a.v[__float_as_uint(a.xold[i].w)] = o.result(d);
     TILE_LOOP_END
+}
+
+__global__ void __launch_bounds__(kSmallBlock, 8) k_xsph_small(StepArgs a, uint32_t tile)
+{
+    SMALL_LOOP_BEGIN
+    const SceneDesc d = a.scenes[s];
+    if (d.xsph_mode != PBF_XSPH_LIST) continue;
+    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
+    if (local >= live) continue;
+    const uint32_t i = d.p_off + local;
+    const float4 *__restrict__ pa = a.pa;
+    const float2 *__restrict__ pb = a.pb;
+    const float4 A = pa[i];
+    const float2 B = pb[i];
+    XsphSum o(A, make_float4(A.w, B.x, B.y, 0.f), d);
+    list_walk_wide(
+        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; },
+        [&](const PhaseRec &r, bool on) { o.add(r.A, r.A.w, r.B.x, r.B.y, on); });
+    a.v[__float_as_uint(a.xold[i].w)] = o.result(d);
+    SMALL_LOOP_END
 }
 
 // The reference's uncapped 27-cell walk (scenes with PBF_XSPH_WALK), sorted
@@ -2047,30 +2221,58 @@ __global__ void k_aos3_to_f4(const float *__restrict__ src, float4 *__restrict__
     if (i < n) dst[i] = make_float4(src[3 * i], src[3 * i + 1], src[3 * i + 2], 0.f);
 }
 
-__global__ void k_f4_to_aos3(const float4 *__restrict__ src, float *__restrict__ dst, uint32_t n)
+// A scene's n uploaded particles widened into the phase and numbered, and the
+// scene's counters, in one launch: five small launches (x, v, ids, two
+// counters) took SETOLD us for 4,096 particles, this one SETNEW.  next_id:
+// null for an append, whose ids continue from *id0 (bumped by a launch of its
+// own: other blocks may not have read it yet).
+__global__ void k_load_phase(const float *__restrict__ sx, const float *__restrict__ sv, float4 *__restrict__ x,
+                             float4 *__restrict__ v, uint32_t *__restrict__ id, const uint32_t *id0, uint32_t *next_id,
+                             uint32_t *scene_num, uint32_t n, uint32_t total)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        const float4 v = src[i];
-        dst[3 * i] = v.x;
-        dst[3 * i + 1] = v.y;
-        dst[3 * i + 2] = v.z;
+    if (i == 0) {
+        *scene_num = total;
+        if (next_id) *next_id = n;
+    }
+    if (i >= n) return;
+    const uint32_t first = next_id ? 0u : *id0;
+    x[i] = make_float4(sx[3 * i], sx[3 * i + 1], sx[3 * i + 2], 0.f);
+    v[i] = sv ? make_float4(sv[3 * i], sv[3 * i + 1], sv[3 * i + 2], 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+    id[i] = first + i;
+}
+
+// Either or both of x, v narrowed for the caller.
+__global__ void k_store_phase(const float4 *__restrict__ x, const float4 *__restrict__ v, float *__restrict__ dx,
+                              float *__restrict__ dv, uint32_t n)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (dx) {
+        const float4 t = x[i];
+        dx[3 * i] = t.x;
+        dx[3 * i + 1] = t.y;
+        dx[3 * i + 2] = t.z;
+    }
+    if (dv) {
+        const float4 t = v[i];
+        dv[3 * i] = t.x;
+        dv[3 * i + 1] = t.y;
+        dv[3 * i + 2] = t.z;
     }
 }
 
 }  // namespace
 
-// The lambda / delta-p variants by neighbour chunk, selected at run time.
+// The large steps' lambda / delta-p variants by neighbour chunk, selected at
+// run time.
 template <int CH>
 struct PassFns {
-    static const void *lambda() { return (const void *)k_lambda<CH, true>; }
+    static const void *lambda() { return (const void *)k_lambda<CH>; }
     static const void *dp() { return (const void *)k_dp<CH, true>; }
-    static void launch_lambda(const StepArgs &a, const LaunchShape &sh, float4 *cur, bool lamw, cudaStream_t st)
+    static void launch_lambda(const StepArgs &a, const LaunchShape &sh, float4 *cur, cudaStream_t st)
     {
-        if (lamw)
-            k_lambda<CH, true><<<sh.grid_lambda, sh.tile, 0, st>>>(a, cur);
-        else
-            k_lambda<CH, false><<<sh.grid_lambda, sh.tile, 0, st>>>(a, cur);
+        k_lambda<CH><<<sh.grid_lambda, sh.tile, 0, st>>>(a, cur);
     }
     // lamw: lambda in .w of cur (iterations >= 1); iteration 0 reads it from lam
     static void launch_dp(const StepArgs &a, const LaunchShape &sh, const float4 *cur, float4 *out, int last,
@@ -2138,9 +2340,16 @@ void launch_aos3_to_f4(const float *src, float4 *dst, uint32_t n, cudaStream_t s
     if (n) k_aos3_to_f4<<<(n + 255) / 256, 256, 0, st>>>(src, dst, n);
 }
 
-void launch_f4_to_aos3(const float4 *src, float *dst, uint32_t n, cudaStream_t st)
+void launch_load_phase(const float *sx, const float *sv, float4 *x, float4 *v, uint32_t *id, uint32_t *next_id,
+                       uint32_t *scene_num, uint32_t n, uint32_t total, bool append, cudaStream_t st)
 {
-    if (n) k_f4_to_aos3<<<(n + 255) / 256, 256, 0, st>>>(src, dst, n);
+    k_load_phase<<<n ? (n + 255) / 256 : 1, 256, 0, st>>>(sx, sv, x, v, id, next_id, append ? nullptr : next_id,
+                                                          scene_num, n, total);
+}
+
+void launch_store_phase(const float4 *x, const float4 *v, float *dx, float *dv, uint32_t n, cudaStream_t st)
+{
+    if (n) k_store_phase<<<(n + 255) / 256, 256, 0, st>>>(x, v, dx, dv, n);
 }
 
 void launch_set_u32(uint32_t *dst, uint32_t value, cudaStream_t st) { k_set_u32<<<1, 1, 0, st>>>(dst, value); }
@@ -2288,30 +2497,47 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
             k_neighbors_lambda<false><<<sh.grid_nb, b, 0, st>>>(a);
         PBF_LAUNCHED("k_neighbors_lambda");
     }
-    float4 *cur = a.xa, *nxt = a.xb;
-    for (int it = 0; it < iters; ++it) {
-        if (it > 0) {
-            PBF_PASS_DISPATCH(sh.chunk, launch_lambda(a, sh, cur, !sh.small, st));
-            PBF_LAUNCHED("k_lambda");
+    if (sh.small) {  // (position, lambda) in xb, positions in xa
+        const uint32_t gs = sh.grid_small;
+        for (int it = 0; it < iters; ++it) {
+            if (it > 0) {
+                k_lambda_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile, a.xa, a.xb);
+                PBF_LAUNCHED("k_lambda");
+            }
+            k_dp_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile, a.xb, a.xa, it == iters - 1 ? 1 : 0);
+            PBF_LAUNCHED("k_dp");
         }
-        PBF_PASS_DISPATCH(sh.chunk, launch_dp(a, sh, cur, nxt, it == iters - 1 ? 1 : 0, it > 0 && !sh.small, st));
-        PBF_LAUNCHED("k_dp");
-        std::swap(cur, nxt);
+    } else {
+        float4 *cur = a.xa, *nxt = a.xb;
+        for (int it = 0; it < iters; ++it) {
+            if (it > 0) {
+                PBF_PASS_DISPATCH(sh.chunk, launch_lambda(a, sh, cur, st));
+                PBF_LAUNCHED("k_lambda");
+            }
+            PBF_PASS_DISPATCH(sh.chunk, launch_dp(a, sh, cur, nxt, it == iters - 1 ? 1 : 0, it > 0, st));
+            PBF_LAUNCHED("k_dp");
+            std::swap(cur, nxt);
+        }
     }
     if (iters <= 0) {
         k_finalize<<<g, b, 0, st>>>(a);
         PBF_LAUNCHED("k_finalize");
     }
-    // the list forms run one instance per list format present
+    // the list forms: one instance per list format present, or the small steps'
     const bool l16 = (post & kPostList16) != 0, l32 = (post & kPostList32) != 0;
-#define PBF_POST(kernel, grid)                   \
-    if (l32) {                                   \
-        kernel<false><<<grid[0], b, 0, st>>>(a); \
-        PBF_LAUNCHED(#kernel);                   \
-    }                                            \
-    if (l16) {                                   \
-        kernel<true><<<grid[1], b, 0, st>>>(a);  \
-        PBF_LAUNCHED(#kernel);                   \
+#define PBF_POST(kernel, grid)                                               \
+    if (sh.small) {                                                          \
+        kernel##_small<<<sh.grid_small, kSmallBlock, 0, st>>>(a, sh.tile);   \
+        PBF_LAUNCHED(#kernel);                                               \
+    } else {                                                                 \
+        if (l32) {                                                           \
+            kernel<false><<<grid[0], b, 0, st>>>(a);                         \
+            PBF_LAUNCHED(#kernel);                                           \
+        }                                                                    \
+        if (l16) {                                                           \
+            kernel<true><<<grid[1], b, 0, st>>>(a);                          \
+            PBF_LAUNCHED(#kernel);                                           \
+        }                                                                    \
     }
     if (post & kPostVortTextbook) {
         PBF_POST(k_vort_omega, sh.grid_omega)

@@ -273,26 +273,13 @@ __global__ void k_scatter_by_index(const float4 *__restrict__ x, const float4 *_
     }
 }
 
-__global__ void k_assign_ids(uint32_t *dst, const uint32_t *next_id, uint32_t n, int append)
-{
-    const uint32_t id0 = append ? *next_id : 0u;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) dst[k] = id0 + k;
-}
-
-__global__ void k_bump_next_id(uint32_t *next_id, uint32_t n, int append)
-{
-    *next_id = (append ? *next_id : 0u) + n;
-}
+__global__ void k_bump_next_id(uint32_t *next_id, uint32_t n) { *next_id += n; }
 
 uint32_t blocks_for(uint64_t n) { return (uint32_t)std::min<uint64_t>((n + 255) / 256, 4096); }
 
 }  // namespace
 
-void launch_assign_ids(uint32_t *dst, uint32_t *next_id, uint32_t n, bool append, cudaStream_t st)
-{
-    if (n) k_assign_ids<<<blocks_for(n), 256, 0, st>>>(dst, next_id, n, append ? 1 : 0);
-    k_bump_next_id<<<1, 1, 0, st>>>(next_id, n, append ? 1 : 0);
-}
+void launch_bump_next_id(uint32_t *next_id, uint32_t n, cudaStream_t st) { k_bump_next_id<<<1, 1, 0, st>>>(next_id, n); }
 
 // ------------------------------------------------------ batch methods --
 
