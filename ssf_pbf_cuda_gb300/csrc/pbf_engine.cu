@@ -189,7 +189,7 @@ Batch::~Batch()
     if (small_done_) cudaEventDestroy(small_done_);
     if (h_small_) cudaFreeHost(h_small_);
     void *ptrs[] = {d_scenes_, d_tile_scene_, d_tile_start_, d_ctrl_, d_scene_num_, d_flags_, d_x_, d_v_,
-                    d_xs_, d_xa_, d_xb_, d_xold_, d_w_, d_pa_, d_pb_, d_vs_, d_key_, d_slot_, d_tmp_, d_perm_, d_count_,
+                    d_xs_, d_xa_, d_xb_, d_xold_, d_w_, d_pa_, d_pb_, d_vs_, d_tile_hdr_, d_key_, d_slot_, d_tmp_, d_perm_, d_count_,
                     d_offsets_, d_bsum_, d_lam_, d_nbr_, d_nnb_, d_self_, d_bnd_, d_pack_off_, d_active_, d_id_, d_id_tmp_,
                     d_next_id_, d_cls_, d_chist_, d_wpos_, d_dense_, d_mid_};
     for (void *p : ptrs)
@@ -232,6 +232,7 @@ pbf_status Batch::init(uint32_t max_scenes, uint64_t max_particles, uint64_t max
     // four and may read up to three past the end of a range (never accepted)
     for (float4 **p : f4) CK(A((void **)p, 16 * (P + kWalkSpare)));
     CK(A((void **)&d_pb_, 8 * (P + kWalkSpare)));
+    CK(A((void **)&d_tile_hdr_, 16 * kSmallTiles));
     uint32_t **u4[] = {&d_key_, &d_slot_, &d_tmp_, &d_perm_, &d_id_, &d_id_tmp_, &d_wpos_};
     for (uint32_t **p : u4) CK(A((void **)p, 4 * P));
     CK(A((void **)&d_count_, 4 * (C + 4)));
@@ -772,9 +773,8 @@ LaunchShape Batch::shape_for(uint32_t tile) const
     }
     sh.grid_cells = pow2(std::max<uint32_t>(1, ctrl_.n_cell_tiles));  // a block per cell tile
     sh.cell_tile = cell_tile_;
-    sh.small = (uint64_t)nt * tile <= kSmallStep ? 1u : 0u;
-    sh.grid_split = std::min<uint32_t>((uint32_t)sms_ * std::max<uint32_t>(1, o.split), ntb * (tile / (256 / kSplit)));
-    sh.grid_small = ntb * (tile / kSmallBlock);
+    sh.small = (uint64_t)nt * tile <= kSmallStep && scenes_.size() <= (1u << 22) ? 1u : 0u;  // (a header's scene bits)
+    sh.small_tiles = ntb;
     const uint32_t scan_tiles = std::max<uint32_t>(1, (ctrl_.n_cells + kScanTile - 1) / kScanTile);
     sh.scan_grid = std::min<uint32_t>(pow2(scan_tiles), (uint32_t)sms_ * 8);
     {  // the block's lists in shared memory when they fit
@@ -835,6 +835,8 @@ StepArgs Batch::args() const
     a.vs = d_vs_;
     a.bnd = d_bnd_;
     a.nbr_stride = max_particles_;
+    a.nbr_rows = (max_pair_ - 1u + 3u) / 4u;
+    a.tile_hdr = d_tile_hdr_;
     a.pin = d_pin_;
     a.pack_off = d_pack_off_;
     return a;

@@ -145,6 +145,7 @@ private:
     float4 *d_x_ = nullptr, *d_v_ = nullptr, *d_xs_ = nullptr, *d_xa_ = nullptr, *d_xb_ = nullptr,
            *d_xold_ = nullptr, *d_w_ = nullptr, *d_pa_ = nullptr, *d_vs_ = nullptr;
     float2 *d_pb_ = nullptr;
+    uint4 *d_tile_hdr_ = nullptr;                     // small steps' tile headers
     uint32_t *d_key_ = nullptr, *d_slot_ = nullptr, *d_tmp_ = nullptr, *d_perm_ = nullptr;
     uint32_t *d_count_ = nullptr, *d_offsets_ = nullptr, *d_bsum_ = nullptr;
     float *d_lam_ = nullptr;

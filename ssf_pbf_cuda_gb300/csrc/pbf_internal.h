@@ -124,6 +124,8 @@ struct StepArgs {
     uint64_t *chist;              // per cell: 8 x 8-bit class ends of its bucket, or kClassWhole
     uint32_t *next_id;            // per scene: id of the next particle added
     uint64_t nbr_stride;
+    uint32_t nbr_rows;            // 16-byte rows a list has
+    uint4 *tile_hdr;              // small steps: the tiles' headers (SMALL_LOOP_BEGIN)
     const PackedIn *pin;          // packed-input steps: the input buffers
     const uint32_t *pack_off;     // packed-input steps: first packed particle of each scene
 };
@@ -142,14 +144,13 @@ struct LaunchShape {
     uint32_t cell_tile;   // cells per cell tile = threads per k_rank_cells block (autotuned)
     uint32_t small;       // latency-bound step (at most kSmallStep particle slots): split
                           // neighbour walk, per-particle rank, wide list reads
-    uint32_t grid_split;  // grid of k_neighbors_split (blocks of 256 threads, 256 / kSplit particles each)
-    uint32_t grid_small;  // grid of the small steps' list passes (blocks of kSmallBlock particles)
+    uint32_t small_tiles; // small steps: tiles rounded up to a power of two, for which headers are written
     uint32_t nb_smem;     // k_neighbors_lambda: bytes of shared memory for the block's lists (0 = stored directly)
     bool operator==(const LaunchShape &o) const
     {
         return tile == o.tile && grid == o.grid && scan_grid == o.scan_grid && scan_rounds == o.scan_rounds && scan_cluster == o.scan_cluster &&
                chunk == o.chunk &&
-               grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && grid_split == o.grid_split && grid_small == o.grid_small && nb_smem == o.nb_smem &&
+               grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && small_tiles == o.small_tiles && nb_smem == o.nb_smem &&
                grid_nb == o.grid_nb && grid_lambda == o.grid_lambda && grid_dp == o.grid_dp &&
                grid_omega[0] == o.grid_omega[0] && grid_omega[1] == o.grid_omega[1] && grid_apply[0] == o.grid_apply[0] &&
                grid_apply[1] == o.grid_apply[1] && grid_xsph[0] == o.grid_xsph[0] && grid_xsph[1] == o.grid_xsph[1];
@@ -158,7 +159,7 @@ struct LaunchShape {
 
 // Resident blocks per SM of each kernel class at a tile size / chunk.
 struct Occupancy {
-    uint32_t light, nb, lambda, dp, cells, split;
+    uint32_t light, nb, lambda, dp, cells;
     uint32_t omega[2], apply[2], xsph[2];
 };
 Occupancy occupancy(uint32_t tile, uint32_t chunk);
@@ -223,12 +224,14 @@ constexpr uint32_t kBlockScanMax = 8192;      // cells up to which one block sca
 constexpr uint32_t kScanClusterMax = 16;      // blocks of the scan's cluster (1024 threads each)
 constexpr uint32_t kScanRoundsMax = 18;       // cells a thread of it may hold: tables are 2^k + 1 cells, up to 2^18 + 1
 constexpr uint32_t kNbSmemMax = 96 * 1024;  // shared-memory budget for a k_neighbors_lambda block's lists
-constexpr uint32_t kSmallBlock = 64;        // threads of a block of the small steps' list passes
-constexpr uint32_t kSplit = 4;  // small steps: lanes per particle in the split neighbour walk (blocks of 256)
+constexpr uint32_t kSmallStep = 131072;     // particle slots up to which a step is latency bound
+constexpr uint32_t kSmallBlock = 64;        // particles of a block of the small steps' list passes
+constexpr uint32_t kSmallTiles = kSmallStep / 64;  // tiles a small step may have (a power of two)
+constexpr uint32_t kSplit = 4;              // small steps: lanes per particle in the split neighbour walk
+constexpr uint32_t kSplitBlock = kSplit * kSmallBlock;
 constexpr uint32_t kCellTile = 256;         // default cells per cell tile = threads per k_rank_cells block
 constexpr uint32_t kCellTileMin = 64, kCellTileMax = 512;  // the autotuner's range
 constexpr uint32_t kMidMin = 16;            // buckets with more members are queued (warp or block per bucket)
-constexpr uint32_t kSmallStep = 131072;     // particle slots up to which a step is latency bound
 constexpr uint32_t kList16Max = 65536;      // scenes of at most this many slots keep u16 neighbour lists
 constexpr uint8_t kNotListed = 0xFF;        // selfat of a particle the cap cut from its own list
 constexpr uint32_t kWalkSpare = 4;          // spare float4 records after each per-particle array

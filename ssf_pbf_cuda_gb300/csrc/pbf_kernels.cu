@@ -565,27 +565,29 @@ __device__ __forceinline__ void list_walk_any(bool l16, const uint32_t *__restri
 // Small, latency-bound steps: a pass's time is one thread's chain of dependent
 // loads, so the list is read 32 slots at a time (all their rows at once) and
 // the neighbours' records 16 at a time, instead of one row and 8 (and the
-// last, partial row's one by one): lambda at 4,096 particles SMOLD us, SMNEW
-// (both alone, cold).  ld(q) loads the record of slot base + q, use(record, on)
+// last, partial row's one by one): at 4,096 particles (each kernel alone, cold
+// caches) delta-p 10.4 -> 7.8 us, omega 12.0 -> 8.7, its second pass 12.1 ->
+// 9.1.  ld(q) loads the record of slot base + q, use(record, on)
 // adds it in list order; slots past the count load the particle's own record
-// (self, as q) and are used with on = false.
+// (self, as q) and are used with on = false.  rows: 16-byte rows a list has.
 template <class LD, class USE>
-__device__ __forceinline__ void list_walk_wide(bool l16, const uint32_t *__restrict__ nl, uint64_t stride, uint32_t nn,
-                                               uint32_t base, uint32_t self, LD &&ld, USE &&use)
+__device__ __forceinline__ void list_walk_wide(bool l16, const uint32_t *__restrict__ nl, uint64_t stride, uint32_t rows,
+                                               uint32_t nn, uint32_t base, uint32_t self, LD &&ld, USE &&use)
 {
     const uint4 *p = reinterpret_cast<const uint4 *>(nl);
-    for (uint32_t k0 = 0; k0 < nn; k0 += 32) {
+    uint32_t k0 = 0;
+    do {  // the first rows are requested whatever the count, beside it
         uint32_t q[32];
         if (l16) {
             uint4 r[4];
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) r[j] = k0 + 8 * j < nn ? list_ld(p + (uint64_t)(k0 / 8 + j) * stride) : make_uint4(0u, 0u, 0u, 0u);
+            for (uint32_t j = 0; j < 4; ++j) r[j] = k0 / 8 + j < rows ? list_ld(p + (uint64_t)(k0 / 8 + j) * stride) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (uint32_t c = 0; c < 32; ++c) q[c] = base + oct_at(r[c / 8], c % 8);
         } else {
             uint4 r[8];
 #pragma unroll
-            for (uint32_t j = 0; j < 8; ++j) r[j] = k0 + 4 * j < nn ? list_ld(p + (uint64_t)(k0 / 4 + j) * stride) : make_uint4(0u, 0u, 0u, 0u);
+            for (uint32_t j = 0; j < 8; ++j) r[j] = k0 / 4 + j < rows ? list_ld(p + (uint64_t)(k0 / 4 + j) * stride) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (uint32_t c = 0; c < 32; ++c) q[c] = quad_at(r[c / 4], c % 4);
         }
@@ -599,18 +601,25 @@ __device__ __forceinline__ void list_walk_wide(bool l16, const uint32_t *__restr
                 for (uint32_t c = 0; c < 16; ++c) use(rec[c], k0 + h + c < nn);
             }
         }
-    }
+        k0 += 32;
+    } while (k0 < nn);
 }
 
 // Small steps' blocks: kSmallBlock threads, tile / kSmallBlock of them a tile,
-// so that few particles spread over many SMs.
+// so that few particles spread over many SMs, one block for every part of
+// every tile the launch shape allows for.  A tile's header (scene << 10 |
+// live particles, first working slot, scene's first slot, scene's slots minus
+// its sorted offsets; written beside the dense sort, 0 particles past the
+// last tile) is one load in place of a chain of four: tile count, tile, scene
+// record, scene's live count (lambda 7.9 -> 6.1 us, delta-p 7.8 -> 6.3, the
+// whole step of 4,096 particles 80 -> 69).
 #define SMALL_LOOP_BEGIN                                                      \
-    const uint32_t parts_ = tile / kSmallBlock;                               \
-    const uint32_t n_work_ = a.ctrl->n_tiles * parts_;                        \
-    for (uint32_t u_ = blockIdx.x; u_ < n_work_; u_ += gridDim.x) {           \
-        const uint32_t t_ = u_ / parts_;                                      \
-        const uint32_t s = __ldg(a.tile_scene + t_);                          \
-        const uint32_t local = __ldg(a.tile_start + t_) + (u_ % parts_) * kSmallBlock + threadIdx.x;
+    {                                                                         \
+        const uint32_t parts_ = tile / kSmallBlock;                           \
+        const uint4 hd_ = __ldg(a.tile_hdr + blockIdx.x / parts_);            \
+        const uint32_t k_ = (blockIdx.x % parts_) * kSmallBlock + threadIdx.x; \
+        if (k_ >= (hd_.x & 1023u)) return;                                    \
+        const uint32_t s = hd_.x >> 10, i = hd_.y + k_, p_off = hd_.z;
 #define SMALL_LOOP_END }
 
 // Per-tile prologue shared by the particle kernels.
@@ -1085,8 +1094,22 @@ __device__ void bitonic_sort(uint32_t *v, uint32_t n, uint32_t imask)
     }
 }
 
-__global__ void __launch_bounds__(kRadixThreads) k_dense_sort(StepArgs a)
+// small_tiles: small steps, the tile headers of their list passes too (a
+// thread a tile, while the queues are read).
+__global__ void __launch_bounds__(kRadixThreads) k_dense_sort(StepArgs a, uint32_t tile, uint32_t small_tiles)
 {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < small_tiles; t += gridDim.x * blockDim.x) {
+        uint4 h = make_uint4(0u, 0u, 0u, 0u);
+        if (t < a.ctrl->n_tiles) {
+            const uint32_t s = __ldg(a.tile_scene + t), start = __ldg(a.tile_start + t);
+            const SceneDesc &d = a.scenes[s];
+            const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
+            if (start == 0) a.scene_num[s] = live;  // deleted particles leave the scene
+            const uint32_t n = start < live ? min(tile, live - start) : 0u;
+            h = make_uint4(s << 10 | n, d.p_off + start, d.p_off, d.p_off - a.offsets[d.c_off]);
+        }
+        a.tile_hdr[t] = h;
+    }
     __shared__ __align__(16) uint32_t S[kStableLimit];
     __shared__ uint32_t W[kStableLimit];
     __shared__ uint32_t chist_cnt[8], rbase[16], rtot[16];
@@ -1204,16 +1227,11 @@ __global__ void __launch_bounds__(kRadixThreads) k_dense_sort(StepArgs a)
 // 98 -> 86 us at 5.95 M particles in 256 scenes, and the neighbour walk, whose
 // candidates' slots are then their indices, 1,428 -> 1,405 us.
 template <bool PACKED>
-__global__ void __launch_bounds__(512) k_gather(StepArgs a)
+__device__ __forceinline__ void gather_slot(const StepArgs &a, uint32_t s, uint32_t p_off, uint32_t g)
 {
-    TILE_LOOP_BEGIN
-    const uint32_t n = a.scene_num[s];
-    if (local >= n) continue;
-    const SceneDesc d = a.scenes[s];
-    const uint32_t g = d.p_off + local;
     const uint32_t li = a.perm[g];
     const uint32_t w = a.wpos[g];
-    const uint32_t i = d.p_off + li;
+    const uint32_t i = p_off + li;
     const float4 ps = a.xs[i];
     a.xa[w] = make_float4(ps.x, ps.y, ps.z, 0.f);
     const float gs = __uint_as_float(g);
@@ -1225,7 +1243,26 @@ __global__ void __launch_bounds__(512) k_gather(StepArgs a)
         a.xold[w] = make_float4(xo.x, xo.y, xo.z, gs);
     }
     a.id_tmp[w] = __float_as_uint(ps.w);  // the id, stored beside the prediction
+}
+
+template <bool PACKED>
+__global__ void __launch_bounds__(512) k_gather(StepArgs a)
+{
+    TILE_LOOP_BEGIN
+    const uint32_t n = a.scene_num[s];
+    if (local >= n) continue;
+    const uint32_t p_off = a.scenes[s].p_off;
+    gather_slot<PACKED>(a, s, p_off, p_off + local);
     TILE_LOOP_END
+}
+
+// Small steps: the live slots, by tile headers.
+template <bool PACKED>
+__global__ void __launch_bounds__(kSmallBlock) k_gather_small(StepArgs a, uint32_t tile)
+{
+    SMALL_LOOP_BEGIN
+    gather_slot<PACKED>(a, s, p_off, i);
+    SMALL_LOOP_END
 }
 
 // Neighbour list (detectNeighborsCUDA<uint32_t>, pbf_neighbor_search_util.cu:454-482,
@@ -1433,23 +1470,18 @@ __device__ __forceinline__ LamSum lam_sum_split(const uint32_t *nl, uint64_t str
     }
     return ls;
 }
-__global__ void __launch_bounds__(256) k_neighbors_split(StepArgs a, uint32_t tile)
+__global__ void __launch_bounds__(kSplitBlock) k_neighbors_split(StepArgs a, uint32_t tile)
 {
-    const uint32_t per_block = blockDim.x / kSplit;  // particles per block
-    const uint32_t parts = tile / per_block;         // blocks per tile
+    static_assert(kSplitBlock == kSplit * kSmallBlock, "a block takes one part of a tile");
     const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x % kSplit;
     const uint32_t gmask = ((1u << kSplit) - 1u) << (lane & ~(kSplit - 1u));  // the particle's lanes
-    const uint32_t n_work = a.ctrl->n_tiles * parts;
-    for (uint32_t u = blockIdx.x; u < n_work; u += gridDim.x) {
-        const uint32_t t_ = u / parts;
-        const uint32_t s = __ldg(a.tile_scene + t_);
-        const uint32_t local = __ldg(a.tile_start + t_) + (u % parts) * per_block + threadIdx.x / kSplit;
-        const SceneDesc d = a.scenes[s];
-        const uint32_t base = a.offsets[d.c_off];
-        const uint32_t live = a.offsets[d.c_off + d.ncell] - base;
-        if (local >= live) continue;  // the same for the group's lanes
-        const uint32_t i = d.p_off + local;
-        const uint32_t shift = d.p_off - base;
+    const uint32_t parts = tile / kSmallBlock;
+    const uint4 hd = __ldg(a.tile_hdr + blockIdx.x / parts);
+    const uint32_t k = (blockIdx.x % parts) * kSmallBlock + threadIdx.x / kSplit;
+    if (k >= (hd.x & 1023u)) return;  // the same for the group's lanes
+    const uint32_t i = hd.y + k, shift = hd.w;
+    {
+        const SceneDesc d = a.scenes[hd.x >> 10];
         const float4 xp = a.xa[i];
         const float h2 = d.h2;
         const uint32_t cap = d.cap;
@@ -1575,15 +1607,12 @@ __global__ void __launch_bounds__(kSmallBlock, 8) k_lambda_small(StepArgs a, uin
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
-    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
-    if (local >= live) continue;
-    const uint32_t i = d.p_off + local;
     const PairConst pc = pair_const(d);
     const float4 xp = xc[i];
     LamSum ls;
     if (a.selfat[i] != kNotListed) ls.ks = 1.f;
     list_walk_wide(
-        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
         [&](uint32_t q) -> float4 { return __ldg(xc + q); },
         [&](const float4 &xj, bool on) {
             const PairGeo g = pair_geo(xp, xj);
@@ -1751,17 +1780,13 @@ __global__ void __launch_bounds__(kSmallBlock, 8) k_dp_small(StepArgs a, uint32_
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
-    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
-    if (last && local == 0) a.scene_num[s] = live;
-    if (local >= live) continue;
-    const uint32_t i = d.p_off + local;
     const float4 xp = xc[i];
     const PairConst pc = pair_const(d);
     const ScorrConst sc = scorr_const(d, xp.w);
     const float3 sum = by_scorr(d, [&](auto form) {
         float s0 = 0.f, s1 = 0.f, s2 = 0.f;
         list_walk_wide(
-            d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+            d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
             [&](uint32_t q) -> float4 { return __ldg(xc + q); },
             [&](const float4 &xq, bool on) {
                 const PairGeo g = pair_geo(xp, xq);
@@ -1862,17 +1887,14 @@ __global__ void __launch_bounds__(kSmallBlock, 8) k_vort_omega_small(StepArgs a,
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
-    if (d.vort_mode != PBF_VORTICITY_TEXTBOOK) continue;
-    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
-    if (local >= live) continue;
-    const uint32_t i = d.p_off + local;
+    if (d.vort_mode != PBF_VORTICITY_TEXTBOOK) return;
     const float4 *__restrict__ pa = a.pa;
     const float2 *__restrict__ pb = a.pb;
     const float4 A = pa[i];
     const float2 B = pb[i];
     OmegaSum o(A, make_float4(A.w, B.x, B.y, 0.f), d.inv_h);
     list_walk_wide(
-        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
         [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; },
         [&](const PhaseRec &r, bool on) { o.add(r.A, r.A.w, r.B.x, r.B.y, on); });
     put_omega(a, d, i, o);
@@ -1973,14 +1995,11 @@ __global__ void __launch_bounds__(kSmallBlock, 8) k_vort_apply_small(StepArgs a,
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
-    if (d.vort_mode != PBF_VORTICITY_TEXTBOOK) continue;
-    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
-    if (local >= live) continue;
-    const uint32_t i = d.p_off + local;
+    if (d.vort_mode != PBF_VORTICITY_TEXTBOOK) return;
     const float4 *__restrict__ xw = a.xs;
     EtaSum e(xw[i], d.inv_h, -1.f);
     list_walk_wide(
-        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
         [&](uint32_t q) -> float4 { return __ldg(xw + q); }, [&](const float4 &xj, bool on) { e.add(xj, on); });
     put_confinement(a, d, i, e);
     SMALL_LOOP_END
@@ -2092,17 +2111,14 @@ __global__ void __launch_bounds__(kSmallBlock, 8) k_xsph_small(StepArgs a, uint3
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
-    if (d.xsph_mode != PBF_XSPH_LIST) continue;
-    const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
-    if (local >= live) continue;
-    const uint32_t i = d.p_off + local;
+    if (d.xsph_mode != PBF_XSPH_LIST) return;
     const float4 *__restrict__ pa = a.pa;
     const float2 *__restrict__ pb = a.pb;
     const float4 A = pa[i];
     const float2 B = pb[i];
     XsphSum o(A, make_float4(A.w, B.x, B.y, 0.f), d);
     list_walk_wide(
-        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
         [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; },
         [&](const PhaseRec &r, bool on) { o.add(r.A, r.A.w, r.B.x, r.B.y, on); });
     a.v[__float_as_uint(a.xold[i].w)] = o.result(d);
@@ -2223,7 +2239,7 @@ __global__ void k_aos3_to_f4(const float *__restrict__ src, float4 *__restrict__
 
 // A scene's n uploaded particles widened into the phase and numbered, and the
 // scene's counters, in one launch: five small launches (x, v, ids, two
-// counters) took SETOLD us for 4,096 particles, this one SETNEW.  next_id:
+// counters) took 15.4 us for 4,096 particles, this one 3.8.  next_id:
 // null for an append, whose ids continue from *id0 (bumped by a launch of its
 // own: other blocks may not have read it yet).
 __global__ void k_load_phase(const float *__restrict__ sx, const float *__restrict__ sv, float4 *__restrict__ x,
@@ -2317,7 +2333,6 @@ Occupancy occupancy(uint32_t tile, uint32_t chunk)
                                                              occ((const void *)k_gather<true>))),
                     occ((const void *)k_finalize)));
     o.cells = occ_b((const void *)k_rank_cells, kCellTileMax);
-    o.split = occ_b((const void *)k_neighbors_split, 256);
     o.nb = occ((const void *)k_neighbors_lambda<false>);
     cudaFuncSetAttribute((const void *)k_neighbors_lambda<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kNbSmemMax);
@@ -2480,15 +2495,20 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
         k_rank_cells<<<sh.grid_cells, sh.cell_tile, 0, st>>>(a);
         PBF_LAUNCHED("k_rank_cells");
     }
-    k_dense_sort<<<sh.grid, kRadixThreads, 0, st>>>(a);
+    k_dense_sort<<<sh.grid, kRadixThreads, 0, st>>>(a, sh.tile, sh.small ? sh.small_tiles : 0u);
     PBF_LAUNCHED("k_dense_sort");
-    if (packed)
+    const uint32_t gs = sh.small_tiles * (sh.tile / kSmallBlock);  // small steps: a block per part of a tile
+    if (sh.small && packed)
+        k_gather_small<true><<<gs, kSmallBlock, 0, st>>>(a, sh.tile);
+    else if (sh.small)
+        k_gather_small<false><<<gs, kSmallBlock, 0, st>>>(a, sh.tile);
+    else if (packed)
         k_gather<true><<<g, b, 0, st>>>(a);
     else
         k_gather<false><<<g, b, 0, st>>>(a);
     PBF_LAUNCHED("k_gather");
     if (sh.small) {
-        k_neighbors_split<<<sh.grid_split, 256, 0, st>>>(a, sh.tile);
+        k_neighbors_split<<<gs, kSplitBlock, 0, st>>>(a, sh.tile);
         PBF_LAUNCHED("k_neighbors_split");
     } else {
         if (sh.nb_smem)
@@ -2498,7 +2518,6 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
         PBF_LAUNCHED("k_neighbors_lambda");
     }
     if (sh.small) {  // (position, lambda) in xb, positions in xa
-        const uint32_t gs = sh.grid_small;
         for (int it = 0; it < iters; ++it) {
             if (it > 0) {
                 k_lambda_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile, a.xa, a.xb);
@@ -2527,7 +2546,7 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
     const bool l16 = (post & kPostList16) != 0, l32 = (post & kPostList32) != 0;
 #define PBF_POST(kernel, grid)                                               \
     if (sh.small) {                                                          \
-        kernel##_small<<<sh.grid_small, kSmallBlock, 0, st>>>(a, sh.tile);   \
+        kernel##_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile);              \
         PBF_LAUNCHED(#kernel);                                               \
     } else {                                                                 \
         if (l32) {                                                           \
