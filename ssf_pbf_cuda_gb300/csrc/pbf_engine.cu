@@ -228,8 +228,9 @@ pbf_status Batch::init(uint32_t max_scenes, uint64_t max_particles, uint64_t max
     CK(A((void **)&d_flags_, 4ull * max_scenes));
     CK(A((void **)&d_next_id_, 4ull * max_scenes));
     float4 **f4[] = {&d_x_, &d_v_, &d_xs_, &d_xa_, &d_xb_, &d_xold_, &d_w_, &d_pa_, &d_vs_};
-    // + kWalkSpare records: the neighbour walk reads candidates in groups of
-    // four and may read up to three past the end of a range (never accepted)
+    // + kWalkSpare records: the neighbour walks read candidates in groups of
+    // four or eight and may read up to seven past the end of a range (never
+    // accepted)
     for (float4 **p : f4) CK(A((void **)p, 16 * (P + kWalkSpare)));
     CK(A((void **)&d_pb_, 8 * (P + kWalkSpare)));
     CK(A((void **)&d_tile_hdr_, 16 * kSmallTiles));
@@ -780,6 +781,17 @@ LaunchShape Batch::shape_for(uint32_t tile) const
     {  // the block's lists in shared memory when they fit
         const uint64_t b = (uint64_t)tile * (max_pair_ - 1u) * 4u;
         sh.nb_smem = b <= kNbSmemMax ? (uint32_t)b : 0u;
+        // small steps: the lists and the cells' ranges (27 per particle at
+        // most, kSplit lanes a particle or one: the same per block)
+        sh.small_split = 0;
+        if (sh.small) {
+            sh.nb_smem = kSmallBlock * (max_pair_ - 1u) * 4u + kSmallWalkSmem;
+            const uint32_t split = sh.nb_smem + kSplitBlock * (max_pair_ - 1u) * 4u;
+            if ((uint64_t)nt * tile <= kSplitStep && split <= kNbSmemMax) {
+                sh.small_split = 1;
+                sh.nb_smem = split;
+            }
+        }
     }
     // one kernel while the table fits in registers: one block, then a cluster
     sh.scan_cluster = sh.scan_rounds = 0;

@@ -144,13 +144,14 @@ struct LaunchShape {
     uint32_t cell_tile;   // cells per cell tile = threads per k_rank_cells block (autotuned)
     uint32_t small;       // latency-bound step (at most kSmallStep particle slots): split
                           // neighbour walk, per-particle rank, wide list reads
+    uint32_t small_split; // small steps: their walk takes kSplit lanes a particle
     uint32_t small_tiles; // small steps: tiles rounded up to a power of two, for which headers are written
     uint32_t nb_smem;     // k_neighbors_lambda: bytes of shared memory for the block's lists (0 = stored directly)
     bool operator==(const LaunchShape &o) const
     {
         return tile == o.tile && grid == o.grid && scan_grid == o.scan_grid && scan_rounds == o.scan_rounds && scan_cluster == o.scan_cluster &&
                chunk == o.chunk &&
-               grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && small_tiles == o.small_tiles && nb_smem == o.nb_smem &&
+               grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && small_tiles == o.small_tiles && small_split == o.small_split && nb_smem == o.nb_smem &&
                grid_nb == o.grid_nb && grid_lambda == o.grid_lambda && grid_dp == o.grid_dp &&
                grid_omega[0] == o.grid_omega[0] && grid_omega[1] == o.grid_omega[1] && grid_apply[0] == o.grid_apply[0] &&
                grid_apply[1] == o.grid_apply[1] && grid_xsph[0] == o.grid_xsph[0] && grid_xsph[1] == o.grid_xsph[1];
@@ -224,16 +225,27 @@ constexpr uint32_t kBlockScanMax = 8192;      // cells up to which one block sca
 constexpr uint32_t kScanClusterMax = 16;      // blocks of the scan's cluster (1024 threads each)
 constexpr uint32_t kScanRoundsMax = 18;       // cells a thread of it may hold: tables are 2^k + 1 cells, up to 2^18 + 1
 constexpr uint32_t kNbSmemMax = 96 * 1024;  // shared-memory budget for a k_neighbors_lambda block's lists
-constexpr uint32_t kSmallStep = 131072;     // particle slots up to which a step is latency bound
+// Particle slots up to which a step is bound by latency rather than throughput:
+// the small steps' list passes fit one wave (8 blocks of 64 on 152 SMs).  At 65,000
+// particles they take 114 us a step and the large steps' 138, at 80,000 (two
+// waves) 158 and 145.
+constexpr uint32_t kSmallStep = 77824;
 constexpr uint32_t kSmallBlock = 64;        // particles of a block of the small steps' list passes
-constexpr uint32_t kSmallTiles = kSmallStep / 64;  // tiles a small step may have (a power of two)
-constexpr uint32_t kSplit = 4;              // small steps: lanes per particle in the split neighbour walk
+constexpr uint32_t kSmallTiles = 2048;      // tiles a small step may have, rounded up to a power of two
+static_assert(kSmallTiles >= kSmallStep / 64, "a header per tile of a small step");
+// shared memory of their walk beside the lists: per warp 27 ranges of up to 32 cells and the cells' coordinates
+constexpr uint32_t kSmallWalkSmem = kSmallBlock / 32 * (32 * 27 * 8 + 96 * 4);
+constexpr uint32_t kSplit = 4;              // lanes a particle in the smallest steps' walk
 constexpr uint32_t kSplitBlock = kSplit * kSmallBlock;
+// Particle slots up to which the walk is split: 15,000 particles 76 us a step
+// against 78 with one lane a particle, 20,000 84 against 80 (10,648 at h = 1.4
+// spacings 47 against 51).
+constexpr uint32_t kSplitStep = 16384;
 constexpr uint32_t kCellTile = 256;         // default cells per cell tile = threads per k_rank_cells block
 constexpr uint32_t kCellTileMin = 64, kCellTileMax = 512;  // the autotuner's range
 constexpr uint32_t kMidMin = 16;            // buckets with more members are queued (warp or block per bucket)
 constexpr uint32_t kList16Max = 65536;      // scenes of at most this many slots keep u16 neighbour lists
 constexpr uint8_t kNotListed = 0xFF;        // selfat of a particle the cap cut from its own list
-constexpr uint32_t kWalkSpare = 4;          // spare float4 records after each per-particle array
+constexpr uint32_t kWalkSpare = 8;          // spare float4 records after each per-particle array
 
 }  // namespace pbf103

@@ -1396,181 +1396,315 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
     TILE_LOOP_END
 }
 
-// Small (latency-bound) steps: one particle's walk split over kSplit lanes
-// of a warp, each walking a contiguous run of the nine (dz, dy) rows into a
-// private buffer of at most cap entries.  A prefix over the group's counts
-// then places every lane's entries after those of the rows before it, so the
-// list holds the first cap accepted candidates in the reference's walk
-// order, as k_neighbors_lambda's.  The group then sums the iteration-0
-// lambda over the list in list order (lam_sum_split: the same sum, bit for
-// bit).  Scenes with more than kSplitCap list slots walk in one lane.
-constexpr uint32_t kSplitCap = 64;
-static_assert(kSplit == 4 || kSplit == 8, "a particle's lanes share one aligned group of a warp");
-
-// The (dz, dy) rows [rr0, rr1) of a particle's lane sub: rows shared evenly,
-// the first lane taking the one left over.
-__device__ __forceinline__ void split_rows(uint32_t sub, int &rr0, int &rr1)
+// Small (latency-bound) steps' walk, one particle a lane.  The one-lane walk of
+// large steps is a chain of dependent loads a cell at a time: the cell's
+// range, then its candidates four at a time.  Here the 27 ranges of each of
+// the warp's distinct cells are looked up first, all at once, by the warp's
+// lanes together (lanes hold consecutive working slots, so a cell's particles
+// are neighbouring lanes), and each lane then goes through the ranges near
+// it with the next 8 candidates requested before it tests the current 8.
+// Lists, counts and lambda as k_neighbors_lambda's.  The whole step of 32,768
+// particles 95 -> 88 us, of 65,000 132 -> 114 us, against four lanes a
+// particle that each looked up and walked a run of the nine rows.
+//
+// Shared memory: the block's accepted slots [slot][thread], then per warp the
+// ranges and the cells' coordinates.
+__device__ __forceinline__ uint32_t near_cells(const SceneDesc &d, float4 xp, int32_t icx, int32_t icy, int32_t icz)
 {
-    constexpr int per = 9 / (int)kSplit, extra = 9 - per * (int)kSplit;
-    rr0 = sub == 0 ? 0 : extra + per * (int)sub;
-    rr1 = extra + per * ((int)sub + 1);
-}
-
-// Small steps: a sum over one particle's list split over the particle's
-// kSplit lanes.  Lane sub evaluates slots sub, sub + kSplit, ...; each
-// round's terms reach every lane of the group by shuffles and are added in
-// list order, so every lane ends with the one-lane sums, bit for bit.  List
-// indices are requested two rounds ahead and positions one round ahead (a
-// slot past the list reads index 0, a valid slot, and adds nothing).  RO:
-// the list is read through the read-only path (it was not written by this
-// kernel).
-template <bool RO>
-__device__ __forceinline__ uint32_t split_index(const uint32_t *nl, uint64_t stride, uint32_t nn, uint32_t k,
-                                                bool l16, uint32_t base)
-{
-    if (k >= nn) return 0u;
-    if (l16) {
-        const uint16_t *p = reinterpret_cast<const uint16_t *>(nl) + list16_slot(k, stride);
-        return base + (RO ? __ldg(p) : *p);
+    // bit 9 (dz + 1) + 3 (dy + 1) + dx + 1: cells that can hold a particle
+    // within h of xp (see walk27_cells)
+    if (d.gx < 4 || d.gy < 4 || d.gz < 4) return 0x7FFFFFFu;
+    const float lx = xp.x - (float)icx * d.cw, ly = xp.y - (float)icy * d.cw, lz = xp.z - (float)icz * d.cw;
+    const float rx = d.cw - lx, ry = d.cw - ly, rz = d.cw - lz;
+    const float lim = d.h2 * 1.001f;
+    uint32_t m = 0;
+#pragma unroll
+    for (int rr = 0; rr < 9; ++rr) {
+        const int dz = rr / 3 - 1, dy = rr % 3 - 1;
+        const float ez = dz < 0 ? lz : (dz > 0 ? rz : 0.f);
+        const float ey = dy < 0 ? ly : (dy > 0 ? ry : 0.f);
+        const float eyz2 = ey * ey + ez * ez;
+        if (eyz2 <= lim) m |= 2u << (3 * rr);
+        if (eyz2 <= lim && eyz2 + lx * lx <= lim) m |= 1u << (3 * rr);
+        if (eyz2 <= lim && eyz2 + rx * rx <= lim) m |= 4u << (3 * rr);
     }
-    const uint32_t *p = nl + list_slot(k, stride);
-    return RO ? __ldg(p) : *p;
+    return m;
 }
 
-template <bool RO>
-__device__ __forceinline__ LamSum lam_sum_split(const uint32_t *nl, uint64_t stride, uint32_t nn,
-                                                const float4 *__restrict__ xc, float4 xp, const SceneDesc &d,
-                                                uint32_t sub, uint32_t gmask, bool self_listed)
+// The candidate ranges of a warp's distinct cells (n of them, coordinates in
+// cells), 27 a cell, by the warp's lanes: lane k takes cell k of the 27 around
+// each.  A range is the slots that hold the cell's particles, as walk27_cells
+// visits them; none when x >= y.
+__device__ __forceinline__ void warp_ranges(const SceneDesc &d, const StepArgs &a, uint32_t shift, uint32_t n,
+                                            const int32_t *cells, uint2 *rng)
 {
-    const PairConst pc = pair_const(d);
-    const bool l16 = d.list16 != 0;
-    const uint32_t base = d.p_off;
-    LamSum ls;
-    if (self_listed) ls.ks = 1.f;  // the particle's own w(0), first as in the one-lane passes
-    float4 x0 = __ldg(xc + split_index<RO>(nl, stride, nn, sub, l16, base));
-    uint32_t q1 = split_index<RO>(nl, stride, nn, sub + kSplit, l16, base);
-    for (uint32_t k0 = 0; k0 < nn; k0 += kSplit) {
-        const float4 x1 = __ldg(xc + q1);
-        q1 = split_index<RO>(nl, stride, nn, k0 + 2 * kSplit + sub, l16, base);
-        // this lane's pair (slot k0 + sub); a slot past the list reads
-        // index 0 and is not added
-        const PairGeo g = pair_geo(xp, x0);
-        const PairWS k = pair_ws(g.r2, pc);
-#pragma unroll
-        for (uint32_t j = 0; j < kSplit; ++j) {
-            const float W = __shfl_sync(gmask, k.W, j, kSplit);
-            const float s = __shfl_sync(gmask, k.s, j, kSplit);
-            const float d0 = __shfl_sync(gmask, g.d0, j, kSplit);
-            const float d1 = __shfl_sync(gmask, g.d1, j, kSplit);
-            const float d2 = __shfl_sync(gmask, g.d2, j, kSplit);
-            const float sr = __shfl_sync(gmask, k.sr, j, kSplit);
-            if (k0 + j < nn) ls.add(W, s, d0, d1, d2, sr);
+    const uint32_t lane = threadIdx.x & 31u;
+    const int32_t dz = (int32_t)(lane / 9u) - 1, dy = (int32_t)(lane / 3u % 3u) - 1, dx = (int32_t)(lane % 3u) - 1;
+    const uint32_t *off = a.offsets + d.c_off;
+    const uint64_t *ch = a.chist + d.c_off;
+    if (lane < 27) {
+#pragma unroll 4
+        for (uint32_t c = 0; c < n; ++c) {
+            const int32_t tx = cells[3 * c] + dx, ty = cells[3 * c + 1] + dy, tz = cells[3 * c + 2] + dz;
+            const uint32_t b = hash3((uint32_t)tx, (uint32_t)ty, (uint32_t)tz, d);
+            uint32_t st = __ldg(off + b), en = __ldg(off + b + 1);
+            const uint64_t h = __ldg(reinterpret_cast<const unsigned long long *>(ch + b));
+            if (h != kClassWhole && st != en) {  // an empty bucket's class ends are stale
+                const uint32_t k = alias_class(tx, ty, tz, d);
+                const uint32_t h0 = (uint32_t)h, h1 = (uint32_t)(h >> 32);
+                en = st + (__byte_perm(h0, h1, k) & 0xFFu);
+                st += __byte_perm(h0 << 8, __funnelshift_l(h0, h1, 8), k) & 0xFFu;
+            }
+            rng[27 * c + lane] = make_uint2(st + shift, en + shift);
         }
-        x0 = x1;
     }
-    return ls;
+    __syncwarp();
 }
-__global__ void __launch_bounds__(kSplitBlock) k_neighbors_split(StepArgs a, uint32_t tile)
+
+// A lane's walk over the ranges todo of its cell's 27: puts the slots accepted
+// in order, at most cap, and returns their number; self: the particle's own
+// place among them.
+template <class PUT>
+__device__ __forceinline__ uint32_t walk_ranges(const uint2 *mine, uint32_t todo, const float4 *__restrict__ xa,
+                                                float4 xp, float h2, uint32_t cap, uint32_t i, uint32_t &self, PUT &&put)
 {
-    static_assert(kSplitBlock == kSplit * kSmallBlock, "a block takes one part of a tile");
-    const uint32_t lane = threadIdx.x & 31u, sub = threadIdx.x % kSplit;
-    const uint32_t gmask = ((1u << kSplit) - 1u) << (lane & ~(kSplit - 1u));  // the particle's lanes
-    const uint32_t parts = tile / kSmallBlock;
-    const uint4 hd = __ldg(a.tile_hdr + blockIdx.x / parts);
-    const uint32_t k = (blockIdx.x % parts) * kSmallBlock + threadIdx.x / kSplit;
-    if (k >= (hd.x & 1023u)) return;  // the same for the group's lanes
-    const uint32_t i = hd.y + k, shift = hd.w;
-    {
-        const SceneDesc d = a.scenes[hd.x >> 10];
-        const float4 xp = a.xa[i];
-        const float h2 = d.h2;
-        const uint32_t cap = d.cap;
-        const uint64_t stride = a.nbr_stride;
-        uint32_t *nl = list_of(a.nbr, i);
-        uint16_t *nl16 = reinterpret_cast<uint16_t *>(nl);
-        const bool l16 = d.list16 != 0;
-        auto put = [&](uint32_t k, uint32_t q) {  // slot k of the list := sorted slot q
-            if (l16)
-                nl16[list16_slot(k, stride)] = (uint16_t)(q - d.p_off);
-            else
-                nl[list_slot(k, stride)] = q;
-        };
-        const float4 *__restrict__ xa = a.xa;
-        // rows shared over the lanes (split_rows); one lane takes all nine
-        // when the list does not fit the private buffer
-        const bool one = cap > kSplitCap;
-        int rr0 = sub == 0 ? 0 : 9, rr1 = 9;
-        if (!one) split_rows(sub, rr0, rr1);
-        uint32_t buf[kSplitCap];
-        // cnt: candidates this lane accepted, the particle itself included
-        // (it counts toward the cap at its walk position but is not stored;
-        // tself is its place in this lane's run)
-        uint32_t cnt = 0, tself = kNotListed;
-        if (one && sub == 0) {  // write straight into the list
-            walk27_cells<true>(d, a.offsets, a.chist, shift, xp, [&](uint32_t st, uint32_t en) -> bool {
-                for (uint32_t q = st; q < en; ++q) {
-                    const float4 c = __ldg(xa + q);
-                    if (dist2_exact(xp, c) < h2) {
-                        if (q == i) tself = cnt;
-                        else put(cnt - (tself < cnt ? 1u : 0u), q);
-                        if (++cnt == cap) return false;
-                    }
-                }
-                return true;
-            });
-        } else if (!one) {
-            walk27_cells<true>(d, a.offsets, a.chist, shift, xp, [&](uint32_t st, uint32_t en) -> bool {
-                for (uint32_t q0 = st; q0 < en; q0 += 4) {
-                    float4 c[4];
-                    const float4 *pq = xa + q0;  // up to three spare records past the range
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) c[k] = __ldg(pq + k);
-                    bool acc[4];
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) acc[k] = (q0 + k < en) && dist2_exact(xp, c[k]) < h2;
-#pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) {
-                        if (acc[k] && cnt < cap) {
-                            const uint32_t qs = q0 + k;
-                            if (qs == i) tself = cnt;
-                            buf[cnt] = qs;
-                            ++cnt;
-                        }
-                    }
-                    if (cnt == cap) return false;
-                }
-                return true;
-            }, rr0, rr1);
+    // the next 8 candidates: [q, min(q + 8, en)); q == en when none are left
+    uint32_t q = 0, en = 0;
+    auto next = [&]() {
+        q += 8;
+        while (q >= en && todo) {
+            const uint2 r = mine[__ffs((int)todo) - 1];
+            todo &= todo - 1u;
+            q = r.x;
+            en = r.y;
         }
-        // place the group's runs one after the other, up to cap
-        uint32_t incl = cnt;
+        if (q >= en) q = en = 0;
+    };
+    float4 c[8];
+    auto load = [&]() {
+        if (q < en) {
 #pragma unroll
-        for (uint32_t o = 1; o < kSplit; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(gmask, incl, o, kSplit);
-            if (sub >= o) incl += v;
+            for (uint32_t k = 0; k < 8; ++k) c[k] = __ldg(xa + q + k);  // up to 7 spare records past the range
         }
-        const uint32_t total = __shfl_sync(gmask, incl, kSplit - 1, kSplit);
-        const uint32_t pre = incl - cnt;
-        // the particle's own place in the group's list (one lane holds it)
-        uint32_t gself = tself != kNotListed ? pre + tself : 0xFFFFFFFFu;
+    };
+    next();
+    load();
+    uint32_t cnt = 0;
+    while (q < en && cnt < cap) {
+        float4 t[8];
 #pragma unroll
-        for (uint32_t o = 1; o < kSplit; o <<= 1) gself = min(gself, __shfl_xor_sync(gmask, gself, o, kSplit));
-        const bool listed = gself < cap;
-        if (!one) {
-            for (uint32_t t = 0; t < cnt && pre + t < cap; ++t) {
-                const uint32_t g = pre + t;
-                if (g != gself) put(g - (g > gself ? 1u : 0u), buf[t]);
+        for (uint32_t k = 0; k < 8; ++k) t[k] = c[k];
+        const uint32_t q0 = q, left = en - q;
+        next();
+        load();
+        bool acc[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) acc[k] = k < left && dist2_exact(xp, t[k]) < h2;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (acc[k] && cnt < cap) {
+                if (q0 + k == i) self = cnt;
+                put(cnt, q0 + k);
+                ++cnt;
             }
         }
-        const uint32_t nn = (total < cap ? total : cap) - (listed ? 1u : 0u);
-        __syncwarp(gmask);  // the list entries of the group are visible to all its lanes
-        // lambda of iteration 0 over the list, split over the group's lanes
-        const LamSum ls = lam_sum_split<false>(nl, stride, nn, xa, xp, d, sub, gmask, listed);
-        if (sub == 0) {
-            a.nnb[i] = (uint8_t)nn;
-            a.selfat[i] = listed ? (uint8_t)gself : kNotListed;
-            a.xb[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));  // the first delta-p pass gathers both
+    }
+    return cnt;
+}
+
+__global__ void __launch_bounds__(kSmallBlock, 8) k_neighbors_small(StepArgs a, uint32_t tile)
+{
+    extern __shared__ __align__(8) uint32_t s_small[];
+    const uint32_t parts = tile / kSmallBlock;
+    const uint4 hd = __ldg(a.tile_hdr + blockIdx.x / parts);
+    const uint32_t kk = (blockIdx.x % parts) * kSmallBlock + threadIdx.x, lane = threadIdx.x & 31u;
+    const uint32_t n = hd.x & 1023u;
+    if (kk - lane >= n) return;  // whole warps
+    const bool on = kk < n;
+    const uint32_t i = hd.y + kk, p_off = hd.z, shift = hd.w;
+    const float4 xp = on ? a.xa[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const SceneDesc d = a.scenes[hd.x >> 10];
+    const uint32_t cap = d.cap;
+    uint32_t *list = s_small + threadIdx.x;
+    uint32_t *const warps = s_small + cap * kSmallBlock;
+    uint2 *rng = reinterpret_cast<uint2 *>(warps) + (threadIdx.x >> 5) * (32u * 27u);
+    int32_t *cells = reinterpret_cast<int32_t *>(warps + (kSmallBlock >> 5) * (32u * 27u * 2u)) + (threadIdx.x >> 5) * 96u;
+    const int32_t icx = cell_coord(xp.x, d.cw), icy = cell_coord(xp.y, d.cw), icz = cell_coord(xp.z, d.cw);
+    const int32_t ux = __shfl_up_sync(0xffffffffu, icx, 1), uy = __shfl_up_sync(0xffffffffu, icy, 1),
+                  uz = __shfl_up_sync(0xffffffffu, icz, 1);
+    const bool same = ux == icx && uy == icy && uz == icz;
+    const uint32_t heads = __ballot_sync(0xffffffffu, on && (lane == 0 || !same));
+    const uint32_t seg = __popc(heads & (0xFFFFFFFFu >> (31u - lane))) - 1u;  // the lane's cell of the warp's
+    if (heads >> lane & 1u) {
+        cells[3 * seg] = icx;
+        cells[3 * seg + 1] = icy;
+        cells[3 * seg + 2] = icz;
+    }
+    __syncwarp();
+    warp_ranges(d, a, shift, __popc(heads), cells, rng);
+    if (!on) return;  // no warp-wide operation follows
+    uint32_t todo = near_cells(d, xp, icx, icy, icz);
+    const uint2 *mine = rng + 27u * seg;
+    const float4 *__restrict__ xa = a.xa;
+    // the particle itself is accepted and counts toward the cap, but is not
+    // stored (see k_neighbors_lambda)
+    uint32_t selfat = kNotListed;
+    uint32_t cnt = walk_ranges(mine, todo, xa, xp, d.h2, cap, i, selfat,
+                               [&](uint32_t k, uint32_t q) { list[k * kSmallBlock] = q; });
+    cnt -= selfat < cnt ? 1u : 0u;
+    a.nnb[i] = (uint8_t)cnt;
+    a.selfat[i] = (uint8_t)selfat;
+    LamSum ls;
+    if (selfat != kNotListed) ls.ks = 1.f;
+    const PairConst pc = pair_const(d);
+    const uint64_t stride = a.nbr_stride;
+    uint4 *row = reinterpret_cast<uint4 *>(list_of(a.nbr, i));
+    for (uint32_t k0 = 0; k0 < cnt; k0 += 16) {
+        uint32_t s[16];  // slots past the count load the particle itself and add nothing
+#pragma unroll
+        for (uint32_t k = 0; k < 16; ++k)
+            s[k] = k0 + k < cnt ? list[(k0 + k + (k0 + k >= selfat ? 1u : 0u)) * kSmallBlock] : i;
+        float4 x[16];
+#pragma unroll
+        for (uint32_t k = 0; k < 16; ++k) x[k] = __ldg(xa + s[k]);
+        if (d.list16) {
+#pragma unroll
+            for (uint32_t j = 0; j < 16; j += 8) {
+                uint32_t w[4];
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) w[k] = (s[j + 2 * k] - p_off) | (s[j + 2 * k + 1] - p_off) << 16;
+                if (k0 + j < cnt) list_st(row + (uint64_t)((k0 + j) >> 3) * stride, make_uint4(w[0], w[1], w[2], w[3]));
+            }
+        } else {
+#pragma unroll
+            for (uint32_t j = 0; j < 16; j += 4)
+                if (k0 + j < cnt)
+                    list_st(row + (uint64_t)((k0 + j) >> 2) * stride, make_uint4(s[j], s[j + 1], s[j + 2], s[j + 3]));
         }
+#pragma unroll
+        for (uint32_t k = 0; k < 16; ++k) {
+            const PairGeo g = pair_geo(xp, x[k]);
+            ls.add(g, masked(pair_ws(g.r2, pc), k0 + k < cnt));
+        }
+    }
+    a.xb[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));  // the first delta-p pass gathers both
+}
+
+// The smallest steps: the same walk over kSplit lanes a particle, so that few
+// particles still fill the SMs and each lane's chain is a quarter: every lane
+// takes a run of the near cells into its own part of shared memory, a prefix
+// over the group's counts lays the runs end to end up to the cap (the
+// reference's first cap accepted candidates in walk order), lane k writes
+// every fourth row of the list, and the lambda terms of slots k, k + kSplit,
+// ... reach the group by shuffles and are added in list order by each lane
+// (the one-lane sums, bit for bit).  The step of 4,096 particles 73 -> 68 us
+// against the split without shared ranges; a fourth block a SM (64 registers)
+// spills and takes 72.
+__global__ void __launch_bounds__(kSplitBlock, 3) k_neighbors_split(StepArgs a, uint32_t tile)
+{
+    extern __shared__ __align__(8) uint32_t s_small[];
+    const uint32_t parts = tile / kSmallBlock, p = threadIdx.x / kSplit;
+    const uint4 hd = __ldg(a.tile_hdr + blockIdx.x / parts);
+    const uint32_t k0 = (blockIdx.x % parts) * kSmallBlock, kk = k0 + p, lane = threadIdx.x & 31u;
+    const uint32_t sub = lane % kSplit, gmask = ((1u << kSplit) - 1u) << (lane & ~(kSplit - 1u));
+    const uint32_t n = hd.x & 1023u;
+    if (k0 + (threadIdx.x & ~31u) / kSplit >= n) return;  // whole warps
+    const bool on = kk < n;
+    const uint32_t i = hd.y + kk, p_off = hd.z, shift = hd.w;
+    const float4 xp = on ? a.xa[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const SceneDesc d = a.scenes[hd.x >> 10];
+    const uint32_t cap = d.cap;
+    // shared memory: every lane's accepted slots [slot][thread], the merged
+    // lists [slot][particle], then per warp the ranges and the cells
+    uint32_t *run = s_small + threadIdx.x, *list = s_small + cap * kSplitBlock + p;
+    uint32_t *const warps = s_small + cap * (kSplitBlock + kSmallBlock);
+    constexpr uint32_t kParts = 32 / kSplit;  // particles, and so cells, of a warp
+    uint2 *rng = reinterpret_cast<uint2 *>(warps) + (threadIdx.x >> 5) * (kParts * 27u);
+    int32_t *cells = reinterpret_cast<int32_t *>(warps + (kSplitBlock >> 5) * (kParts * 27u * 2u)) +
+                     (threadIdx.x >> 5) * (3u * kParts);
+    const int32_t icx = cell_coord(xp.x, d.cw), icy = cell_coord(xp.y, d.cw), icz = cell_coord(xp.z, d.cw);
+    const int32_t ux = __shfl_up_sync(0xffffffffu, icx, 1), uy = __shfl_up_sync(0xffffffffu, icy, 1),
+                  uz = __shfl_up_sync(0xffffffffu, icz, 1);
+    const bool same = ux == icx && uy == icy && uz == icz;
+    const uint32_t heads = __ballot_sync(0xffffffffu, on && (lane == 0 || !same));
+    const uint32_t seg = __popc(heads & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+    if (heads >> lane & 1u) {
+        cells[3 * seg] = icx;
+        cells[3 * seg + 1] = icy;
+        cells[3 * seg + 2] = icz;
+    }
+    __syncwarp();
+    warp_ranges(d, a, shift, __popc(heads), cells, rng);
+    if (!on) return;  // whole groups; only the groups' own lanes meet from here on
+    uint32_t todo = near_cells(d, xp, icx, icy, icz);
+    {  // this lane's run of the near cells
+        const uint32_t m = __popc(todo), lo = m * sub / kSplit, hi = m * (sub + 1) / kSplit;
+        for (uint32_t k = 0; k < lo; ++k) todo &= todo - 1u;
+        uint32_t rest = todo;
+        for (uint32_t k = lo; k < hi; ++k) rest &= rest - 1u;
+        todo ^= rest;
+    }
+    const float4 *__restrict__ xa = a.xa;
+    uint32_t tself = kNotListed;
+    const uint32_t cnt = walk_ranges(rng + 27u * seg, todo, xa, xp, d.h2, cap, i, tself,
+                                     [&](uint32_t k, uint32_t q) { run[k * kSplitBlock] = q; });
+    uint32_t incl = cnt;
+#pragma unroll
+    for (uint32_t o = 1; o < kSplit; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(gmask, incl, o, kSplit);
+        if (sub >= o) incl += v;
+    }
+    const uint32_t total = __shfl_sync(gmask, incl, kSplit - 1, kSplit), pre = incl - cnt;
+    // the particle's own place in the group's list (one lane holds it)
+    uint32_t gself = tself != kNotListed ? pre + tself : 0xFFFFFFFFu;
+#pragma unroll
+    for (uint32_t o = 1; o < kSplit; o <<= 1) gself = min(gself, __shfl_xor_sync(gmask, gself, o, kSplit));
+    const bool listed = gself < cap;
+    for (uint32_t t = 0; t < cnt && pre + t < cap; ++t) {
+        const uint32_t g = pre + t;
+        if (g != gself) list[(g - (g > gself ? 1u : 0u)) * kSmallBlock] = run[t * kSplitBlock];
+    }
+    const uint32_t nn = min(total, cap) - (listed ? 1u : 0u);
+    __syncwarp(gmask);
+    {  // the list's rows, one lane each in turn
+        const uint64_t stride = a.nbr_stride;
+        uint4 *row = reinterpret_cast<uint4 *>(list_of(a.nbr, i));
+        const uint32_t per = d.list16 ? 8u : 4u;
+        for (uint32_t r = sub; r * per < nn; r += kSplit) {
+            uint32_t s[8];
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) s[k] = k < per && r * per + k < nn ? list[(r * per + k) * kSmallBlock] - p_off : 0u;
+            if (d.list16)
+                list_st(row + r * stride, make_uint4(s[0] | s[1] << 16, s[2] | s[3] << 16, s[4] | s[5] << 16, s[6] | s[7] << 16));
+            else
+                list_st(row + r * stride, make_uint4(s[0] + p_off, s[1] + p_off, s[2] + p_off, s[3] + p_off));
+        }
+    }
+    LamSum ls;
+    if (listed) ls.ks = 1.f;
+    const PairConst pc = pair_const(d);
+    for (uint32_t r0 = 0; r0 < nn; r0 += 8 * kSplit) {  // 8 slots a lane at once
+        float4 x[8];
+#pragma unroll
+        for (uint32_t r = 0; r < 8; ++r) {
+            const uint32_t k = r0 + r * kSplit + sub;
+            x[r] = __ldg(xa + (k < nn ? list[k * kSmallBlock] : i));
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < 8; ++r) {
+            const PairGeo g = pair_geo(xp, x[r]);
+            const PairWS k = masked(pair_ws(g.r2, pc), r0 + r * kSplit + sub < nn);
+#pragma unroll
+            for (uint32_t j = 0; j < kSplit; ++j)
+                ls.add(__shfl_sync(gmask, k.W, j, kSplit), __shfl_sync(gmask, k.s, j, kSplit),
+                       __shfl_sync(gmask, g.d0, j, kSplit), __shfl_sync(gmask, g.d1, j, kSplit),
+                       __shfl_sync(gmask, g.d2, j, kSplit), __shfl_sync(gmask, k.sr, j, kSplit));
+        }
+    }
+    if (sub == 0) {
+        a.nnb[i] = (uint8_t)nn;
+        a.selfat[i] = listed ? (uint8_t)gself : kNotListed;
+        a.xb[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));  // the first delta-p pass gathers both
     }
 }
 
@@ -2336,6 +2470,8 @@ Occupancy occupancy(uint32_t tile, uint32_t chunk)
     o.nb = occ((const void *)k_neighbors_lambda<false>);
     cudaFuncSetAttribute((const void *)k_neighbors_lambda<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kNbSmemMax);
+    cudaFuncSetAttribute((const void *)k_neighbors_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNbSmemMax);
+    cudaFuncSetAttribute((const void *)k_neighbors_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNbSmemMax);
     const bool c4 = chunk == 4;
     o.lambda = occ(c4 ? PassFns<4>::lambda() : PassFns<8>::lambda());
     o.dp = occ(c4 ? PassFns<4>::dp() : PassFns<8>::dp());
@@ -2508,7 +2644,10 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
         k_gather<false><<<g, b, 0, st>>>(a);
     PBF_LAUNCHED("k_gather");
     if (sh.small) {
-        k_neighbors_split<<<gs, kSplitBlock, 0, st>>>(a, sh.tile);
+        if (sh.small_split)
+            k_neighbors_split<<<gs, kSplitBlock, sh.nb_smem, st>>>(a, sh.tile);
+        else
+            k_neighbors_small<<<gs, kSmallBlock, sh.nb_smem, st>>>(a, sh.tile);
         PBF_LAUNCHED("k_neighbors_split");
     } else {
         if (sh.nb_smem)
