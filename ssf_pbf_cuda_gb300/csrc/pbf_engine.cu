@@ -1,5 +1,6 @@
 // Host runtime of the PBF engine (see pbf_engine.h).
 #include "pbf_engine.h"
+#include "pbf_scan.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -799,10 +800,10 @@ LaunchShape Batch::shape_for(uint32_t tile) const
     if (cells <= kBlockScanMax) {
         sh.scan_grid = 0;
         sh.scan_rounds = (cells + 1023u) / 1024u;
-    } else if (cells <= lim * 1024u * kScanRoundsMax) {
+    } else if (const uint32_t r = cluster_scan_rounds(cells, lim)) {
         sh.scan_grid = 0;
         sh.scan_cluster = lim;
-        sh.scan_rounds = std::min(pow2((cells + lim * 1024u - 1u) / (lim * 1024u)), kScanRoundsMax);
+        sh.scan_rounds = r;
     }
     return sh;
 }

@@ -15,14 +15,13 @@
 // acceptance) uses explicitly rounded intrinsics so that it is bit-exact
 // against the CPU oracle.  Floating-point solver math follows the reference's
 // operation order but uses rsqrtf (as the reference does).
-#include <cooperative_groups.h>
-
 #include <map>
 #include <mutex>
 #include <tuple>
 #include <utility>
 
 #include "pbf_internal.h"
+#include "pbf_scan.cuh"
 #include "pbf_sort.cuh"
 #include "pbf103.h"
 
@@ -684,17 +683,6 @@ __global__ void __launch_bounds__(512) k_predict_hash(StepArgs a)
 }
 
 // ---- exclusive scan of the cell counts (reduce, spine, down-sweep) ----
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
-{
-    const uint32_t lane = threadIdx.x & 31u;
-#pragma unroll
-    for (uint32_t o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += u;
-    }
-    return v;
-}
-
 __global__ void __launch_bounds__(256) k_scan_reduce(StepArgs a)
 {
     __shared__ uint32_t ws[kScanWarps];
@@ -804,65 +792,24 @@ __global__ void __launch_bounds__(1024) k_scan_single_reg(StepArgs a)
     }
 }
 
-// The whole scan in one thread-block cluster, for the tables between the
-// one-block scan and the three-kernel one: each block holds a run of 1024 * R
-// cells in registers as k_scan_single_reg does, its total goes into every
-// other block's shared memory, and after the cluster's barrier each block
-// adds the totals before it.  Bound by the latency of the one launch: 32,769
-// cells (event-timed, launch included) took 27.7 us in one block looping over
-// rounds of 1024 cells and take 8.4 here (9.3 in a cluster of 8), 65,537
-// cells 20.2 us in three kernels and 9.3 here.
+// The whole scan in one thread-block cluster (cluster_scan), for the tables
+// between the one-block scan and the three-kernel one.  Bound by the latency
+// of the one launch: 32,769 cells (event-timed, launch included) took 27.7 us
+// in one block looping over rounds of 1024 cells and take 8.4 here (9.3 in a
+// cluster of 8), 65,537 cells 20.2 us in three kernels and 9.3 here.
 template <uint32_t R>
 __global__ void __launch_bounds__(1024) k_scan_cluster(StepArgs a)
 {
-    namespace cg = cooperative_groups;
-    const cg::cluster_group cluster = cg::this_cluster();
-    __shared__ uint32_t ws[R][32], tot[kScanClusterMax];
-    const uint32_t n = a.ctrl->n_cells, rank = cluster.block_rank(), blocks = cluster.num_blocks();
-    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, base = rank * (1024u * R);
-    if (rank == 0 && t == 0) {
+    const uint32_t n = a.ctrl->n_cells;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         *a.dense = 0;  // the bucket queues of this step's rank kernel
         *a.mid = 0;
     }
-    uint32_t v[R], inc[R];
-#pragma unroll
-    for (uint32_t k = 0; k < R; ++k) {
-        const uint32_t idx = base + k * 1024u + t;
-        v[k] = idx < n ? a.count[idx] : 0u;
-    }
-#pragma unroll
-    for (uint32_t k = 0; k < R; ++k) {
-        inc[k] = warp_incl_scan(v[k]);
-        if (lane == 31) ws[k][warp] = inc[k];
-    }
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t carry = 0;
-#pragma unroll
-        for (uint32_t k = 0; k < R; ++k) {
-            const uint32_t wv = ws[k][lane];
-            const uint32_t wi = warp_incl_scan(wv);
-            ws[k][lane] = carry + wi - wv;
-            carry += __shfl_sync(0xffffffffu, wi, 31);
-        }
-        if (lane < blocks) *cluster.map_shared_rank(&tot[rank], lane) = carry;
-    }
-    cluster.sync();  // every block's totals are in; no block writes another's memory after it
-    uint32_t before = 0, all = 0;
-    for (uint32_t k = 0; k < blocks; ++k) {
-        const uint32_t x = tot[k];
-        before += k < rank ? x : 0u;
-        all += x;
-    }
-#pragma unroll
-    for (uint32_t k = 0; k < R; ++k) {
-        const uint32_t idx = base + k * 1024u + t;
-        if (idx < n) {
-            a.offsets[idx] = before + ws[k][warp] + inc[k] - v[k];
-            a.count[idx] = 0u;  // ready for the next step's histogram
-        }
-    }
-    if (rank == 0 && t == 0) a.offsets[n] = all;
+    const uint32_t all = cluster_scan<R>(a.count, n, [&](uint32_t c, uint32_t offset, uint32_t) {
+        a.offsets[c] = offset;
+        a.count[c] = 0u;  // ready for the next step's histogram
+    });
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.offsets[n] = all;
 }
 
 __global__ void __launch_bounds__(256) k_scan_down(StepArgs a)
@@ -1030,10 +977,17 @@ __global__ void __launch_bounds__(512) k_rank_reorder(StepArgs a)
         continue;
     }
     uint32_t diff = 0;
-    for (uint32_t t = st; t < en; ++t) {
-        const uint32_t e = __ldg(a.tmp + t);
-        rank += ((e & imask) < local) ? 1u : 0u;
-        diff |= (e >> kClsShift) ^ my_cls;
+    for (uint32_t t = st; t < en; t += 8) {  // 8 members requested together
+        uint32_t e[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) e[k] = t + k < en ? __ldg(a.tmp + t + k) : 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (t + k < en) {
+                rank += ((e[k] & imask) < local) ? 1u : 0u;
+                diff |= (e[k] >> kClsShift) ^ my_cls;
+            }
+        }
     }
     if (grouped && diff) {  // several classes: the class histogram and my place in the walk copy
         mixed = true;
@@ -2556,22 +2510,7 @@ uint32_t scan_cluster_limit()
     const auto it = cache.find(dev);
     if (it != cache.end()) return it->second;
     bool ok = true;
-    for (uint32_t r : {1u, 2u, 4u, 8u, 16u, kScanRoundsMax}) {
-        const ScanFn fn = scan_cluster_fn(r);
-        ok = ok && cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(kScanClusterMax);
-        cfg.blockDim = dim3(1024);
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = kScanClusterMax;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int n = 0;
-        ok = ok && cudaOccupancyMaxActiveClusters(&n, (const void *)fn, &cfg) == cudaSuccess && n > 0;
-    }
-    cudaGetLastError();  // a refused attribute is an answer, not an error
+    for (uint32_t r : {1u, 2u, 4u, 8u, 16u, kScanRoundsMax}) ok = allows_cluster(scan_cluster_fn(r)) && ok;
     cache[dev] = ok ? kScanClusterMax : 8u;
     return cache[dev];
 }
@@ -2592,17 +2531,7 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
         k_predict_hash<false><<<g, b, 0, st>>>(a);
     PBF_LAUNCHED("k_predict_hash");
     if (sh.scan_grid == 0 && sh.scan_cluster) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(sh.scan_cluster);
-        cfg.blockDim = dim3(1024);
-        cfg.stream = st;
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = sh.scan_cluster;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, scan_cluster_fn(sh.scan_rounds), a);
+        launch_cluster(scan_cluster_fn(sh.scan_rounds), sh.scan_cluster, st, a);
         PBF_LAUNCHED("k_scan_single");  // the profile's name for the scan in one launch
     } else if (sh.scan_grid == 0) {  // small table: one block
         switch (sh.scan_rounds) {  // rounds of 1024 cells held in registers
