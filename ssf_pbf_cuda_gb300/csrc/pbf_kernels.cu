@@ -2153,10 +2153,12 @@ struct XsphSum {
         // root per pair; the two differ by rounding only)
         const float q2 = (p0 * p0 + p1 * p1 + p2 * p2) * ih2;
         const float t = 1.f - q2;
-        const float W = (on && q2 <= 1.f) ? alpha6 * t * t * t : 0.f;
-        s0 += (vx - vi.x) * W;
-        s1 += (vy - vi.y) * W;
-        s2 += (vz - vi.z) * W;
+        const float W = q2 <= 1.f ? alpha6 * t * t * t : 0.f;
+        if (on) {  // (not W = 0: an infinite velocity's difference from itself is NaN)
+            s0 += (vx - vi.x) * W;
+            s1 += (vy - vi.y) * W;
+            s2 += (vz - vi.z) * W;
+        }
     }
     __device__ __forceinline__ float4 result(const SceneDesc &d) const
     {

@@ -21,7 +21,7 @@ def _scenes():
     return out
 
 
-def _run(scs, params, filler, max_pair, capacity):
+def _run(scs, params, filler, max_pair, capacity, steps=4):
     small = [(sc, H.resolved(params, sc)) for sc in scs]
     fill = [scenes.dam_break(52, 52, 50, (4.0, 4.0, 4.0), scene_id=390)] if filler else []
     rest = [(sc, H.resolved(params, sc)) for sc in fill]
@@ -31,7 +31,7 @@ def _run(scs, params, filler, max_pair, capacity):
     for sc, p in small + rest:
         bnd = api.Boundary(points_on_planes=sc.planes[0], normals_on_planes=sc.planes[1])
         ids.append(b.add_scene(p, max(sc.n, capacity), sc.domain_end, bnd, sc.area, sc.x, sc.v))
-    b.step(4)
+    b.step(steps)
     return [b.get_scene(i) for i in ids[:len(small)]]
 
 
@@ -46,3 +46,25 @@ def test_small_step_lists_equal_large_steps(gpu, max_pair, capacity):
         assert len(xa) == scs[k].n
         assert np.array_equal(xa.view(np.uint32), xb.view(np.uint32)), k
         assert np.array_equal(va.view(np.uint32), vb.view(np.uint32)), k
+
+
+@pytest.mark.parametrize("filler", [False, True], ids=["small", "large"])
+@pytest.mark.parametrize("capacity", [0, 70000], ids=["u16", "u32"])
+def test_infinite_velocities_count_listed_neighbours_only(gpu, capacity, filler):
+    """Pairs far apart from each other whose confinement overflows to opposite
+    infinite velocities: XSPH adds c (v_j - v_i) W for the one listed neighbour
+    (the particle itself is not listed), inf - inf = NaN in every component;
+    the slots past a list's end, whose loads are the particle's own, add
+    nothing (their v_i - v_i = NaN would trip the pass's NaN guard)."""
+    params = api.config_params(scorr_k=1e-4, vc_parameter=float("inf"))
+    rng = np.random.default_rng(5)
+    m = 5
+    c = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3) * 0.3 + 0.3
+    off = rng.normal(size=c.shape)
+    off *= 0.03 / np.linalg.norm(off, axis=1, keepdims=True)
+    sc = scenes.dam_break(m, m, 2 * m, (2.0, 2.0, 2.0), scene_id=310, spacing=0.05)
+    sc.x = np.concatenate([c + off, c - off]).astype(np.float32)
+    sc.v = rng.normal(scale=0.1, size=sc.x.shape).astype(np.float32)
+    xs, vs = _run([sc], params, filler, params["max_pair_particle_num"], capacity, steps=1)[0]
+    assert len(xs) == sc.n and np.isfinite(xs).all()
+    assert np.isnan(vs).all()
