@@ -175,9 +175,9 @@ pbf_status derive_desc(const pbf_params &p, const float domain_end[3], SceneDesc
 
 uint64_t bytes_per_particle(uint32_t max_pair)
 {
-    // x v xs xa xb xold w pa vs (float4) + pb (float2) + key slot tmp perm id id_tmp wpos + lam + nnb +
+    // x v xs xa xb xold w pa vs (float4) + pb (float2) + key slot tmp perm id id_tmp wpos + nnb +
     // selfat + cls + nbr
-    return 9 * 16 + 8 + 7 * 4 + 4 + 1 + 1 + 1 + 16ull * ((max_pair - 1 + 3) / 4);  // list slots in whole quads
+    return 9 * 16 + 8 + 7 * 4 + 1 + 1 + 1 + 16ull * ((max_pair - 1 + 3) / 4);  // list slots in whole quads
 }
 
 // ---------------------------------------------------------------- batch --
@@ -191,7 +191,7 @@ Batch::~Batch()
     if (h_small_) cudaFreeHost(h_small_);
     void *ptrs[] = {d_scenes_, d_tile_scene_, d_tile_start_, d_ctrl_, d_scene_num_, d_flags_, d_x_, d_v_,
                     d_xs_, d_xa_, d_xb_, d_xold_, d_w_, d_pa_, d_pb_, d_vs_, d_tile_hdr_, d_key_, d_slot_, d_tmp_, d_perm_, d_count_,
-                    d_offsets_, d_bsum_, d_lam_, d_nbr_, d_nnb_, d_self_, d_bnd_, d_pack_off_, d_active_, d_id_, d_id_tmp_,
+                    d_offsets_, d_bsum_, d_nbr_, d_nnb_, d_self_, d_bnd_, d_pack_off_, d_active_, d_id_, d_id_tmp_,
                     d_next_id_, d_cls_, d_chist_, d_wpos_, d_dense_, d_mid_};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -240,7 +240,6 @@ pbf_status Batch::init(uint32_t max_scenes, uint64_t max_particles, uint64_t max
     CK(A((void **)&d_count_, 4 * (C + 4)));
     CK(A((void **)&d_offsets_, 4 * (C + 4)));
     CK(A((void **)&d_bsum_, 4 * ((C + kScanTile - 1) / kScanTile + 4)));
-    CK(A((void **)&d_lam_, 4 * P));
     CK(A((void **)&d_nbr_, 16ull * ((max_pair - 1 + 3) / 4) * P));  // quads of 4 slots per particle
     CK(A((void **)&d_nnb_, P));
     CK(A((void **)&d_self_, P));
@@ -838,7 +837,6 @@ StepArgs Batch::args() const
     a.chist = d_chist_;
     a.id_tmp = d_id_tmp_;
     a.next_id = d_next_id_;
-    a.lam = d_lam_;
     a.nbr = d_nbr_;
     a.nnb = d_nnb_;
     a.selfat = d_self_;

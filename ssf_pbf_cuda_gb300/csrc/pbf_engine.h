@@ -148,7 +148,6 @@ private:
     uint4 *d_tile_hdr_ = nullptr;                     // small steps' tile headers
     uint32_t *d_key_ = nullptr, *d_slot_ = nullptr, *d_tmp_ = nullptr, *d_perm_ = nullptr;
     uint32_t *d_count_ = nullptr, *d_offsets_ = nullptr, *d_bsum_ = nullptr;
-    float *d_lam_ = nullptr;
     uint32_t *d_nbr_ = nullptr;
     uint8_t *d_nnb_ = nullptr;
     uint8_t *d_self_ = nullptr;  // walk-order position of each particle in its own list

@@ -106,8 +106,7 @@ struct StepArgs {
     uint32_t *key, *slot, *tmp, *perm;
     uint32_t *count, *offsets, *bsum;
     // working slots: sorted slots, with a bucket of several alias classes grouped by class
-    float4 *xa, *xb, *xold;       // working positions (ping-pong), old x (.w = sorted slot)
-    float *lam;
+    float4 *xa, *xb, *xold;       // working positions, (position, lambda), old x (.w = sorted slot)
     uint32_t *nbr;                // neighbour lists, in rows of 16 bytes per working slot
     uint8_t *nnb;                 // list entries stored (the particle itself is not stored)
     uint8_t *selfat;              // position of the particle itself in its walk-order list, kNotListed if cut

@@ -6,9 +6,15 @@
 // with a fixed launch shape that a CUDA graph can capture once.
 //
 // Data layout (flat arrays over every scene's particle slots):
-//   x, v, xs, xa, xb, xold, w, vt : float4 (xyz + unused w), 16-byte aligned
+//   x, v                          : float4, the particles' state (xyz)
+//   xs                            : float4, sorted positions; later (x, |omega|)
+//   xa, xb                        : float4, working positions; (position, lambda)
+//   xold                          : float4, old position, sorted slot in w
+//   pa, pb                        : float4 + float2, (x, v) for the post passes
+//   w, vs                         : float4, vorticity; velocities in sorted order
 //   key, slot, tmp, perm          : uint32 per particle
-//   nbr                           : uint32 [slot k][particle i] (coalesced per k)
+//   nbr                           : rows of 16 bytes per particle (4 u32 or 8 u16
+//                                   list slots), row after row
 //   count / offsets               : uint32 per cell (+1 deleted bucket per scene)
 //
 // Integer work (predict, cell hash, stable counting sort, neighbour
@@ -18,7 +24,6 @@
 #include <map>
 #include <mutex>
 #include <tuple>
-#include <utility>
 
 #include "pbf_internal.h"
 #include "pbf_scan.cuh"
@@ -476,37 +481,6 @@ __device__ __forceinline__ uint32_t quad_at(const uint4 &v, int j)
     return j == 0 ? v.x : (j == 1 ? v.y : (j == 2 ? v.z : v.w));
 }
 
-// Visit list slots [0, nn) of one particle in list order.  Indices are
-// requested CH at a time (CH / 4 quads), one chunk ahead of their use; the
-// chunk (loads in flight against registers) is picked by the autotuner.
-// Whole chunks call f without per-slot predicates; only the quad requests
-// and the final partial chunk test against nn.
-template <int CH, class F>
-__device__ __forceinline__ void list_walk(const uint32_t *__restrict__ nl, uint64_t stride, uint32_t nn, F &&f)
-{
-    static_assert(CH % 4 == 0, "a chunk holds whole quads");
-    constexpr int NQ = CH / 4;
-    const uint4 *p = reinterpret_cast<const uint4 *>(nl);  // quad kq of the particle at p[kq * stride]
-    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    uint4 qn[NQ];
-#pragma unroll
-    for (int c = 0; c < NQ; ++c) qn[c] = ((uint32_t)(4 * c) < nn) ? list_ld(p + c * stride) : z;
-    uint32_t k0 = 0;
-    for (; k0 + CH <= nn; k0 += CH) {
-        uint4 q[NQ];
-#pragma unroll
-        for (int c = 0; c < NQ; ++c) q[c] = qn[c];
-        p += NQ * stride;
-#pragma unroll
-        for (int c = 0; c < NQ; ++c) qn[c] = (k0 + CH + 4 * c < nn) ? list_ld(p + c * stride) : z;
-#pragma unroll
-        for (int c = 0; c < CH; ++c) f(quad_at(q[c >> 2], c & 3));
-    }
-#pragma unroll
-    for (int c = 0; c < CH - 1; ++c)
-        if (k0 + c < nn) f(quad_at(qn[c >> 2], c & 3));
-}
-
 // Scenes of at most kList16Max particle slots (every batched scene) keep
 // their lists as u16 scene-local indices in octs of 8 slots: slot k of
 // particle slot i at nbr16[((k / 8) * stride + i) * 8 + k % 8], the same
@@ -524,14 +498,63 @@ __device__ __forceinline__ uint32_t oct_at(const uint4 &v, int j)
     return (j & 1) ? (w >> 16) : (w & 0xFFFFu);
 }
 
-// list_walk over a u16 list: octs requested one chunk (8 slots) ahead;
-// f gets base + the scene-local index: the particle's sorted slot for base
-// = the scene's first slot, the scene-local index itself for base = 0 (for
-// arrays offset by the scene's first slot, which saves the add per slot;
-// measured faster in the XSPH and vorticity-apply passes only).
-template <class F>
+// Visit slots [k0, k0 + n) of a particle's list: ld(q) loads the record of
+// index q, use(record, on) adds it.  All n records are requested before the
+// first is used; with PART only the first `left` slots are the list's, the
+// others load the particle's own record (self) and are used with on = false,
+// so a list's last slots cost one round trip together, not one each.  A list
+// of 30 neighbours ends in a partial chunk of 8 in most warps; with its slots
+// taken one by one (and the whole chunk's loads left to the compiler's order)
+// the passes at 256 scenes, 5.95 M particles, u16 lists, were: lambda 3 x 285,
+// delta-p 4 x 301, omega 448, and are 3 x 261, 4 x 291, 381 us.
+template <int N, bool PART, class IDX, class LD, class USE>
+__device__ __forceinline__ void list_group(uint32_t left, uint32_t self, IDX &&idx, LD &&ld, USE &&use)
+{
+    decltype(ld(0u)) rec[N];
+#pragma unroll
+    for (int c = 0; c < N; ++c) rec[c] = ld(!PART || (uint32_t)c < left ? idx(c) : self);
+#pragma unroll
+    for (int c = 0; c < N; ++c) use(rec[c], !PART || (uint32_t)c < left);
+}
+
+// Visit list slots [0, nn) of one particle in list order.  Indices are
+// requested CH at a time (CH / 4 quads), one chunk ahead of their use; the
+// chunk (loads in flight against registers) is picked by the autotuner.  The
+// last, partial chunk is taken in groups of four.
+template <int CH, class LD, class USE>
+__device__ __forceinline__ void list_walk(const uint32_t *__restrict__ nl, uint64_t stride, uint32_t nn, uint32_t self,
+                                          LD &&ld, USE &&use)
+{
+    constexpr int NQ = (CH + 3) / 4;  // (a u16 list's group of 2 compiles, unused, as one quad)
+    const uint4 *p = reinterpret_cast<const uint4 *>(nl);  // quad kq of the particle at p[kq * stride]
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    uint4 qn[NQ];
+#pragma unroll
+    for (int c = 0; c < NQ; ++c) qn[c] = ((uint32_t)(4 * c) < nn) ? list_ld(p + c * stride) : z;
+    uint32_t k0 = 0;
+    for (; k0 + CH <= nn; k0 += CH) {
+        uint4 q[NQ];
+#pragma unroll
+        for (int c = 0; c < NQ; ++c) q[c] = qn[c];
+        p += NQ * stride;
+#pragma unroll
+        for (int c = 0; c < NQ; ++c) qn[c] = (k0 + CH + 4 * c < nn) ? list_ld(p + c * stride) : z;
+        list_group<CH, false>(CH, self, [&](int c) { return quad_at(q[c >> 2], c & 3); }, ld, use);
+    }
+#pragma unroll
+    for (int c = 0; c < NQ; ++c)
+        if (k0 + 4 * c < nn)
+            list_group<4, true>(nn - k0 - 4 * c, self, [&](int e) { return quad_at(qn[c], e); }, ld, use);
+}
+
+// list_walk over a u16 list: octs requested one chunk (8 slots) ahead, the
+// records of G slots at a time; ld gets base + the scene-local index: the
+// working slot for base = the scene's first slot, the scene-local index itself
+// for base = 0 (for arrays offset by the scene's first slot, which saves the
+// add per slot; measured faster in the vorticity-apply pass only).
+template <int G, class LD, class USE>
 __device__ __forceinline__ void list_walk16(const uint32_t *__restrict__ nl, uint64_t stride, uint32_t nn,
-                                            uint32_t base, F &&f)
+                                            uint32_t base, uint32_t self, LD &&ld, USE &&use)
 {
     const uint4 *p = reinterpret_cast<const uint4 *>(nl);  // oct ko of the particle at p[ko * stride]
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
@@ -542,23 +565,25 @@ __device__ __forceinline__ void list_walk16(const uint32_t *__restrict__ nl, uin
         p += stride;
         qn = (k0 + 8 < nn) ? list_ld(p) : z;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) f(base + oct_at(q, c));
+        for (int h = 0; h < 8; h += G)
+            list_group<G, false>(G, self, [&](int c) { return base + oct_at(q, h + c); }, ld, use);
     }
 #pragma unroll
-    for (int c = 0; c < 7; ++c)
-        if (k0 + c < nn) f(base + oct_at(qn, c));
+    for (int h = 0; h < 8; h += 4)
+        if (k0 + h < nn)
+            list_group<4, true>(nn - k0 - h, self, [&](int c) { return base + oct_at(qn, h + c); }, ld, use);
 }
 
-// The list of one particle in either form: u32 quads (indices are sorted
+// The list of one particle in either form: u32 quads (indices are working
 // slots) or u16 octs (scene-local indices, base = the scene's first slot).
-template <int CH, class F>
-__device__ __forceinline__ void list_walk_any(bool l16, const uint32_t *__restrict__ nl, uint64_t stride,
-                                              uint32_t nn, uint32_t base, F &&f)
+template <int CH, class LD, class USE>
+__device__ __forceinline__ void list_walk_any(bool l16, const uint32_t *__restrict__ nl, uint64_t stride, uint32_t nn,
+                                              uint32_t base, uint32_t self, LD &&ld, USE &&use)
 {
     if (l16)
-        list_walk16(nl, stride, nn, base, f);
+        list_walk16<CH>(nl, stride, nn, base, self, ld, use);
     else
-        list_walk<CH>(nl, stride, nn, f);
+        list_walk<CH>(nl, stride, nn, self, ld, use);
 }
 
 // Small, latency-bound steps: a pass's time is one thread's chain of dependent
@@ -1346,7 +1371,7 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
             lam_add(ls, xp, __ldg(xa + q), pc);
         }
     }
-    a.lam[i] = ls.lambda(d);
+    a.xb[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));  // the first delta-p pass gathers both
     TILE_LOOP_END
 }
 
@@ -1665,9 +1690,10 @@ __global__ void __launch_bounds__(kSplitBlock, 3) k_neighbors_split(StepArgs a, 
 // lambda for iterations >= 1 (memorizeKernelCalc + calcScalingFactor,
 // pbf_kernel_memorization.cu:93-134 and pbf_constraint.cu:168-209, without the
 // per-pair cache: W and grad W are recomputed from positions).  One thread
-// per particle; the neighbour sums run in list order.
+// per particle; the neighbour sums run in list order.  (position, lambda) goes
+// into the other buffer, which the delta-p pass gathers.
 template <int kChunk>
-__global__ void __launch_bounds__(512, 2) k_lambda(StepArgs a, float4 *__restrict__ xc)
+__global__ void __launch_bounds__(512, 2) k_lambda(StepArgs a, const float4 *__restrict__ xc, float4 *__restrict__ xo)
 {
     TILE_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
@@ -1679,16 +1705,17 @@ __global__ void __launch_bounds__(512, 2) k_lambda(StepArgs a, float4 *__restric
     const float4 xp = xc[i];
     LamSum ls;
     if (a.selfat[i] != kNotListed) ls.ks = 1.f;  // the particle's own w(0), not stored in the list
-    list_walk_any<kChunk>(d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off,
-                          [&](uint32_t q) { lam_add(ls, xp, __ldg(xc + q), pc); });
-    // lambda rides in .w of the positions this pass reads and the delta-p
-    // pass gathers next (neighbours here use only .xyz)
-    reinterpret_cast<float *>(xc + i)[3] = ls.lambda(d);
+    list_walk_any<kChunk>(
+        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        [&](uint32_t q) -> float4 { return __ldg(xc + q); },
+        [&](const float4 &xj, bool on) {
+            const PairGeo g = pair_geo(xp, xj);
+            ls.add(g, masked(pair_ws(g.r2, pc), on));
+        });
+    xo[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));
     TILE_LOOP_END
 }
 
-// Small steps: (position, lambda) into the other buffer, which the delta-p
-// pass gathers.
 __global__ void __launch_bounds__(kSmallBlock, 8) k_lambda_small(StepArgs a, uint32_t tile,
                                                                  const float4 *__restrict__ xc,
                                                                  float4 *__restrict__ xo)
@@ -1802,37 +1829,6 @@ __device__ __forceinline__ void dp_finish(const StepArgs &a, const SceneDesc &d,
         xo[i] = xn;
 }
 
-// Sum over the list of -(lambda_i + lambda_j + s_corr) grad W (the body of
-// calcPositionUpdateCUDA, pbf_position_update.cu:131-188), in list order:
-// each pair adds (coefficient * s) d.  LAMW: lambda in .w of the positions
-// (iterations >= 1 of large steps; their iteration 0 reads it from lam), and
-// the x and y differences and sums by one packed operation each (the same
-// bits; measured faster there only).
-template <int kChunk, int FORM, bool LAMW>
-__device__ __forceinline__ float3 dp_sum(const StepArgs &a, const SceneDesc &d, const float4 *__restrict__ xc,
-                                         uint32_t i, float4 xp, float li)
-{
-    const PairConst pc = pair_const(d);
-    const ScorrConst sc = scorr_const(d, li);
-    const float *__restrict__ lam = a.lam;
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-    list_walk_any<kChunk>(d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, [&](uint32_t q) {
-        const float4 xq = __ldg(xc + q);
-        const PairGeo g = pair_geo<LAMW>(xp, xq);
-        const PairWS k = pair_ws(g.r2, pc);
-        const float lj = LAMW ? xq.w : __ldg(lam + q);
-        const float f = __fmul_rn(dp_coef<FORM>(li, lj, k.W, sc), k.s);
-        if (LAMW) {
-            fma2(s0, s1, f, f, g.d0, g.d1);
-        } else {
-            s0 = __fmaf_rn(f, g.d0, s0);
-            s1 = __fmaf_rn(f, g.d1, s1);
-        }
-        s2 = __fmaf_rn(f, g.d2, s2);
-    });
-    return make_float3(s0, s1, s2);
-}
-
 // The s_corr form once per tile (a tile belongs to one scene): f<FORM>().
 template <class F>
 __device__ __forceinline__ float3 by_scorr(const SceneDesc &d, F &&f)
@@ -1843,8 +1839,36 @@ __device__ __forceinline__ float3 by_scorr(const SceneDesc &d, F &&f)
     return f(std::integral_constant<int, kScorrOff>());
 }
 
-// delta-p with s_corr (calcPositionUpdateCUDA cached, pbf_position_update.cu:131-188).
-template <int kChunk, bool LAMW>
+// One pair's share of the sum of -(lambda_i + lambda_j + s_corr) grad W (the
+// body of calcPositionUpdateCUDA, pbf_position_update.cu:131-188): adds
+// (coefficient * s) d.  Lambdas in .w.  PK: the x and y differences and sums by
+// one packed operation each (the same bits; measured faster in large steps only).
+template <int FORM, bool PK>
+struct DpSum {
+    float4 xp;
+    PairConst pc;
+    ScorrConst sc;
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+    __device__ __forceinline__ DpSum(const SceneDesc &d, float4 x) : xp(x), pc(pair_const(d)), sc(scorr_const(d, x.w)) {}
+    __device__ __forceinline__ void add(const float4 &xq, bool on)
+    {
+        const PairGeo g = pair_geo<PK>(xp, xq);
+        const PairWS k = pair_ws(g.r2, pc);
+        const float f0 = __fmul_rn(dp_coef<FORM>(xp.w, xq.w, k.W, sc), k.s);
+        const float f = on ? f0 : 0.f;
+        if (PK) {
+            fma2(s0, s1, f, f, g.d0, g.d1);
+        } else {
+            s0 = __fmaf_rn(f, g.d0, s0);
+            s1 = __fmaf_rn(f, g.d1, s1);
+        }
+        s2 = __fmaf_rn(f, g.d2, s2);
+    }
+};
+
+// delta-p with s_corr (calcPositionUpdateCUDA cached, pbf_position_update.cu:131-188),
+// in list order.
+template <int kChunk>
 __global__ void __launch_bounds__(512, 2) k_dp(StepArgs a, const float4 *__restrict__ xc, float4 *__restrict__ xo,
                                                int last)
 {
@@ -1856,36 +1880,29 @@ __global__ void __launch_bounds__(512, 2) k_dp(StepArgs a, const float4 *__restr
     if (local >= live) continue;
     const uint32_t i = d.p_off + local;
     const float4 xp = xc[i];
-    const float li = LAMW ? xp.w : a.lam[i];
-    const float3 sum = by_scorr(d, [&](auto form) { return dp_sum<kChunk, decltype(form)::value, LAMW>(a, d, xc, i, xp, li); });
+    const float3 sum = by_scorr(d, [&](auto form) {
+        DpSum<decltype(form)::value, true> o(d, xp);
+        list_walk_any<kChunk>(
+            d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+            [&](uint32_t q) -> float4 { return __ldg(xc + q); }, [&](const float4 &xq, bool on) { o.add(xq, on); });
+        return make_float3(o.s0, o.s1, o.s2);
+    });
     dp_finish(a, d, s, i, xp, sum, xo, last);
     TILE_LOOP_END
 }
 
-// Small steps: (position, lambda) gathered together.
 __global__ void __launch_bounds__(kSmallBlock, 8) k_dp_small(StepArgs a, uint32_t tile, const float4 *__restrict__ xc,
                                                              float4 *__restrict__ xo, int last)
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
     const float4 xp = xc[i];
-    const PairConst pc = pair_const(d);
-    const ScorrConst sc = scorr_const(d, xp.w);
     const float3 sum = by_scorr(d, [&](auto form) {
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+        DpSum<decltype(form)::value, false> o(d, xp);
         list_walk_wide(
             d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
-            [&](uint32_t q) -> float4 { return __ldg(xc + q); },
-            [&](const float4 &xq, bool on) {
-                const PairGeo g = pair_geo(xp, xq);
-                const PairWS k = pair_ws(g.r2, pc);
-                const float f0 = __fmul_rn(dp_coef<decltype(form)::value>(xp.w, xq.w, k.W, sc), k.s);
-                const float f = on ? f0 : 0.f;
-                s0 = __fmaf_rn(f, g.d0, s0);
-                s1 = __fmaf_rn(f, g.d1, s1);
-                s2 = __fmaf_rn(f, g.d2, s2);
-            });
-        return make_float3(s0, s1, s2);
+            [&](uint32_t q) -> float4 { return __ldg(xc + q); }, [&](const float4 &xq, bool on) { o.add(xq, on); });
+        return make_float3(o.s0, o.s1, o.s2);
     });
     dp_finish(a, d, s, i, xp, sum, xo, last);
     SMALL_LOOP_END
@@ -1905,6 +1922,12 @@ __global__ void __launch_bounds__(512) k_finalize(StepArgs a)
     put_final(a, d, i, make_float4(xn.x, xn.y, xn.z, 0.f));
     TILE_LOOP_END
 }
+
+// A neighbour's (x, v) as the list passes load it.
+struct PhaseRec {
+    float4 A;
+    float2 B;
+};
 
 // Vorticity, pass 1 (calcVorticityCUDA, pbf_vorticity_confinement.cu:87-115):
 // omega_i = m/rho0 * sum_j (v_j - v_i) x r_hat * W'(r).
@@ -1942,7 +1965,7 @@ __device__ __forceinline__ void put_omega(const StepArgs &a, const SceneDesc &d,
 // skips the other format's scenes) keeps its registers, and so its
 // occupancy, to that format's loop.
 template <bool L16>
-__global__ void __launch_bounds__(512) k_vort_omega(StepArgs a)
+__global__ void __launch_bounds__(512, 2) k_vort_omega(StepArgs a)
 {
     TILE_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
@@ -1956,20 +1979,15 @@ __global__ void __launch_bounds__(512) k_vort_omega(StepArgs a)
     OmegaSum o(A, make_float4(A.w, B.x, B.y, 0.f), d.inv_h);
     const float4 *__restrict__ pa = a.pa;
     const float2 *__restrict__ pb = a.pb;
-    list_walk_any<4>(L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, [&](uint32_t q) {
-        const float4 xj = __ldg(pa + q);
-        const float2 vj = __ldg(pb + q);
-        o.add(xj, xj.w, vj.x, vj.y);
-    });
+    // groups of 4 in 64 registers: 381 us (u16, 5.95 M particles) and 80 us
+    // (u32, 1 M); groups of 8 hold 48 record registers and take 550 us
+    list_walk_any<4>(
+        L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; },
+        [&](const PhaseRec &r, bool on) { o.add(r.A, r.A.w, r.B.x, r.B.y, on); });
     put_omega(a, d, i, o);
     TILE_LOOP_END
 }
-
-// A neighbour's (x, v) as the small steps' passes load it.
-struct PhaseRec {
-    float4 A;
-    float2 B;
-};
 
 __global__ void __launch_bounds__(kSmallBlock, 8) k_vort_omega_small(StepArgs a, uint32_t tile)
 {
@@ -2062,7 +2080,7 @@ __device__ __forceinline__ void put_confinement(const StepArgs &a, const SceneDe
 }
 
 template <bool L16>
-__global__ void __launch_bounds__(512) k_vort_apply(StepArgs a)
+__global__ void __launch_bounds__(512, 2) k_vort_apply(StepArgs a)
 {
     TILE_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
@@ -2074,7 +2092,12 @@ __global__ void __launch_bounds__(512) k_vort_apply(StepArgs a)
     // u16 lists index the array offset by the scene's first slot (no add per slot)
     const float4 *__restrict__ xw = a.xs + (L16 ? d.p_off : 0u);
     EtaSum e(a.xs[i], d.inv_h, -1.f);
-    list_walk_any<4>(L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], 0u, [&](uint32_t q) { e.add(__ldg(xw + q)); });
+    // u16 in groups of 2: 282 us at 5.95 M particles (286 by 4, 294 by 8, 274
+    // slot by slot); u32 by 4: 59 us at 1 M (62 slot by slot); 128 against
+    // 150 us for a batch with both formats
+    list_walk_any<(L16 ? 2 : 4)>(
+        L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], 0u, L16 ? i - d.p_off : i,
+        [&](uint32_t q) -> float4 { return __ldg(xw + q); }, [&](const float4 &xj, bool on) { e.add(xj, on); });
     put_confinement(a, d, i, e);
     TILE_LOOP_END
 }
@@ -2137,7 +2160,7 @@ __global__ void __launch_bounds__(512) k_vort_apply_walk(StepArgs a)
 // XSPH (calcXSPHCUDA, pbf_xsph.cu:84-113): v_i += c m/rho0 sum_j (v_j - v_i) W(r_ij),
 // NaN guard.  Bound by the L1 wavefronts of its gathers: a neighbour's
 // position and velocity as 16 + 8 bytes instead of two float4 took the list
-// form from 446 to 355 us at 5.95 M particles (u16 lists), 96 to 77 us at
+// form from 446 to 358 us at 5.95 M particles (u16 lists), 96 to 75 us at
 // 1,048,576 (u32 lists).
 struct XsphSum {
     float4 xi, vi;
@@ -2188,11 +2211,11 @@ __global__ void __launch_bounds__(512) k_xsph(StepArgs a)
     const float4 A = a.pa[i];
     const float2 B = a.pb[i];
     XsphSum o(A, make_float4(A.w, B.x, B.y, 0.f), d);
-    list_walk_any<4>(L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, [&](uint32_t q) {
-        const float4 xj = __ldg(pa + q);
-        const float2 vj = __ldg(pb + q);
-        o.add(xj, xj.w, vj.x, vj.y);
-    });
+    // groups of 8: 358 us (u16, 5.95 M particles) and 75 us (u32, 1 M), 372 and 77 in groups of 4
+    list_walk_any<8>(
+        L16, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
+        [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; },
+        [&](const PhaseRec &r, bool on) { o.add(r.A, r.A.w, r.B.x, r.B.y, on); });
     a.v[__float_as_uint(a.xold[i].w)] = o.result(d);
     TILE_LOOP_END
 }
@@ -2375,19 +2398,14 @@ __global__ void k_store_phase(const float4 *__restrict__ x, const float4 *__rest
 template <int CH>
 struct PassFns {
     static const void *lambda() { return (const void *)k_lambda<CH>; }
-    static const void *dp() { return (const void *)k_dp<CH, true>; }
-    static void launch_lambda(const StepArgs &a, const LaunchShape &sh, float4 *cur, cudaStream_t st)
+    static const void *dp() { return (const void *)k_dp<CH>; }
+    static void launch_lambda(const StepArgs &a, const LaunchShape &sh, cudaStream_t st)
     {
-        k_lambda<CH><<<sh.grid_lambda, sh.tile, 0, st>>>(a, cur);
+        k_lambda<CH><<<sh.grid_lambda, sh.tile, 0, st>>>(a, a.xa, a.xb);
     }
-    // lamw: lambda in .w of cur (iterations >= 1); iteration 0 reads it from lam
-    static void launch_dp(const StepArgs &a, const LaunchShape &sh, const float4 *cur, float4 *out, int last,
-                          bool lamw, cudaStream_t st)
+    static void launch_dp(const StepArgs &a, const LaunchShape &sh, int last, cudaStream_t st)
     {
-        if (lamw)
-            k_dp<CH, true><<<sh.grid_dp, sh.tile, 0, st>>>(a, cur, out, last);
-        else
-            k_dp<CH, false><<<sh.grid_dp, sh.tile, 0, st>>>(a, cur, out, last);
+        k_dp<CH><<<sh.grid_dp, sh.tile, 0, st>>>(a, a.xb, a.xa, last);
     }
 };
 
@@ -2587,26 +2605,22 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
             k_neighbors_lambda<false><<<sh.grid_nb, b, 0, st>>>(a);
         PBF_LAUNCHED("k_neighbors_lambda");
     }
-    if (sh.small) {  // (position, lambda) in xb, positions in xa
-        for (int it = 0; it < iters; ++it) {
-            if (it > 0) {
+    for (int it = 0; it < iters; ++it) {  // positions in xa, (position, lambda) in xb
+        const int last = it == iters - 1 ? 1 : 0;
+        if (it > 0) {
+            if (sh.small) {
                 k_lambda_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile, a.xa, a.xb);
-                PBF_LAUNCHED("k_lambda");
+            } else {
+                PBF_PASS_DISPATCH(sh.chunk, launch_lambda(a, sh, st));
             }
-            k_dp_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile, a.xb, a.xa, it == iters - 1 ? 1 : 0);
-            PBF_LAUNCHED("k_dp");
+            PBF_LAUNCHED("k_lambda");
         }
-    } else {
-        float4 *cur = a.xa, *nxt = a.xb;
-        for (int it = 0; it < iters; ++it) {
-            if (it > 0) {
-                PBF_PASS_DISPATCH(sh.chunk, launch_lambda(a, sh, cur, st));
-                PBF_LAUNCHED("k_lambda");
-            }
-            PBF_PASS_DISPATCH(sh.chunk, launch_dp(a, sh, cur, nxt, it == iters - 1 ? 1 : 0, it > 0, st));
-            PBF_LAUNCHED("k_dp");
-            std::swap(cur, nxt);
+        if (sh.small) {
+            k_dp_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile, a.xb, a.xa, last);
+        } else {
+            PBF_PASS_DISPATCH(sh.chunk, launch_dp(a, sh, last, st));
         }
+        PBF_LAUNCHED("k_dp");
     }
     if (iters <= 0) {
         k_finalize<<<g, b, 0, st>>>(a);
