@@ -168,6 +168,9 @@ pbf_status pbf_create(const pbf_params *params, uint32_t capacity, const float d
     const float amin[3] = {-big, -big, -big}, amax[3] = {big, big, big};
     uint32_t id = 0;
     rc = h->b.add_scene(*params, capacity, domain_end, nullptr, amin, amax, nullptr, nullptr, 0, false, 0, &id);
+    // the scene's counters are cleared on the default stream, which the
+    // caller's streams need not wait for
+    if (rc == PBF_SUCCESS && cudaStreamSynchronize(0) != cudaSuccess) rc = PBF_ERROR_CUDA;
     if (rc != PBF_SUCCESS) {
         delete h;
         return rc;

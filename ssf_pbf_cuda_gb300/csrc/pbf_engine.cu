@@ -263,6 +263,7 @@ pbf_status Batch::init(uint32_t max_scenes, uint64_t max_particles, uint64_t max
     CK(cudaMemset(d_self_, kNotListed, P));
     CK(cudaMemset(d_v_, 0, 16 * P));
     CK(cudaMemset(d_x_, 0, 16 * P));
+    CK(cudaStreamSynchronize(0));  // the first use may be on a stream that does not wait for this one
     CK(cudaStreamCreateWithFlags(&cap_stream_, cudaStreamNonBlocking));
     palloc_.reset(P);
     calloc_.reset(C);
