@@ -251,7 +251,7 @@ pbf_status Batch::init(uint32_t max_scenes, uint64_t max_particles, uint64_t max
     CK(A((void **)&d_pack_off_, 4ull * max_scenes));
     CK(A((void **)&d_active_, 4ull * max_scenes));
     CK(A((void **)&d_pin_, sizeof(PackedIn)));
-    CK(cudaMallocHost((void **)&h_small_, 8ull * max_scenes + 64));
+    CK(cudaMallocHost((void **)&h_small_, 12ull * max_scenes + 64));
     CK(cudaEventCreateWithFlags(&small_done_, cudaEventDisableTiming));
     CK(cudaMemset(d_count_, 0, 4 * (C + 4)));
     CK(cudaMemset(d_offsets_, 0, 4 * (C + 4)));
@@ -1026,20 +1026,55 @@ pbf_status Batch::get_num(uint32_t id, uint32_t *num, cudaStream_t st)
     return PBF_SUCCESS;
 }
 
+// A scene's particles into device arrays; waits until the stream has come to
+// the copy (all before it is done, the copy itself may be in flight) and
+// takes over the count.  The copy is enqueued before the wait, bounded by the
+// host's upper bound and by the count on the device, and its first block
+// writes the count to pinned memory, which the host polls.  A 4-byte copy to
+// the host, its wait and only then the launch left the GPU idle meanwhile:
+// set, step and get of 4,096 particles 97 us so, 87 us now (91 with a stream
+// synchronisation in place of the poll); 32,768 particles 122 and 108.
+pbf_status Batch::store_device(uint32_t id, float *x, float *v, uint32_t *num, cudaStream_t st)
+{
+    if (id >= scenes_.size() || !scenes_[id].active) return PBF_ERROR_NOT_FOUND;
+    CK(cudaSetDevice(device_));
+    SceneHost &s = scenes_[id];
+    uint32_t n = 0;
+    volatile uint32_t *slot = h_small_ + 2ull * max_scenes_ + id;
+    if (s.num_upper) {
+        constexpr uint32_t kUnset = 0xFFFFFFFFu;  // no count: capacities lie below
+        *slot = kUnset;
+        launch_store_phase(d_x_ + s.desc.p_off, d_v_ + s.desc.p_off, x, v, s.num_upper, st, d_scene_num_ + id, slot);
+        CK(cudaGetLastError());
+        uint32_t polls = 0;
+        while ((n = *slot) == kUnset)
+            if ((++polls & 1023u) == 0 && cudaStreamQuery(st) != cudaErrorNotReady) break;
+        if (n != kUnset || (n = *slot) != kUnset) {
+            if (n != s.num_upper) {
+                s.num_upper = n;
+                dirty_tiles_ = true;
+            }
+            if (num) *num = n;
+            return PBF_SUCCESS;
+        }
+    }
+    // no particles, or the stream ended without a count (an error, or another
+    // thread's call took the slot)
+    const pbf_status rc = get_num(id, &n, st);
+    if (rc == PBF_SUCCESS && num) *num = n;
+    return rc;
+}
+
 pbf_status Batch::get_particles(uint32_t id, float *x, float *v, uint32_t *num, bool dst_dev, cudaStream_t st)
 {
     uint32_t n = 0;
+    if (dst_dev) return store_device(id, x, v, num, st);
     pbf_status rc = get_num(id, &n, st);
     if (rc != PBF_SUCCESS) return rc;
     if (num) *num = n;
     if (!n) return PBF_SUCCESS;
     const SceneHost &s = scenes_[id];
     const float4 *sx = d_x_ + s.desc.p_off, *sv = d_v_ + s.desc.p_off;
-    if (dst_dev) {
-        launch_store_phase(sx, sv, x, v, n, st);
-        CK(cudaGetLastError());
-        return PBF_SUCCESS;
-    }
     // the scene's slices of xs and pa are free between steps
     float *stx = reinterpret_cast<float *>(d_xs_ + s.desc.p_off), *stv = reinterpret_cast<float *>(d_pa_ + s.desc.p_off);
     launch_store_phase(sx, sv, x ? stx : nullptr, v ? stv : nullptr, n, st);
@@ -1158,12 +1193,7 @@ pbf_status Batch::import_x_device(uint32_t id, const float *x_dev, uint32_t n, c
 
 pbf_status Batch::export_x_device(uint32_t id, float *x_dev, cudaStream_t st)
 {
-    uint32_t n = 0;
-    pbf_status rc = get_num(id, &n, st);
-    if (rc != PBF_SUCCESS) return rc;
-    launch_store_phase(d_x_ + scenes_[id].desc.p_off, nullptr, x_dev, nullptr, n, st);
-    CK(cudaGetLastError());
-    return PBF_SUCCESS;
+    return store_device(id, x_dev, nullptr, nullptr, st);
 }
 
 pbf_status Batch::set_tile(uint32_t tile)

@@ -70,6 +70,7 @@ public:
     // step reads the packed input where it lies
     pbf_status step_packed(int iters, const uint32_t *counts, const float *x, const float *v, cudaStream_t st);
     pbf_status get_num(uint32_t id, uint32_t *num, cudaStream_t st);
+    pbf_status store_device(uint32_t id, float *x, float *v, uint32_t *num, cudaStream_t st);
     pbf_status get_particles(uint32_t id, float *x, float *v, uint32_t *num, bool dst_dev, cudaStream_t st);
     pbf_status get_flags(uint32_t id, uint32_t *flags, bool clear, cudaStream_t st);
     // live counts and flag words of every scene slot with one device read
@@ -162,7 +163,7 @@ private:
     uint32_t *d_wpos_ = nullptr;                      // sorted slot -> working slot
     uint32_t *d_dense_ = nullptr;                     // dense-bucket queue
     uint32_t *d_mid_ = nullptr;                       // medium-bucket queue
-    uint32_t *h_small_ = nullptr;     // pinned host scratch: pack offsets + counts
+    uint32_t *h_small_ = nullptr;     // pinned host scratch: pack offsets + counts + counts stored by the device
     cudaEvent_t small_done_ = nullptr;
     uint64_t bnd_capacity_ = 0;
     uint64_t max_tiles_ = 0;

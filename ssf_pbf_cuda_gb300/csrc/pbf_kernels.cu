@@ -2371,11 +2371,17 @@ __global__ void k_load_phase(const float *__restrict__ sx, const float *__restri
     id[i] = first + i;
 }
 
-// Either or both of x, v narrowed for the caller.
+// Either or both of x, v narrowed for the caller.  num: the particle count on
+// the device (n is then its bound), written to num_out, pinned host memory.
 __global__ void k_store_phase(const float4 *__restrict__ x, const float4 *__restrict__ v, float *__restrict__ dx,
-                              float *__restrict__ dv, uint32_t n)
+                              float *__restrict__ dv, uint32_t n, const uint32_t *__restrict__ num,
+                              volatile uint32_t *num_out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (num) {
+        n = min(n, __ldg(num));
+        if (i == 0) *num_out = n;
+    }
     if (i >= n) return;
     if (dx) {
         const float4 t = x[i];
@@ -2472,9 +2478,10 @@ void launch_load_phase(const float *sx, const float *sv, float4 *x, float4 *v, u
                                                           scene_num, n, total);
 }
 
-void launch_store_phase(const float4 *x, const float4 *v, float *dx, float *dv, uint32_t n, cudaStream_t st)
+void launch_store_phase(const float4 *x, const float4 *v, float *dx, float *dv, uint32_t n, cudaStream_t st,
+                        const uint32_t *num, volatile uint32_t *num_out)
 {
-    if (n) k_store_phase<<<(n + 255) / 256, 256, 0, st>>>(x, v, dx, dv, n);
+    if (n) k_store_phase<<<(n + 255) / 256, 256, 0, st>>>(x, v, dx, dv, n, num, num_out);
 }
 
 void launch_set_u32(uint32_t *dst, uint32_t value, cudaStream_t st) { k_set_u32<<<1, 1, 0, st>>>(dst, value); }
