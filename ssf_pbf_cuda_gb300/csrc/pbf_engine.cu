@@ -222,8 +222,9 @@ pbf_status Batch::init(uint32_t max_scenes, uint64_t max_particles, uint64_t max
         return cudaMalloc(p, bytes ? bytes : 16);
     };
     CK(A((void **)&d_scenes_, sizeof(SceneDesc) * max_scenes));
-    CK(A((void **)&d_tile_scene_, 4 * max_tiles_));
-    CK(A((void **)&d_tile_start_, 4 * max_tiles_));
+    // + kSmallTiles: small steps read entries past the last tile (never used)
+    CK(A((void **)&d_tile_scene_, 4 * (max_tiles_ + kSmallTiles)));
+    CK(A((void **)&d_tile_start_, 4 * (max_tiles_ + kSmallTiles)));
     CK(A((void **)&d_ctrl_, sizeof(Ctrl)));
     CK(A((void **)&d_scene_num_, 4ull * max_scenes));
     CK(A((void **)&d_flags_, 4ull * max_scenes));
@@ -804,6 +805,19 @@ LaunchShape Batch::shape_for(uint32_t tile) const
         sh.scan_grid = 0;
         sh.scan_cluster = lim;
         sh.scan_rounds = r;
+    }
+    // everything before the walk in one cluster, a particle a thread (16,384
+    // slots: 84 against 88 us for 4,096 particles; more would need two a thread,
+    // which loses)
+    sh.front = sh.front_cluster = 0;
+    sh.tile_shift = 0;
+    while ((1u << sh.tile_shift) < tile) ++sh.tile_shift;
+    if (sh.small && (uint64_t)ntb * tile <= lim * 1024u && max_particles_ <= kFrontSlots) {
+        const uint32_t r = cluster_scan_rounds(cells, lim);
+        if (r && r <= kFrontRounds) {
+            sh.front = r;
+            sh.front_cluster = lim;
+        }
     }
     return sh;
 }

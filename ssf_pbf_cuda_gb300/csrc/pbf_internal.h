@@ -143,6 +143,9 @@ struct LaunchShape {
     uint32_t cell_tile;   // cells per cell tile = threads per k_rank_cells block (autotuned)
     uint32_t small;       // latency-bound step (at most kSmallStep particle slots): split
                           // neighbour walk, per-particle rank, wide list reads
+    uint32_t front;       // small steps: k_front's rounds of 1024 cells a block, 0 = a kernel per phase
+    uint32_t front_cluster; // blocks of its cluster
+    uint32_t tile_shift;  // log2 of tile
     uint32_t small_split; // small steps: their walk takes kSplit lanes a particle
     uint32_t small_tiles; // small steps: tiles rounded up to a power of two, for which headers are written
     uint32_t nb_smem;     // k_neighbors_lambda: bytes of shared memory for the block's lists (0 = stored directly)
@@ -151,6 +154,7 @@ struct LaunchShape {
         return tile == o.tile && grid == o.grid && scan_grid == o.scan_grid && scan_rounds == o.scan_rounds && scan_cluster == o.scan_cluster &&
                chunk == o.chunk &&
                grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && small_tiles == o.small_tiles && small_split == o.small_split && nb_smem == o.nb_smem &&
+               front == o.front && front_cluster == o.front_cluster &&
                grid_nb == o.grid_nb && grid_lambda == o.grid_lambda && grid_dp == o.grid_dp &&
                grid_omega[0] == o.grid_omega[0] && grid_omega[1] == o.grid_omega[1] && grid_apply[0] == o.grid_apply[0] &&
                grid_apply[1] == o.grid_apply[1] && grid_xsph[0] == o.grid_xsph[0] && grid_xsph[1] == o.grid_xsph[1];
@@ -235,6 +239,8 @@ constexpr uint32_t kSmallTiles = 2048;      // tiles a small step may have, roun
 static_assert(kSmallTiles >= kSmallStep / 64, "a header per tile of a small step");
 // shared memory of their walk beside the lists: per warp 27 ranges of up to 32 cells and the cells' coordinates
 constexpr uint32_t kSmallWalkSmem = kSmallBlock / 32 * (32 * 27 * 8 + 96 * 4);
+constexpr uint64_t kFrontSlots = 1u << 29;  // k_front: particle slots at most (indices beside an alias class)
+constexpr uint32_t kFrontRounds = 4;        // k_front: rounds of 1024 cells a block at most (1, 2 or 4)
 constexpr uint32_t kSplit = 4;              // lanes a particle in the smallest steps' walk
 constexpr uint32_t kSplitBlock = kSplit * kSmallBlock;
 // Particle slots up to which the walk is split: 15,000 particles 76 us a step

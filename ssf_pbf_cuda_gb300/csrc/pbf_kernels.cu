@@ -24,6 +24,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <utility>
 
 #include "pbf_internal.h"
 #include "pbf_scan.cuh"
@@ -663,34 +664,41 @@ __device__ __forceinline__ void list_walk_wide(bool l16, const uint32_t *__restr
 // PACKED: the input phase is read from the packed AoS float3 buffers of a
 // packed-input step (what k_unpack would have written), and the particles
 // are numbered afresh.
-template <bool PACKED>
-__global__ void __launch_bounds__(512) k_predict_hash(StepArgs a)
-{
-    TILE_LOOP_BEGIN
-    const uint32_t n = a.scene_num[s];
-    if (local >= n) continue;
-    const SceneDesc d = a.scenes[s];
-    const uint32_t i = d.p_off + local;
-    float4 xv, vv;
+struct PhaseIn {
+    float4 x, v;
     uint32_t id;
+};
+template <bool PACKED>
+__device__ __forceinline__ PhaseIn load_phase(const StepArgs &a, const SceneDesc &d, uint32_t s, uint32_t local)
+{
     if (PACKED) {
         const PackedIn pin = *a.pin;
         const uint64_t q = 3ull * ((uint64_t)a.pack_off[s] + local);
-        xv = make_float4(pin.x[q], pin.x[q + 1], pin.x[q + 2], 0.f);
-        vv = pin.v ? make_float4(pin.v[q], pin.v[q + 1], pin.v[q + 2], 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
-        id = local;
-        if (local == 0) a.next_id[s] = n;
-    } else {
-        xv = a.x[i];
-        vv = a.v[i];
-        id = a.id[i];
+        return PhaseIn{make_float4(pin.x[q], pin.x[q + 1], pin.x[q + 2], 0.f),
+                       pin.v ? make_float4(pin.v[q], pin.v[q + 1], pin.v[q + 2], 0.f) : make_float4(0.f, 0.f, 0.f, 0.f),
+                       local};
     }
+    const uint32_t i = d.p_off + local;
+    return PhaseIn{a.x[i], a.v[i], a.id[i]};
+}
+
+struct Predicted {
+    float4 ps;  // .w: the id
+    uint32_t key, cls;
+};
+template <bool PACKED>
+__device__ __forceinline__ Predicted predict_particle(const StepArgs &a, const SceneDesc &d, uint32_t s,
+                                                      uint32_t local, uint32_t n, const PhaseIn &in)
+{
+    if (PACKED && local == 0) a.next_id[s] = n;
+    const float4 xv = in.x, vv = in.v;
+    const uint32_t id = in.id;
     const float dt = d.dt;
     float4 ps;
     ps.x = __fmaf_rn(__fmaf_rn(d.g[0], dt, vv.x), dt, xv.x);
     ps.y = __fmaf_rn(__fmaf_rn(d.g[1], dt, vv.y), dt, xv.y);
     ps.z = __fmaf_rn(__fmaf_rn(d.g[2], dt, vv.z), dt, xv.z);
-    ps.w = __uint_as_float(id);  // the id travels with the prediction to k_gather
+    ps.w = __uint_as_float(id);  // the id travels with the prediction to the gather
     const int32_t cx = cell_coord(ps.x, d.cw), cy = cell_coord(ps.y, d.cw), cz = cell_coord(ps.z, d.cw);
     uint32_t key = hash3((uint32_t)cx, (uint32_t)cy, (uint32_t)cz, d);
     uint32_t cls = alias_class(cx, cy, cz, d);
@@ -699,11 +707,23 @@ __global__ void __launch_bounds__(512) k_predict_hash(StepArgs a)
         key = d.ncell;
         cls = 0;
     }
-    a.cls[i] = (uint8_t)cls;
     if (!(isfinite(ps.x) && isfinite(ps.y) && isfinite(ps.z))) atomicOr(a.flags + s, PBF_FLAG_NONFINITE);
-    a.xs[i] = ps;
-    a.key[i] = key;
-    a.slot[i] = atomicAdd(a.count + d.c_off + key, 1u);
+    return Predicted{ps, key, cls};
+}
+
+template <bool PACKED>
+__global__ void __launch_bounds__(512) k_predict_hash(StepArgs a)
+{
+    TILE_LOOP_BEGIN
+    const uint32_t n = a.scene_num[s];
+    if (local >= n) continue;
+    const SceneDesc d = a.scenes[s];
+    const Predicted p = predict_particle<PACKED>(a, d, s, local, n, load_phase<PACKED>(a, d, s, local));
+    const uint32_t i = d.p_off + local;
+    a.cls[i] = (uint8_t)p.cls;
+    a.xs[i] = p.ps;
+    a.key[i] = p.key;
+    a.slot[i] = atomicAdd(a.count + d.c_off + p.key, 1u);
     TILE_LOOP_END
 }
 
@@ -830,7 +850,7 @@ __global__ void __launch_bounds__(1024) k_scan_cluster(StepArgs a)
         *a.dense = 0;  // the bucket queues of this step's rank kernel
         *a.mid = 0;
     }
-    const uint32_t all = cluster_scan<R>(a.count, n, [&](uint32_t c, uint32_t offset, uint32_t) {
+    const uint32_t all = cluster_scan<R>([&](uint32_t c) { return a.count[c]; }, n, [&](uint32_t c, uint32_t offset, uint32_t) {
         a.offsets[c] = offset;
         a.count[c] = 0u;  // ready for the next step's histogram
     });
@@ -966,12 +986,65 @@ __global__ void __launch_bounds__(kCellTileMax) k_rank_cells(StepArgs a)
     }
 }
 
+// A particle's place in its bucket of at most kDenseMin members [st, en), by
+// counting: the members with a smaller input index (stable sorted order), and
+// for a bucket of several alias classes (grouped) also the members of a
+// smaller class and those of its class with a smaller input index (its place
+// in working order), and the bucket's class histogram.
+struct Place {
+    uint32_t rank, work;
+    uint64_t hist;
+};
+template <class LD>
+__device__ __forceinline__ Place bucket_place(LD &&ld, uint32_t st, uint32_t en, uint32_t local, uint32_t my_cls,
+                                              uint32_t imask, bool grouped)
+{
+    Place p;
+    p.rank = 0;
+    p.hist = (uint64_t)(en - st) << (8u * my_cls);  // every member of my class
+    uint32_t diff = 0;
+    for (uint32_t t = st; t < en; t += 8) {  // 8 members requested together
+        uint32_t e[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) e[k] = t + k < en ? ld(t + k) : 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (t + k < en) {
+                p.rank += ((e[k] & imask) < local) ? 1u : 0u;
+                diff |= (e[k] >> kClsShift) ^ my_cls;
+            }
+        }
+    }
+    p.work = p.rank;
+    if (grouped && diff) {
+        uint32_t below = 0, frank = 0;
+        p.hist = 0;
+        for (uint32_t t = st; t < en; ++t) {
+            const uint32_t e = ld(t);
+            const uint32_t mc = e >> kClsShift;
+            below += (mc < my_cls) ? 1u : 0u;
+            frank += (mc == my_cls && (e & imask) < local) ? 1u : 0u;
+            p.hist += 1ull << (8u * mc);
+        }
+        p.work = below + frank;
+    }
+    return p;
+}
+
+// A dense bucket: queued by its first member by atomic slot.
+__device__ __forceinline__ void queue_dense(const StepArgs &a, uint32_t slot, uint32_t gk, uint32_t s)
+{
+    if (slot != 0) return;
+    const uint32_t k = atomicAdd(a.dense, 1u);
+    a.dense[1 + 2 * k] = gk;
+    a.dense[2 + 2 * k] = s;
+}
+
 // The same ranks from the particle side, for small steps (latency bound:
 // the per-cell kernel's b^2 loop in one thread lengthens the critical
 // path): each particle counts the smaller input indices of its bucket.
 // Buckets above kDenseMin members (of any size) are queued for
-// k_dense_sort by their first member (atomic slot 0); nothing is queued for
-// the warp tier.
+// k_dense_sort; nothing is queued for the warp tier.
 __global__ void __launch_bounds__(512) k_rank_reorder(StepArgs a)
 {
     TILE_LOOP_BEGIN
@@ -981,59 +1054,22 @@ __global__ void __launch_bounds__(512) k_rank_reorder(StepArgs a)
     const uint32_t i = d.p_off + local;
     const uint32_t gk = d.c_off + a.key[i];
     const uint32_t st = a.offsets[gk], en = a.offsets[gk + 1];
-    // rank: members with a smaller input index (stable sorted order); for the
-    // walk copy also members of a smaller class, members of the same class
-    // with a smaller input index, and the bucket's class histogram
     const bool packed = d.capacity <= kClsLimit;
-    const uint32_t imask = packed ? kClsLimit - 1u : 0xFFFFFFFFu;
-    const uint32_t my_cls = a.cls[i];
-    uint32_t rank = 0, below = 0, frank = 0;
-    const bool grouped = packed && en - st <= kClassMax && d.gx >= 4 && d.gy >= 4 && d.gz >= 4;
-    uint64_t hist = (uint64_t)(en - st) << (8u * my_cls);  // every member of my class
-    bool mixed = false;
+    const bool grouped = packed && d.gx >= 4 && d.gy >= 4 && d.gz >= 4;
     if (en - st > kDenseMin) {
-        // a dense bucket: one block of k_dense_sort orders it; its first
-        // member by atomic slot queues it
-        if (a.slot[i] == 0) {
-            const uint32_t k = atomicAdd(a.dense, 1u);
-            a.dense[1 + 2 * k] = gk;
-            a.dense[2 + 2 * k] = s;
-        }
+        queue_dense(a, a.slot[i], gk, s);
         continue;
     }
-    uint32_t diff = 0;
-    for (uint32_t t = st; t < en; t += 8) {  // 8 members requested together
-        uint32_t e[8];
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) e[k] = t + k < en ? __ldg(a.tmp + t + k) : 0u;
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-            if (t + k < en) {
-                rank += ((e[k] & imask) < local) ? 1u : 0u;
-                diff |= (e[k] >> kClsShift) ^ my_cls;
-            }
-        }
-    }
-    if (grouped && diff) {  // several classes: the class histogram and my place in the walk copy
-        mixed = true;
-        hist = 0;
-        for (uint32_t t = st; t < en; ++t) {
-            const uint32_t e = __ldg(a.tmp + t);
-            const uint32_t mc = e >> kClsShift;
-            below += (mc < my_cls) ? 1u : 0u;
-            frank += (mc == my_cls && (e & imask) < local) ? 1u : 0u;
-            hist += 1ull << (8u * mc);
-        }
-    }
-    const uint32_t base = a.offsets[d.c_off];
-    const uint32_t g = d.p_off + (st - base) + rank;
+    const Place p = bucket_place([&](uint32_t t) { return __ldg(a.tmp + t); }, st, en, local, a.cls[i],
+                                 packed ? kClsLimit - 1u : 0xFFFFFFFFu, grouped);
+    const uint32_t g0 = d.p_off + (st - a.offsets[d.c_off]);
     // only 4-byte entries are scattered here; k_gather moves the 16-byte
     // particle data in sorted order (coalesced writes, as the reference's
     // reorderDataCUDA gathers).  Buckets holding more than one alias class
-    // also place the particle in the class-grouped walk copy.
-    a.wpos[g] = mixed ? d.p_off + (st - base) + below + frank : g;
-    if (rank == 0) a.chist[gk] = grouped ? class_ends(hist) : kClassWhole;
-    a.perm[g] = local;
+    // also place the particle in working order.
+    a.wpos[g0 + p.rank] = g0 + p.work;
+    if (p.rank == 0) a.chist[gk] = grouped ? class_ends(p.hist) : kClassWhole;
+    a.perm[g0 + p.rank] = local;
     TILE_LOOP_END
 }
 
@@ -1053,12 +1089,12 @@ __device__ __forceinline__ uint32_t dense_key(uint32_t e, uint32_t imask)
     return e == 0xFFFFFFFFu ? 0xFFFFFFFFu : (e & imask);  // padding sorts last
 }
 
-template <bool FULL>
-__device__ void bitonic_sort(uint32_t *v, uint32_t n, uint32_t imask)
+template <bool FULL, class SYNC>
+__device__ void bitonic_sort(uint32_t *v, uint32_t n, uint32_t imask, SYNC &&sync)
 {
     for (uint32_t size = 2; size <= n; size <<= 1) {
         for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t t = threadIdx.x; t < (n >> 1); t += blockDim.x) {
+            for (uint32_t t = threadIdx.x; t < (n >> 1); t += kRadixThreads) {
                 const uint32_t i = 2 * stride * (t / stride) + (t % stride), j = i + stride;
                 const uint32_t vi = v[i], vj = v[j];
                 const uint32_t ki = FULL ? vi : dense_key(vi, imask), kj = FULL ? vj : dense_key(vj, imask);
@@ -1068,8 +1104,88 @@ __device__ void bitonic_sort(uint32_t *v, uint32_t n, uint32_t imask)
                     v[j] = vi;
                 }
             }
-            __syncthreads();
+            sync();
         }
+    }
+}
+
+// Small steps: the header of tile t (SMALL_LOOP_BEGIN), and the scene's live
+// count with its first tile's.
+__device__ __forceinline__ void put_tile_header(const StepArgs &a, uint32_t t, uint32_t tile)
+{
+    uint4 h = make_uint4(0u, 0u, 0u, 0u);
+    if (t < a.ctrl->n_tiles) {
+        const uint32_t s = __ldg(a.tile_scene + t), start = __ldg(a.tile_start + t);
+        const SceneDesc &d = a.scenes[s];
+        const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
+        if (start == 0) a.scene_num[s] = live;  // deleted particles leave the scene
+        const uint32_t n = start < live ? min(tile, live - start) : 0u;
+        h = make_uint4(s << 10 | n, d.p_off + start, d.p_off, d.p_off - a.offsets[d.c_off]);
+    }
+    a.tile_hdr[t] = h;
+}
+
+// The queued dense buckets, a block each (by its first kRadixThreads threads).
+template <class SYNC>
+__device__ __forceinline__ void sort_dense_buckets(const StepArgs &a, uint32_t nd, uint32_t (&S)[kStableLimit],
+                                                   uint32_t (&W)[kStableLimit], SYNC &&sync)
+{
+    __shared__ uint32_t chist_cnt[8], rbase[16], rtot[16];
+    for (uint32_t k = blockIdx.x; k < nd; k += gridDim.x) {
+        const uint32_t gk = a.dense[1 + 2 * k], s = a.dense[2 + 2 * k];
+        const SceneDesc &d = a.scenes[s];
+        const uint32_t st = a.offsets[gk], en = a.offsets[gk + 1], b = en - st;
+        const uint32_t base = a.offsets[d.c_off];
+        const uint32_t g0 = d.p_off + (st - base);
+        const bool packed = d.capacity <= kClsLimit;
+        const uint32_t imask = packed ? kClsLimit - 1u : 0xFFFFFFFFu;
+        if (b > kStableLimit) {  // the bucket's scatter entries are scratch once sorted into perm
+            block_radix_stable(a.tmp + st, a.perm + g0, b, imask, radix_bits(d.capacity),
+                               *reinterpret_cast<RadixSmem *>(S), rbase, rtot, sync);
+            for (uint32_t t = threadIdx.x; t < b; t += kRadixThreads) a.wpos[g0 + t] = g0 + t;
+            if (threadIdx.x == 0) a.chist[gk] = kClassWhole;
+            sync();
+            continue;
+        }
+        const bool grouped = packed && b <= kClassMax && d.gx >= 4 && d.gy >= 4 && d.gz >= 4;
+        uint32_t P = 1;
+        while (P < b) P <<= 1;
+        if (threadIdx.x < 8) chist_cnt[threadIdx.x] = 0;
+        sync();
+        for (uint32_t t = threadIdx.x; t < P; t += kRadixThreads) {
+            const uint32_t e = t < b ? a.tmp[st + t] : 0xFFFFFFFFu;
+            S[t] = e;
+            W[t] = e;
+            if (t < b && grouped) atomicAdd(&chist_cnt[e >> kClsShift], 1u);
+        }
+        sync();
+        bitonic_sort<false>(S, P, imask, sync);
+        uint64_t hist = 0;
+        uint32_t classes = 0;
+        for (uint32_t c = 0; c < 8; ++c) {
+            hist |= (uint64_t)chist_cnt[c] << (8u * c);
+            classes += chist_cnt[c] ? 1u : 0u;
+        }
+        const bool mixed = grouped && classes > 1;
+        if (mixed) bitonic_sort<true>(W, P, imask, sync);  // (class, index) order
+        for (uint32_t t = threadIdx.x; t < b; t += kRadixThreads) {
+            a.perm[g0 + t] = S[t] & imask;
+            if (!mixed) a.wpos[g0 + t] = g0 + t;
+        }
+        if (mixed) {
+            for (uint32_t w = threadIdx.x; w < b; w += kRadixThreads) {
+                const uint32_t key = W[w] & imask;  // its place in S (sorted by index)
+                uint32_t lo = 0, hi = b;
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if ((S[mid] & imask) < key) lo = mid + 1;
+                    else hi = mid;
+                }
+                a.wpos[g0 + lo] = g0 + w;
+            }
+        }
+        if (threadIdx.x == 0) a.chist[gk] = grouped ? class_ends(hist) : kClassWhole;
+        sync();
     }
 }
 
@@ -1077,21 +1193,8 @@ __device__ void bitonic_sort(uint32_t *v, uint32_t n, uint32_t imask)
 // thread a tile, while the queues are read).
 __global__ void __launch_bounds__(kRadixThreads) k_dense_sort(StepArgs a, uint32_t tile, uint32_t small_tiles)
 {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < small_tiles; t += gridDim.x * blockDim.x) {
-        uint4 h = make_uint4(0u, 0u, 0u, 0u);
-        if (t < a.ctrl->n_tiles) {
-            const uint32_t s = __ldg(a.tile_scene + t), start = __ldg(a.tile_start + t);
-            const SceneDesc &d = a.scenes[s];
-            const uint32_t live = a.offsets[d.c_off + d.ncell] - a.offsets[d.c_off];
-            if (start == 0) a.scene_num[s] = live;  // deleted particles leave the scene
-            const uint32_t n = start < live ? min(tile, live - start) : 0u;
-            h = make_uint4(s << 10 | n, d.p_off + start, d.p_off, d.p_off - a.offsets[d.c_off]);
-        }
-        a.tile_hdr[t] = h;
-    }
-    __shared__ __align__(16) uint32_t S[kStableLimit];
-    __shared__ uint32_t W[kStableLimit];
-    __shared__ uint32_t chist_cnt[8], rbase[16], rtot[16];
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < small_tiles; t += gridDim.x * blockDim.x)
+        put_tile_header(a, t, tile);
     {
         const uint32_t nm = *(volatile const uint32_t *)a.mid;
         const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5;
@@ -1134,63 +1237,9 @@ __global__ void __launch_bounds__(kRadixThreads) k_dense_sort(StepArgs a, uint32
             if (lane == 0) a.chist[gk] = grouped ? class_ends(hist) : kClassWhole;
         }
     }
-    const uint32_t nd = *(volatile const uint32_t *)a.dense;
-    for (uint32_t k = blockIdx.x; k < nd; k += gridDim.x) {
-        const uint32_t gk = a.dense[1 + 2 * k], s = a.dense[2 + 2 * k];
-        const SceneDesc &d = a.scenes[s];
-        const uint32_t st = a.offsets[gk], en = a.offsets[gk + 1], b = en - st;
-        const uint32_t base = a.offsets[d.c_off];
-        const uint32_t g0 = d.p_off + (st - base);
-        const bool packed = d.capacity <= kClsLimit;
-        const uint32_t imask = packed ? kClsLimit - 1u : 0xFFFFFFFFu;
-        if (b > kStableLimit) {  // the bucket's scatter entries are scratch once sorted into perm
-            block_radix_stable(a.tmp + st, a.perm + g0, b, imask, radix_bits(d.capacity),
-                               *reinterpret_cast<RadixSmem *>(S), rbase, rtot);
-            for (uint32_t t = threadIdx.x; t < b; t += blockDim.x) a.wpos[g0 + t] = g0 + t;
-            if (threadIdx.x == 0) a.chist[gk] = kClassWhole;
-            __syncthreads();
-            continue;
-        }
-        const bool grouped = packed && b <= kClassMax && d.gx >= 4 && d.gy >= 4 && d.gz >= 4;
-        uint32_t P = 1;
-        while (P < b) P <<= 1;
-        if (threadIdx.x < 8) chist_cnt[threadIdx.x] = 0;
-        __syncthreads();
-        for (uint32_t t = threadIdx.x; t < P; t += blockDim.x) {
-            const uint32_t e = t < b ? a.tmp[st + t] : 0xFFFFFFFFu;
-            S[t] = e;
-            W[t] = e;
-            if (t < b && grouped) atomicAdd(&chist_cnt[e >> kClsShift], 1u);
-        }
-        __syncthreads();
-        bitonic_sort<false>(S, P, imask);
-        uint64_t hist = 0;
-        uint32_t classes = 0;
-        for (uint32_t c = 0; c < 8; ++c) {
-            hist |= (uint64_t)chist_cnt[c] << (8u * c);
-            classes += chist_cnt[c] ? 1u : 0u;
-        }
-        const bool mixed = grouped && classes > 1;
-        if (mixed) bitonic_sort<true>(W, P, imask);  // (class, index) order
-        for (uint32_t t = threadIdx.x; t < b; t += blockDim.x) {
-            a.perm[g0 + t] = S[t] & imask;
-            if (!mixed) a.wpos[g0 + t] = g0 + t;
-        }
-        if (mixed) {
-            for (uint32_t w = threadIdx.x; w < b; w += blockDim.x) {
-                const uint32_t key = W[w] & imask;  // its place in S (sorted by index)
-                uint32_t lo = 0, hi = b;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if ((S[mid] & imask) < key) lo = mid + 1;
-                    else hi = mid;
-                }
-                a.wpos[g0 + lo] = g0 + w;
-            }
-        }
-        if (threadIdx.x == 0) a.chist[gk] = grouped ? class_ends(hist) : kClassWhole;
-        __syncthreads();
-    }
+    __shared__ __align__(16) uint32_t S[kStableLimit];
+    __shared__ uint32_t W[kStableLimit];
+    sort_dense_buckets(a, *(volatile const uint32_t *)a.dense, S, W, BlockSync());
 }
 
 // Reorder (reorderDataCUDA x2, pbf_neighbor_search_util.cu:143-154): predicted
@@ -1242,6 +1291,107 @@ __global__ void __launch_bounds__(kSmallBlock) k_gather_small(StepArgs a, uint32
     SMALL_LOOP_BEGIN
     gather_slot<PACKED>(a, s, p_off, i);
     SMALL_LOOP_END
+}
+
+// The smallest steps: everything before the neighbour walk (prediction, cell
+// hash and counts; scan; scatter; ranks and tile headers; reorder) in one
+// cluster of 1024-thread blocks, a particle a thread, R rounds of 1024 cells a
+// block.  Sorted and working orders are the separate kernels'.
+//
+// Bound by latency: four cluster barriers (850 cycles each with nothing to
+// drain, 1,500 with stores) and the loads between them, 12,000 cycles in all,
+// against six launches and the reload in each of what the phase before knew:
+// set, step and get of 4,096 particles 87 -> 82 us, of 10,648 at h = 1.4
+// spacings 67 -> 62.  A particle keeps its prediction, bucket and slot in
+// registers through the phases and writes its records into its working slot
+// itself; counts and offsets are the blocks' shared memory.  Two particles a
+// thread took 32,768 particles' step from 88.2 to 90.1 us, so such steps keep
+// a kernel per phase.
+template <uint32_t R, bool PACKED>
+__global__ void __launch_bounds__(1024) k_front(StepArgs a, uint32_t tile_shift, uint32_t small_tiles)
+{
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), blocks = cluster.num_blocks(), threads = blocks * 1024u;
+    // a cluster's warps take the particles in turn, block after block, so few
+    // particles spread over all its SMs
+    const uint32_t gid = ((threadIdx.x >> 5) * blocks + rank) * 32u + (threadIdx.x & 31u);
+    const uint32_t t = gid >> tile_shift;
+    // the tile is requested beside the count of tiles (the lists have room)
+    const uint32_t n_tiles = a.ctrl->n_tiles, n_cells = a.ctrl->n_cells;
+    const uint32_t s = t < small_tiles ? __ldg(a.tile_scene + t) : 0u;
+    const uint32_t local = (t < small_tiles ? __ldg(a.tile_start + t) : 0u) + (gid & ((1u << tile_shift) - 1u));
+    // the cells' counts, then offsets, block after block in shared memory
+    static_assert(kFrontRounds * 1024u <= kStableLimit, "the dense buckets' sort reuses them");
+    __shared__ __align__(16) uint32_t cells[kStableLimit], counts[kStableLimit];
+    constexpr uint32_t kShift = R == 1 ? 10 : (R == 2 ? 11 : 12), kMask = (1u << kShift) - 1u;
+    static_assert(R * 1024u == 1u << kShift, "a power of two of cells a block");
+    for (uint32_t k = 0; k < R; ++k) counts[k * 1024u + threadIdx.x] = 0u;
+    auto zeroed = cluster.barrier_arrive();
+    if (gid == 0) *a.dense = 0;
+    const SceneDesc *sd = a.scenes + s;
+    bool live = false;  // (with a particle)
+    uint32_t gk = 0, slot = 0, cls = 0;
+    PhaseIn in;
+    float4 ps;
+    if (t < n_tiles) {
+        const uint32_t n = a.scene_num[s];
+        // (its particle is requested beside the scene's count: slots up to the capacity exist)
+        if (!PACKED) in = load_phase<PACKED>(a, *sd, s, min(local, sd->capacity - 1u));
+        live = local < n;
+        if (live) {
+            if (PACKED) in = load_phase<PACKED>(a, *sd, s, local);
+            const Predicted p = predict_particle<PACKED>(a, *sd, s, local, n, in);
+            ps = p.ps;
+            gk = sd->c_off + p.key;
+            cls = p.cls;
+        }
+    }
+    cluster.barrier_wait(std::move(zeroed));
+    if (live) slot = atomicAdd(cluster.map_shared_rank(counts + (gk & kMask), gk >> kShift), 1u);
+    cluster.sync();
+    const uint32_t all = cluster_scan<R>([&](uint32_t c) { return counts[c & kMask]; }, n_cells,
+                                         [&](uint32_t c, uint32_t offset, uint32_t) {
+                                             cells[c & kMask] = offset;
+                                             a.offsets[c] = offset;
+                                         });
+    if (gid == 0) a.offsets[n_cells] = all;
+    cluster.sync();
+    uint32_t st = 0, en = 0, base = 0;
+    if (live) {
+        st = *cluster.map_shared_rank(cells + (gk & kMask), gk >> kShift);
+        en = st + *cluster.map_shared_rank(counts + (gk & kMask), gk >> kShift);
+        base = *cluster.map_shared_rank(cells + (sd->c_off & kMask), sd->c_off >> kShift);
+        a.tmp[st + slot] = local | cls << kClsShift;
+        if (en - st > kDenseMin) queue_dense(a, slot, gk, s);
+    }
+    cluster.sync();
+    if (live) {
+        a.xs[sd->p_off + local] = ps;
+        a.key[sd->p_off + local] = gk - sd->c_off;
+    }
+    if (live && en - st <= kDenseMin) {
+        const bool grouped = sd->gx >= 4 && sd->gy >= 4 && sd->gz >= 4;
+        const Place p = bucket_place([&](uint32_t u) { return a.tmp[u]; }, st, en, local, cls, kClsLimit - 1u, grouped);
+        const uint32_t g0 = sd->p_off + (st - base), g = g0 + p.rank, w = g0 + p.work;
+        a.wpos[g] = w;
+        a.perm[g] = local;
+        if (p.rank == 0) a.chist[gk] = grouped ? class_ends(p.hist) : kClassWhole;
+        if (gk != sd->c_off + sd->ncell) {  // not deleted
+            a.xa[w] = make_float4(ps.x, ps.y, ps.z, 0.f);
+            a.xold[w] = make_float4(in.x.x, in.x.y, in.x.z, __uint_as_float(g));
+            a.id_tmp[w] = __float_as_uint(ps.w);
+        }
+    }
+    // (from the last thread down: the first ones hold the particles of a step with few)
+    for (uint32_t h = threads - 1u - gid; h < small_tiles; h += threads) put_tile_header(a, h, 1u << tile_shift);
+    const uint32_t nd = *(volatile const uint32_t *)a.dense;  // (complete since the last barrier)
+    if (nd == 0) return;
+    if (threadIdx.x < kRadixThreads) sort_dense_buckets(a, nd, cells, counts, RadixSync());
+    cluster.sync();
+    // the dense buckets' particles, through the permutation
+    if (t < n_tiles && local < a.offsets[sd->c_off + sd->ncell] - a.offsets[sd->c_off])
+        gather_slot<PACKED>(a, s, sd->p_off, sd->p_off + local);
 }
 
 // Neighbour list (detectNeighborsCUDA<uint32_t>, pbf_neighbor_search_util.cu:454-482,
@@ -2524,6 +2674,16 @@ static ScanFn scan_cluster_fn(uint32_t rounds)
     }
 }
 
+using FrontFn = void (*)(StepArgs, uint32_t, uint32_t);
+static FrontFn front_fn(uint32_t rounds, bool packed)
+{
+    switch (rounds) {
+    case 1: return packed ? k_front<1, true> : k_front<1, false>;
+    case 2: return packed ? k_front<2, true> : k_front<2, false>;
+    default: return packed ? k_front<4, true> : k_front<4, false>;
+    }
+}
+
 // The largest cluster the scan may use on the current device (16 blocks of
 // 1024 threads are beyond the portable size; a device without room for one
 // such cluster takes 8), asked once per device.
@@ -2538,6 +2698,8 @@ uint32_t scan_cluster_limit()
     if (it != cache.end()) return it->second;
     bool ok = true;
     for (uint32_t r : {1u, 2u, 4u, 8u, 16u, kScanRoundsMax}) ok = allows_cluster(scan_cluster_fn(r)) && ok;
+    for (uint32_t r = 1; r <= kFrontRounds; r *= 2)
+        ok = allows_cluster(front_fn(r, false)) && allows_cluster(front_fn(r, true)) && ok;
     cache[dev] = ok ? kScanClusterMax : 8u;
     return cache[dev];
 }
@@ -2552,53 +2714,59 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
         ++nl;                             \
         if (hook) hook->launched(name);   \
     } while (0)
-    if (packed)
-        k_predict_hash<true><<<g, b, 0, st>>>(a);
-    else
-        k_predict_hash<false><<<g, b, 0, st>>>(a);
-    PBF_LAUNCHED("k_predict_hash");
-    if (sh.scan_grid == 0 && sh.scan_cluster) {
-        launch_cluster(scan_cluster_fn(sh.scan_rounds), sh.scan_cluster, st, a);
-        PBF_LAUNCHED("k_scan_single");  // the profile's name for the scan in one launch
-    } else if (sh.scan_grid == 0) {  // small table: one block
-        switch (sh.scan_rounds) {  // rounds of 1024 cells held in registers
-#define PBF_SCAN_ROUNDS(r) \
-    case r: k_scan_single_reg<r><<<1, 1024, 0, st>>>(a); break;
-        PBF_SCAN_ROUNDS(1) PBF_SCAN_ROUNDS(2) PBF_SCAN_ROUNDS(3) PBF_SCAN_ROUNDS(4)
-        PBF_SCAN_ROUNDS(5) PBF_SCAN_ROUNDS(6) PBF_SCAN_ROUNDS(7)
-#undef PBF_SCAN_ROUNDS
-        default: k_scan_single_reg<8><<<1, 1024, 0, st>>>(a); break;
-        }
-        PBF_LAUNCHED("k_scan_single");
-    } else {
-        k_scan_reduce<<<sh.scan_grid, 256, 0, st>>>(a);
-        PBF_LAUNCHED("k_scan_reduce");
-        k_scan_spine<<<1, 1024, 0, st>>>(a);
-        PBF_LAUNCHED("k_scan_spine");
-        k_scan_down<<<sh.scan_grid, 256, 0, st>>>(a);
-        PBF_LAUNCHED("k_scan_down");
-    }
-    k_scatter<<<g, b, 0, st>>>(a);
-    PBF_LAUNCHED("k_scatter");
-    if (sh.small) {
-        k_rank_reorder<<<g, b, 0, st>>>(a);
-        PBF_LAUNCHED("k_rank_reorder");
-    } else {
-        k_rank_cells<<<sh.grid_cells, sh.cell_tile, 0, st>>>(a);
-        PBF_LAUNCHED("k_rank_cells");
-    }
-    k_dense_sort<<<sh.grid, kRadixThreads, 0, st>>>(a, sh.tile, sh.small ? sh.small_tiles : 0u);
-    PBF_LAUNCHED("k_dense_sort");
     const uint32_t gs = sh.small_tiles * (sh.tile / kSmallBlock);  // small steps: a block per part of a tile
-    if (sh.small && packed)
-        k_gather_small<true><<<gs, kSmallBlock, 0, st>>>(a, sh.tile);
-    else if (sh.small)
-        k_gather_small<false><<<gs, kSmallBlock, 0, st>>>(a, sh.tile);
-    else if (packed)
-        k_gather<true><<<g, b, 0, st>>>(a);
-    else
-        k_gather<false><<<g, b, 0, st>>>(a);
-    PBF_LAUNCHED("k_gather");
+    const bool front = sh.front && !hook;  // (a profile gets the phases one by one)
+    if (front) {
+        launch_cluster(front_fn(sh.front, packed), sh.front_cluster, st, a, sh.tile_shift, sh.small_tiles);
+        PBF_LAUNCHED("k_front");
+    } else {
+        if (packed)
+            k_predict_hash<true><<<g, b, 0, st>>>(a);
+        else
+            k_predict_hash<false><<<g, b, 0, st>>>(a);
+        PBF_LAUNCHED("k_predict_hash");
+        if (sh.scan_grid == 0 && sh.scan_cluster) {
+            launch_cluster(scan_cluster_fn(sh.scan_rounds), sh.scan_cluster, st, a);
+            PBF_LAUNCHED("k_scan_single");  // the profile's name for the scan in one launch
+        } else if (sh.scan_grid == 0) {  // small table: one block
+            switch (sh.scan_rounds) {  // rounds of 1024 cells held in registers
+#define PBF_SCAN_ROUNDS(r) \
+        case r: k_scan_single_reg<r><<<1, 1024, 0, st>>>(a); break;
+            PBF_SCAN_ROUNDS(1) PBF_SCAN_ROUNDS(2) PBF_SCAN_ROUNDS(3) PBF_SCAN_ROUNDS(4)
+            PBF_SCAN_ROUNDS(5) PBF_SCAN_ROUNDS(6) PBF_SCAN_ROUNDS(7)
+#undef PBF_SCAN_ROUNDS
+            default: k_scan_single_reg<8><<<1, 1024, 0, st>>>(a); break;
+            }
+            PBF_LAUNCHED("k_scan_single");
+        } else {
+            k_scan_reduce<<<sh.scan_grid, 256, 0, st>>>(a);
+            PBF_LAUNCHED("k_scan_reduce");
+            k_scan_spine<<<1, 1024, 0, st>>>(a);
+            PBF_LAUNCHED("k_scan_spine");
+            k_scan_down<<<sh.scan_grid, 256, 0, st>>>(a);
+            PBF_LAUNCHED("k_scan_down");
+        }
+        k_scatter<<<g, b, 0, st>>>(a);
+        PBF_LAUNCHED("k_scatter");
+        if (sh.small) {
+            k_rank_reorder<<<g, b, 0, st>>>(a);
+            PBF_LAUNCHED("k_rank_reorder");
+        } else {
+            k_rank_cells<<<sh.grid_cells, sh.cell_tile, 0, st>>>(a);
+            PBF_LAUNCHED("k_rank_cells");
+        }
+        k_dense_sort<<<sh.grid, kRadixThreads, 0, st>>>(a, sh.tile, sh.small ? sh.small_tiles : 0u);
+        PBF_LAUNCHED("k_dense_sort");
+        if (sh.small && packed)
+            k_gather_small<true><<<gs, kSmallBlock, 0, st>>>(a, sh.tile);
+        else if (sh.small)
+            k_gather_small<false><<<gs, kSmallBlock, 0, st>>>(a, sh.tile);
+        else if (packed)
+            k_gather<true><<<g, b, 0, st>>>(a);
+        else
+            k_gather<false><<<g, b, 0, st>>>(a);
+        PBF_LAUNCHED("k_gather");
+    }
     if (sh.small) {
         if (sh.small_split)
             k_neighbors_split<<<gs, kSplitBlock, sh.nb_smem, st>>>(a, sh.tile);

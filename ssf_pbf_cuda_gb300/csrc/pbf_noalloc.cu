@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(1024) na_scan_cluster(uint32_t C, Scratch s, u
                                                         uint32_t *__restrict__ ce)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) s.big[0] = 0;
-    const uint32_t all = pbf103::cluster_scan<R>(s.counts, C, [&](uint32_t c, uint32_t offset, uint32_t count) {
+    const uint32_t all = pbf103::cluster_scan<R>([&](uint32_t c) { return s.counts[c]; }, C, [&](uint32_t c, uint32_t offset, uint32_t count) {
         s.offsets[c] = offset;
         put_range(c, offset, count, cs, ce);
     });
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(pbf103::kRadixThreads) na_big(uint32_t n, Scra
         const uint32_t k = s.big[1 + q];
         const uint32_t st = s.offsets[k], en = s.offsets[k + 1];
         pbf103::block_radix_stable(s.tmp + st, perm + st, en - st, 0xFFFFFFFFu, pbf103::radix_bits(n), sm, base,
-                                   tot);
+                                   tot, pbf103::BlockSync());
     }
 }
 

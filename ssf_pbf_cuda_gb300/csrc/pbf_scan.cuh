@@ -22,21 +22,22 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
 // Each block (1024 threads) of the cluster holds a run of 1024 * R counts in
 // registers, its total goes into every other block's shared memory, and after
 // the cluster's barrier each block adds the totals before it.
-// out(index, offset, count) is called for every index below n; returns the
-// sum of all counts.
-template <uint32_t R, class OUT>
-__device__ __forceinline__ uint32_t cluster_scan(const uint32_t *count, uint32_t n, OUT &&out)
+// count(index) gives a count, out(index, offset, count) is called for every
+// index below n, both by the thread of the block that holds the index; returns
+// the sum of all counts.
+template <uint32_t R, class COUNT, class OUT>
+__device__ __forceinline__ uint32_t cluster_scan(COUNT &&count, uint32_t n, OUT &&out)
 {
     namespace cg = cooperative_groups;
     const cg::cluster_group cluster = cg::this_cluster();
-    __shared__ uint32_t ws[R][32], tot[kScanClusterMax];
+    __shared__ uint32_t ws[R][32], tot[32];
     const uint32_t rank = cluster.block_rank(), blocks = cluster.num_blocks();
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, base = rank * (1024u * R);
     uint32_t v[R], inc[R];
 #pragma unroll
     for (uint32_t k = 0; k < R; ++k) {
         const uint32_t idx = base + k * 1024u + t;
-        v[k] = idx < n ? count[idx] : 0u;
+        v[k] = idx < n ? count(idx) : 0u;
     }
 #pragma unroll
     for (uint32_t k = 0; k < R; ++k) {
@@ -56,12 +57,12 @@ __device__ __forceinline__ uint32_t cluster_scan(const uint32_t *count, uint32_t
         if (lane < blocks) *cluster.map_shared_rank(&tot[rank], lane) = carry;
     }
     cluster.sync();  // every block's totals are in; no block writes another's memory after it
-    uint32_t before = 0, all = 0;
-    for (uint32_t k = 0; k < blocks; ++k) {
-        const uint32_t x = tot[k];
-        before += k < rank ? x : 0u;
-        all += x;
-    }
+    // every warp adds for itself, a block's total a lane: a block has 32 warps,
+    // so each instruction here costs 8 cycles (a loop over the totals 1,300)
+    static_assert(kScanClusterMax <= 32, "a total a lane");
+    const uint32_t x = lane < blocks ? tot[lane] : 0u;
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < rank ? x : 0u);
+    const uint32_t all = __reduce_add_sync(0xffffffffu, x);
 #pragma unroll
     for (uint32_t k = 0; k < R; ++k) {
         const uint32_t idx = base + k * 1024u + t;

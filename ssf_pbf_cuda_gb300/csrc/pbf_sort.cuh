@@ -38,11 +38,12 @@ __host__ __device__ __forceinline__ uint32_t radix_bits(uint32_t bound)
 }
 
 // Sorts the b entries of `a` by (entry & imask) into `out` (masked values).
-// `a` is overwritten.  Every thread of the block must call it with the same
-// arguments; blockDim.x == kRadixThreads.
+// `a` is overwritten.  The block's first kRadixThreads threads call it, all
+// with the same arguments; sync() is a barrier among them.
+template <class SYNC>
 __device__ inline void block_radix_stable(uint32_t *a, uint32_t *out, uint32_t b, uint32_t imask, uint32_t nbits,
                                    RadixSmem &sm, uint32_t *base /* __shared__ [16] */,
-                                   uint32_t *tot /* __shared__ [16] */)
+                                   uint32_t *tot /* __shared__ [16] */, SYNC &&sync)
 {
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
     const uint32_t passes = (nbits + 3u) / 4u;
@@ -52,7 +53,7 @@ __device__ inline void block_radix_stable(uint32_t *a, uint32_t *out, uint32_t b
     uint32_t *src = a, *dst = out;
     if ((passes & 1u) == 0u) {
         for (uint32_t i = t; i < b; i += kRadixThreads) out[i] = a[i] & imask;
-        __syncthreads();
+        sync();
         src = out;
         dst = a;
     }
@@ -60,9 +61,9 @@ __device__ inline void block_radix_stable(uint32_t *a, uint32_t *out, uint32_t b
         const uint32_t shift = 4u * p;
         const uint32_t m = (p == 0 && src == a) ? imask : 0xFFFFFFFFu;
         if (t < 16) base[t] = 0;
-        __syncthreads();
+        sync();
         for (uint32_t i = t; i < b; i += kRadixThreads) atomicAdd(&base[((src[i] & m) >> shift) & 15u], 1u);
-        __syncthreads();
+        sync();
         if (t == 0) {
             uint32_t run = 0;
             for (uint32_t d = 0; d < 16; ++d) {
@@ -71,7 +72,7 @@ __device__ inline void block_radix_stable(uint32_t *a, uint32_t *out, uint32_t b
                 run += c;
             }
         }
-        __syncthreads();
+        sync();
         for (uint32_t c0 = 0; c0 < b; c0 += kRadixChunk) {
             uint32_t v[kRadixItems];
             uint64_t packed = 0;  // 16 digits x 4-bit counts of this thread's items (at most 8 each)
@@ -83,7 +84,7 @@ __device__ inline void block_radix_stable(uint32_t *a, uint32_t *out, uint32_t b
             }
 #pragma unroll
             for (uint32_t d = 0; d < 16; ++d) sm.cnt[d][t] = (uint32_t)(packed >> (4u * d)) & 15u;
-            __syncthreads();
+            sync();
             // exclusive prefix over the chunk's threads, two digits per warp:
             // lane L takes threads 8L .. 8L+7
 #pragma unroll
@@ -106,7 +107,7 @@ __device__ inline void block_radix_stable(uint32_t *a, uint32_t *out, uint32_t b
                 for (uint32_t j = 0; j < 8; ++j) sm.cnt[d][8u * lane + j] = pre + loc[j];
                 if (lane == 31) tot[d] = inc;
             }
-            __syncthreads();
+            sync();
             uint64_t seen = 0;
 #pragma unroll
             for (uint32_t k = 0; k < kRadixItems; ++k) {
@@ -118,15 +119,24 @@ __device__ inline void block_radix_stable(uint32_t *a, uint32_t *out, uint32_t b
                     dst[base[d] + sm.cnt[d][t] + off] = v[k];
                 }
             }
-            __syncthreads();
+            sync();
             if (t < 16) base[t] += tot[t];
-            __syncthreads();
+            sync();
         }
         uint32_t *tmp = src;
         src = dst;
         dst = tmp;
-        __syncthreads();
+        sync();
     }
 }
+
+// The barrier of a block of kRadixThreads threads, and of the first
+// kRadixThreads threads of a larger one.
+struct BlockSync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+struct RadixSync {
+    __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 1, %0;" ::"n"(kRadixThreads) : "memory"); }
+};
 
 }  // namespace pbf103
