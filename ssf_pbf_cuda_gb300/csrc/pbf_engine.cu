@@ -713,7 +713,13 @@ pbf_status Batch::upload(cudaStream_t st)
     CK(cudaSetDevice(device_));
     if (dirty_desc_) {
         std::vector<SceneDesc> h(scenes_.size());
-        for (size_t k = 0; k < scenes_.size(); ++k) h[k] = scenes_[k].desc;
+        long_lists_ = false;
+        for (size_t k = 0; k < scenes_.size(); ++k) {
+            const SceneDesc &d = h[k] = scenes_[k].desc;
+            // neighbours within h at rest density
+            const double ball = 4.18879 * std::pow((double)d.h2, 1.5) / ((double)d.m * d.inv_rho0);
+            long_lists_ = long_lists_ || (scenes_[k].active && ball > 16.0);
+        }
         if (!h.empty())
             CK(cudaMemcpyAsync(d_scenes_, h.data(), sizeof(SceneDesc) * h.size(), cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));
@@ -786,6 +792,9 @@ LaunchShape Batch::shape_for(uint32_t tile) const
         // small steps: the lists and the cells' ranges (27 per particle at
         // most, kSplit lanes a particle or one: the same per block)
         sh.small_split = 0;
+        const uint64_t slots = (uint64_t)nt * tile;
+        const bool lanes = long_lists_ ? slots <= kLanesLong : slots > (uint64_t)sms_ * kSmallBlock && slots <= kLanesStep;
+        sh.small_lanes = sh.small && lanes ? 1u : 0u;
         if (sh.small) {
             sh.nb_smem = kSmallBlock * (max_pair_ - 1u) * 4u + kSmallWalkSmem;
             const uint32_t split = sh.nb_smem + kSplitBlock * (max_pair_ - 1u) * 4u;

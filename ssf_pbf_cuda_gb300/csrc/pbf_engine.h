@@ -163,6 +163,7 @@ private:
     uint32_t *d_wpos_ = nullptr;                      // sorted slot -> working slot
     uint32_t *d_dense_ = nullptr;                     // dense-bucket queue
     uint32_t *d_mid_ = nullptr;                       // medium-bucket queue
+    bool long_lists_ = false;         // some active scene expects more than 16 neighbours a particle
     uint32_t *h_small_ = nullptr;     // pinned host scratch: pack offsets + counts + counts stored by the device
     cudaEvent_t small_done_ = nullptr;
     uint64_t bnd_capacity_ = 0;

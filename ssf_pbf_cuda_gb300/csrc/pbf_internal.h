@@ -147,13 +147,14 @@ struct LaunchShape {
     uint32_t front_cluster; // blocks of its cluster
     uint32_t tile_shift;  // log2 of tile
     uint32_t small_split; // small steps: their walk takes kSplit lanes a particle
+    uint32_t small_lanes; // small steps: their list passes take kLanes lanes a particle
     uint32_t small_tiles; // small steps: tiles rounded up to a power of two, for which headers are written
     uint32_t nb_smem;     // k_neighbors_lambda: bytes of shared memory for the block's lists (0 = stored directly)
     bool operator==(const LaunchShape &o) const
     {
         return tile == o.tile && grid == o.grid && scan_grid == o.scan_grid && scan_rounds == o.scan_rounds && scan_cluster == o.scan_cluster &&
                chunk == o.chunk &&
-               grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && small_tiles == o.small_tiles && small_split == o.small_split && nb_smem == o.nb_smem &&
+               grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && small_tiles == o.small_tiles && small_split == o.small_split && small_lanes == o.small_lanes && nb_smem == o.nb_smem &&
                front == o.front && front_cluster == o.front_cluster &&
                grid_nb == o.grid_nb && grid_lambda == o.grid_lambda && grid_dp == o.grid_dp &&
                grid_omega[0] == o.grid_omega[0] && grid_omega[1] == o.grid_omega[1] && grid_apply[0] == o.grid_apply[0] &&
@@ -247,6 +248,16 @@ constexpr uint32_t kSplitBlock = kSplit * kSmallBlock;
 // against 78 with one lane a particle, 20,000 84 against 80 (10,648 at h = 1.4
 // spacings 47 against 51).
 constexpr uint32_t kSplitStep = 16384;
+// Lanes a particle in the smallest steps' list passes: up to kLanesLong slots
+// where lists are long (more than the 16 slots a lane takes at once, by the
+// neighbours expected within h at rest density), and with short ones between
+// more blocks of kSmallBlock particles than SMs and kLanesStep slots.  A step
+// in us, two lanes against one:
+//   h = 2 spacings    500: 52, 57  4,096: 58, 62  8,192: 60, 66  16,384: 70, 76  24,000: 80, 82  32,768: 105, 87
+//   h = 1.4 spacings  500: 41, 40  4,096: 45, 45  8,192: 46, 45  10,648: 49.5, 51.5  16,384: 54, 56  20,000: 62, 60
+// (four lanes: 55 at 4,096 and 70 at 12,000 against 66).
+constexpr uint32_t kLanes = 2;
+constexpr uint32_t kLanesStep = 16384, kLanesLong = 24576;
 constexpr uint32_t kCellTile = 256;         // default cells per cell tile = threads per k_rank_cells block
 constexpr uint32_t kCellTileMin = 64, kCellTileMax = 512;  // the autotuner's range
 constexpr uint32_t kMidMin = 16;            // buckets with more members are queued (warp or block per bucket)

@@ -630,6 +630,66 @@ __device__ __forceinline__ void list_walk_wide(bool l16, const uint32_t *__restr
     } while (k0 < nn);
 }
 
+// The smallest steps: a particle's list over LANES lanes, 32 / LANES slots of
+// every 32 a lane (whole rows).  Every lane loads its records and makes their
+// terms; the sums then go from lane to lane, each adding its own terms to what
+// the lane before it had, so the additions are the one-lane walk's, in its
+// order.  All the lanes end with the whole sums.  Few particles leave a
+// scheduler with one warp or none, and a pass's time is that warp's: 32 slots
+// in two groups of 16 took 3,700 to 6,200 cycles of its 5,000 to 7,200.
+template <uint32_t LANES, class SUM, class IDX, class LD>
+__device__ __forceinline__ void lanes_sum(uint32_t k0, uint32_t nn, uint32_t self, SUM &sum, IDX &&idx, LD &&ld)
+{
+    constexpr uint32_t N = 32 / LANES;  // slots a lane
+    const uint32_t sub = threadIdx.x % LANES, gmask = ((1u << LANES) - 1u) << (threadIdx.x & (32u - LANES));
+    const uint32_t m = k0 + N * sub;
+    decltype(ld(0u)) rec[N];
+#pragma unroll
+    for (uint32_t c = 0; c < N; ++c) rec[c] = ld(m + c < nn ? idx(c) : self);
+    typename SUM::Term t[N];
+#pragma unroll
+    for (uint32_t c = 0; c < N; ++c) t[c] = sum.term(rec[c], m + c < nn);
+#pragma unroll
+    for (uint32_t l = 0; l < LANES; ++l) {
+        if (k0 + N * l < nn) {
+#pragma unroll
+            for (uint32_t c = 0; c < N; ++c) sum.add(t[c]);
+        }
+        sum.template pass<LANES>(gmask, l);
+    }
+}
+
+template <uint32_t LANES, class SUM, class LD>
+__device__ __forceinline__ void list_walk_lanes(bool l16, const uint32_t *__restrict__ nl, uint64_t stride,
+                                                uint32_t rows, uint32_t nn, uint32_t base, uint32_t self, SUM &sum,
+                                                LD &&ld)
+{
+    const uint4 *p = reinterpret_cast<const uint4 *>(nl);
+    constexpr uint32_t N = 32 / LANES;  // slots a lane
+    const uint32_t sub = threadIdx.x % LANES;
+    uint32_t k0 = 0;
+    do {
+        const uint32_t m = k0 + N * sub;
+        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+        uint32_t q[N];
+        if (l16) {
+            uint4 r[N / 8];
+#pragma unroll
+            for (uint32_t j = 0; j < N / 8; ++j) r[j] = m / 8 + j < rows ? list_ld(p + (uint64_t)(m / 8 + j) * stride) : z;
+#pragma unroll
+            for (uint32_t c = 0; c < N; ++c) q[c] = base + oct_at(r[c / 8], c % 8);
+        } else {
+            uint4 r[N / 4];
+#pragma unroll
+            for (uint32_t j = 0; j < N / 4; ++j) r[j] = m / 4 + j < rows ? list_ld(p + (uint64_t)(m / 4 + j) * stride) : z;
+#pragma unroll
+            for (uint32_t c = 0; c < N; ++c) q[c] = quad_at(r[c / 4], c % 4);
+        }
+        lanes_sum<LANES>(k0, nn, self, sum, [&](uint32_t c) { return q[c]; }, ld);
+        k0 += 32;
+    } while (k0 < nn);
+}
+
 // Small steps' blocks: kSmallBlock threads, tile / kSmallBlock of them a tile,
 // so that few particles spread over many SMs, one block for every part of
 // every tile the launch shape allows for.  A tile's header (scene << 10 |
@@ -642,10 +702,24 @@ __device__ __forceinline__ void list_walk_wide(bool l16, const uint32_t *__restr
     {                                                                         \
         const uint32_t parts_ = tile / kSmallBlock;                           \
         const uint4 hd_ = __ldg(a.tile_hdr + blockIdx.x / parts_);            \
-        const uint32_t k_ = (blockIdx.x % parts_) * kSmallBlock + threadIdx.x; \
+        const uint32_t k_ = (blockIdx.x % parts_) * kSmallBlock + threadIdx.x / LANES; \
         if (k_ >= (hd_.x & 1023u)) return;                                    \
         const uint32_t s = hd_.x >> 10, i = hd_.y + k_, p_off = hd_.z;
 #define SMALL_LOOP_END }
+
+// The list passes of small steps: LANES = 1, or kLanes lanes a particle (and
+// kLanes times the threads a block), of which the first finishes.
+template <uint32_t LANES, class SUM, class LD>
+__device__ __forceinline__ bool small_sum(const StepArgs &a, bool l16, uint32_t i, uint32_t p_off, SUM &sum, LD &&ld)
+{
+    if (LANES == 1) {
+        list_walk_wide(l16, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i, ld,
+                       [&](const decltype(ld(0u)) &r, bool on) { sum.add(sum.term(r, on)); });
+        return true;
+    }
+    list_walk_lanes<LANES>(l16, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i, sum, ld);
+    return threadIdx.x % LANES == 0;
+}
 
 // Per-tile prologue shared by the particle kernels.
 #define TILE_LOOP_BEGIN                                                   \
@@ -1288,6 +1362,7 @@ __global__ void __launch_bounds__(512) k_gather(StepArgs a)
 template <bool PACKED>
 __global__ void __launch_bounds__(kSmallBlock) k_gather_small(StepArgs a, uint32_t tile)
 {
+    constexpr uint32_t LANES = 1;
     SMALL_LOOP_BEGIN
     gather_slot<PACKED>(a, s, p_off, i);
     SMALL_LOOP_END
@@ -1524,6 +1599,28 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
     a.xb[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));  // the first delta-p pass gathers both
     TILE_LOOP_END
 }
+
+// The lambda sums of a particle over records of positions.
+struct LamWalk {
+    float4 xp;
+    PairConst pc;
+    LamSum ls;
+    struct Term {
+        PairGeo g;
+        PairWS k;
+    };
+    __device__ __forceinline__ Term term(const float4 &xj, bool on) const
+    {
+        const PairGeo g = pair_geo(xp, xj);
+        return Term{g, masked(pair_ws(g.r2, pc), on)};
+    }
+    __device__ __forceinline__ void add(const Term &t) { ls.add(t.g, t.k); }
+    template <uint32_t LANES>
+    __device__ __forceinline__ void pass(uint32_t gmask, uint32_t lane)
+    {
+        for (float *f : {&ls.ks, &ls.g0, &ls.g1, &ls.g2, &ls.kg2}) *f = __shfl_sync(gmask, *f, lane, LANES);
+    }
+};
 
 // Small (latency-bound) steps' walk, one particle a lane.  The one-lane walk of
 // large steps is a chain of dependent loads a cell at a time: the cell's
@@ -1809,31 +1906,16 @@ __global__ void __launch_bounds__(kSplitBlock, 3) k_neighbors_split(StepArgs a, 
                 list_st(row + r * stride, make_uint4(s[0] + p_off, s[1] + p_off, s[2] + p_off, s[3] + p_off));
         }
     }
-    LamSum ls;
-    if (listed) ls.ks = 1.f;
-    const PairConst pc = pair_const(d);
-    for (uint32_t r0 = 0; r0 < nn; r0 += 8 * kSplit) {  // 8 slots a lane at once
-        float4 x[8];
-#pragma unroll
-        for (uint32_t r = 0; r < 8; ++r) {
-            const uint32_t k = r0 + r * kSplit + sub;
-            x[r] = __ldg(xa + (k < nn ? list[k * kSmallBlock] : i));
-        }
-#pragma unroll
-        for (uint32_t r = 0; r < 8; ++r) {
-            const PairGeo g = pair_geo(xp, x[r]);
-            const PairWS k = masked(pair_ws(g.r2, pc), r0 + r * kSplit + sub < nn);
-#pragma unroll
-            for (uint32_t j = 0; j < kSplit; ++j)
-                ls.add(__shfl_sync(gmask, k.W, j, kSplit), __shfl_sync(gmask, k.s, j, kSplit),
-                       __shfl_sync(gmask, g.d0, j, kSplit), __shfl_sync(gmask, g.d1, j, kSplit),
-                       __shfl_sync(gmask, g.d2, j, kSplit), __shfl_sync(gmask, k.sr, j, kSplit));
-        }
-    }
+    LamWalk o{xp, pair_const(d), LamSum()};
+    if (listed) o.ls.ks = 1.f;
+    for (uint32_t k0 = 0; k0 < nn; k0 += 32)
+        lanes_sum<kSplit>(
+            k0, nn, i, o, [&](uint32_t c) { return list[(k0 + 8 * sub + c) * kSmallBlock]; },
+            [&](uint32_t q) -> float4 { return __ldg(xa + q); });
     if (sub == 0) {
         a.nnb[i] = (uint8_t)nn;
         a.selfat[i] = listed ? (uint8_t)gself : kNotListed;
-        a.xb[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));  // the first delta-p pass gathers both
+        a.xb[i] = make_float4(xp.x, xp.y, xp.z, o.ls.lambda(d));  // the first delta-p pass gathers both
     }
 }
 
@@ -1866,24 +1948,19 @@ __global__ void __launch_bounds__(512, 2) k_lambda(StepArgs a, const float4 *__r
     TILE_LOOP_END
 }
 
-__global__ void __launch_bounds__(kSmallBlock, 8) k_lambda_small(StepArgs a, uint32_t tile,
+// (two lanes: 3 blocks a SM, 136-168 registers; 4 at 128 spill nothing but take
+// 72.1 us a step of 16,384 particles against 70.3, 5 at 96 spill and take 76.2)
+template <uint32_t LANES>
+__global__ void __launch_bounds__(kSmallBlock *LANES, LANES == 1 ? 8 : 3) k_lambda_small(StepArgs a, uint32_t tile,
                                                                  const float4 *__restrict__ xc,
                                                                  float4 *__restrict__ xo)
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
-    const PairConst pc = pair_const(d);
-    const float4 xp = xc[i];
-    LamSum ls;
-    if (a.selfat[i] != kNotListed) ls.ks = 1.f;
-    list_walk_wide(
-        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
-        [&](uint32_t q) -> float4 { return __ldg(xc + q); },
-        [&](const float4 &xj, bool on) {
-            const PairGeo g = pair_geo(xp, xj);
-            ls.add(g, masked(pair_ws(g.r2, pc), on));
-        });
-    xo[i] = make_float4(xp.x, xp.y, xp.z, ls.lambda(d));
+    LamWalk o{xc[i], pair_const(d), LamSum()};
+    if (a.selfat[i] != kNotListed) o.ls.ks = 1.f;
+    if (small_sum<LANES>(a, d.list16 != 0, i, p_off, o, [&](uint32_t q) -> float4 { return __ldg(xc + q); }))
+        xo[i] = make_float4(o.xp.x, o.xp.y, o.xp.z, o.ls.lambda(d));
     SMALL_LOOP_END
 }
 
@@ -2000,19 +2077,30 @@ struct DpSum {
     ScorrConst sc;
     float s0 = 0.f, s1 = 0.f, s2 = 0.f;
     __device__ __forceinline__ DpSum(const SceneDesc &d, float4 x) : xp(x), pc(pair_const(d)), sc(scorr_const(d, x.w)) {}
-    __device__ __forceinline__ void add(const float4 &xq, bool on)
+    struct Term {
+        float f, d0, d1, d2;
+    };
+    __device__ __forceinline__ Term term(const float4 &xq, bool on) const
     {
         const PairGeo g = pair_geo<PK>(xp, xq);
         const PairWS k = pair_ws(g.r2, pc);
-        const float f0 = __fmul_rn(dp_coef<FORM>(xp.w, xq.w, k.W, sc), k.s);
-        const float f = on ? f0 : 0.f;
+        const float f = __fmul_rn(dp_coef<FORM>(xp.w, xq.w, k.W, sc), k.s);
+        return Term{on ? f : 0.f, g.d0, g.d1, g.d2};
+    }
+    __device__ __forceinline__ void add(const Term &t)
+    {
         if (PK) {
-            fma2(s0, s1, f, f, g.d0, g.d1);
+            fma2(s0, s1, t.f, t.f, t.d0, t.d1);
         } else {
-            s0 = __fmaf_rn(f, g.d0, s0);
-            s1 = __fmaf_rn(f, g.d1, s1);
+            s0 = __fmaf_rn(t.f, t.d0, s0);
+            s1 = __fmaf_rn(t.f, t.d1, s1);
         }
-        s2 = __fmaf_rn(f, g.d2, s2);
+        s2 = __fmaf_rn(t.f, t.d2, s2);
+    }
+    template <uint32_t LANES>
+    __device__ __forceinline__ void pass(uint32_t gmask, uint32_t lane)
+    {
+        for (float *f : {&s0, &s1, &s2}) *f = __shfl_sync(gmask, *f, lane, LANES);
     }
 };
 
@@ -2034,27 +2122,27 @@ __global__ void __launch_bounds__(512, 2) k_dp(StepArgs a, const float4 *__restr
         DpSum<decltype(form)::value, true> o(d, xp);
         list_walk_any<kChunk>(
             d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
-            [&](uint32_t q) -> float4 { return __ldg(xc + q); }, [&](const float4 &xq, bool on) { o.add(xq, on); });
+            [&](uint32_t q) -> float4 { return __ldg(xc + q); }, [&](const float4 &xq, bool on) { o.add(o.term(xq, on)); });
         return make_float3(o.s0, o.s1, o.s2);
     });
     dp_finish(a, d, s, i, xp, sum, xo, last);
     TILE_LOOP_END
 }
 
-__global__ void __launch_bounds__(kSmallBlock, 8) k_dp_small(StepArgs a, uint32_t tile, const float4 *__restrict__ xc,
+template <uint32_t LANES>
+__global__ void __launch_bounds__(kSmallBlock *LANES, LANES == 1 ? 8 : 3) k_dp_small(StepArgs a, uint32_t tile, const float4 *__restrict__ xc,
                                                              float4 *__restrict__ xo, int last)
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
     const float4 xp = xc[i];
+    bool first = true;
     const float3 sum = by_scorr(d, [&](auto form) {
         DpSum<decltype(form)::value, false> o(d, xp);
-        list_walk_wide(
-            d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
-            [&](uint32_t q) -> float4 { return __ldg(xc + q); }, [&](const float4 &xq, bool on) { o.add(xq, on); });
+        first = small_sum<LANES>(a, d.list16 != 0, i, p_off, o, [&](uint32_t q) -> float4 { return __ldg(xc + q); });
         return make_float3(o.s0, o.s1, o.s2);
     });
-    dp_finish(a, d, s, i, xp, sum, xo, last);
+    if (first) dp_finish(a, d, s, i, xp, sum, xo, last);
     SMALL_LOOP_END
 }
 
@@ -2085,18 +2173,36 @@ struct OmegaSum {
     float4 xi, vi;
     float kh, w0 = 0.f, w1 = 0.f, w2 = 0.f;
     __device__ __forceinline__ OmegaSum(float4 x, float4 v, float k) : xi(x), vi(v), kh(k) {}
-    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz, bool on = true)
+    struct Term {
+        float c0, c1, c2, wd;
+        bool on;
+    };
+    __device__ __forceinline__ Term term(float4 xj, float vx, float vy, float vz, bool on) const
     {
         const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
         const float r2 = p0 * p0 + p1 * p1 + p2 * p2;
-        if (on && r2 > 0.f) {
-            const float inv_r = rsqrtf(r2);
-            const float v0 = vx - vi.x, v1 = vy - vi.y, v2 = vz - vi.z;
-            const float wd = wspiky_d(r2 * inv_r, kh) * inv_r;
-            w0 += (v1 * p2 - v2 * p1) * wd;
-            w1 += (v2 * p0 - v0 * p2) * wd;
-            w2 += (v0 * p1 - v1 * p0) * wd;
+        const float inv_r = rsqrtf(r2);
+        const float v0 = vx - vi.x, v1 = vy - vi.y, v2 = vz - vi.z;
+        return Term{v1 * p2 - v2 * p1, v2 * p0 - v0 * p2, v0 * p1 - v1 * p0, wspiky_d(r2 * inv_r, kh) * inv_r,
+                    on && r2 > 0.f};
+    }
+    __device__ __forceinline__ Term term(const PhaseRec &r, bool on) const { return term(r.A, r.A.w, r.B.x, r.B.y, on); }
+    __device__ __forceinline__ void add(const Term &t)
+    {
+        if (t.on) {
+            w0 += t.c0 * t.wd;
+            w1 += t.c1 * t.wd;
+            w2 += t.c2 * t.wd;
         }
+    }
+    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz, bool on = true)
+    {
+        add(term(xj, vx, vy, vz, on));
+    }
+    template <uint32_t LANES>
+    __device__ __forceinline__ void pass(uint32_t gmask, uint32_t lane)
+    {
+        for (float *f : {&w0, &w1, &w2}) *f = __shfl_sync(gmask, *f, lane, LANES);
     }
 };
 
@@ -2139,7 +2245,8 @@ __global__ void __launch_bounds__(512, 2) k_vort_omega(StepArgs a)
     TILE_LOOP_END
 }
 
-__global__ void __launch_bounds__(kSmallBlock, 8) k_vort_omega_small(StepArgs a, uint32_t tile)
+template <uint32_t LANES>
+__global__ void __launch_bounds__(kSmallBlock *LANES, LANES == 1 ? 8 : 3) k_vort_omega_small(StepArgs a, uint32_t tile)
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
@@ -2149,11 +2256,9 @@ __global__ void __launch_bounds__(kSmallBlock, 8) k_vort_omega_small(StepArgs a,
     const float4 A = pa[i];
     const float2 B = pb[i];
     OmegaSum o(A, make_float4(A.w, B.x, B.y, 0.f), d.inv_h);
-    list_walk_wide(
-        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
-        [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; },
-        [&](const PhaseRec &r, bool on) { o.add(r.A, r.A.w, r.B.x, r.B.y, on); });
-    put_omega(a, d, i, o);
+    if (small_sum<LANES>(a, d.list16 != 0, i, p_off, o,
+                         [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; }))
+        put_omega(a, d, i, o);
     SMALL_LOOP_END
 }
 
@@ -2194,17 +2299,30 @@ struct EtaSum {
     float4 xi;
     float kh, sgn, n0 = 0.f, n1 = 0.f, n2 = 0.f;
     __device__ __forceinline__ EtaSum(float4 x, float k, float sg) : xi(x), kh(k), sgn(sg) {}
-    __device__ __forceinline__ void add(float4 xj, bool on = true)  // (x_j, |omega_j|)
+    struct Term {
+        float f, p0, p1, p2;
+        bool on;
+    };
+    __device__ __forceinline__ Term term(float4 xj, bool on) const  // (x_j, |omega_j|)
     {
         const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
         const float r2 = p0 * p0 + p1 * p1 + p2 * p2;
-        if (on && r2 > 0.f) {
-            const float inv_r = rsqrtf(r2);
-            const float f = sgn * xj.w * wspiky_d(r2 * inv_r, kh) * inv_r;
-            n0 += f * p0;
-            n1 += f * p1;
-            n2 += f * p2;
+        const float inv_r = rsqrtf(r2);
+        return Term{sgn * xj.w * wspiky_d(r2 * inv_r, kh) * inv_r, p0, p1, p2, on && r2 > 0.f};
+    }
+    __device__ __forceinline__ void add(const Term &t)
+    {
+        if (t.on) {
+            n0 += t.f * t.p0;
+            n1 += t.f * t.p1;
+            n2 += t.f * t.p2;
         }
+    }
+    __device__ __forceinline__ void add(float4 xj, bool on = true) { add(term(xj, on)); }
+    template <uint32_t LANES>
+    __device__ __forceinline__ void pass(uint32_t gmask, uint32_t lane)
+    {
+        for (float *f : {&n0, &n1, &n2}) *f = __shfl_sync(gmask, *f, lane, LANES);
     }
 };
 
@@ -2252,17 +2370,16 @@ __global__ void __launch_bounds__(512, 2) k_vort_apply(StepArgs a)
     TILE_LOOP_END
 }
 
-__global__ void __launch_bounds__(kSmallBlock, 8) k_vort_apply_small(StepArgs a, uint32_t tile)
+template <uint32_t LANES>
+__global__ void __launch_bounds__(kSmallBlock *LANES, LANES == 1 ? 8 : 3) k_vort_apply_small(StepArgs a, uint32_t tile)
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
     if (d.vort_mode != PBF_VORTICITY_TEXTBOOK) return;
     const float4 *__restrict__ xw = a.xs;
     EtaSum e(xw[i], d.inv_h, -1.f);
-    list_walk_wide(
-        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
-        [&](uint32_t q) -> float4 { return __ldg(xw + q); }, [&](const float4 &xj, bool on) { e.add(xj, on); });
-    put_confinement(a, d, i, e);
+    if (small_sum<LANES>(a, d.list16 != 0, i, p_off, e, [&](uint32_t q) -> float4 { return __ldg(xw + q); }))
+        put_confinement(a, d, i, e);
     SMALL_LOOP_END
 }
 
@@ -2319,19 +2436,36 @@ struct XsphSum {
         : xi(x), vi(v), ih2(d.inv_h * d.inv_h), alpha6(d.alpha6)
     {
     }
-    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz, bool on = true)
+    struct Term {
+        float W, v0, v1, v2;
+        bool on;
+    };
+    __device__ __forceinline__ Term term(float4 xj, float vx, float vy, float vz, bool on) const
     {
         const float p0 = xj.x - xi.x, p1 = xj.y - xi.y, p2 = xj.z - xi.z;
         // Wpoly6 from r^2 (q^2 = r^2 / h^2 instead of (|r| / h)^2: no square
         // root per pair; the two differ by rounding only)
         const float q2 = (p0 * p0 + p1 * p1 + p2 * p2) * ih2;
         const float t = 1.f - q2;
-        const float W = q2 <= 1.f ? alpha6 * t * t * t : 0.f;
-        if (on) {  // (not W = 0: an infinite velocity's difference from itself is NaN)
-            s0 += (vx - vi.x) * W;
-            s1 += (vy - vi.y) * W;
-            s2 += (vz - vi.z) * W;
+        return Term{q2 <= 1.f ? alpha6 * t * t * t : 0.f, vx - vi.x, vy - vi.y, vz - vi.z, on};
+    }
+    __device__ __forceinline__ Term term(const PhaseRec &r, bool on) const { return term(r.A, r.A.w, r.B.x, r.B.y, on); }
+    __device__ __forceinline__ void add(const Term &t)
+    {
+        if (t.on) {  // (not W = 0: an infinite velocity's difference from itself is NaN)
+            s0 += t.v0 * t.W;
+            s1 += t.v1 * t.W;
+            s2 += t.v2 * t.W;
         }
+    }
+    __device__ __forceinline__ void add(float4 xj, float vx, float vy, float vz, bool on = true)
+    {
+        add(term(xj, vx, vy, vz, on));
+    }
+    template <uint32_t LANES>
+    __device__ __forceinline__ void pass(uint32_t gmask, uint32_t lane)
+    {
+        for (float *f : {&s0, &s1, &s2}) *f = __shfl_sync(gmask, *f, lane, LANES);
     }
     __device__ __forceinline__ float4 result(const SceneDesc &d) const
     {
@@ -2370,7 +2504,8 @@ __global__ void __launch_bounds__(512) k_xsph(StepArgs a)
     TILE_LOOP_END
 }
 
-__global__ void __launch_bounds__(kSmallBlock, 8) k_xsph_small(StepArgs a, uint32_t tile)
+template <uint32_t LANES>
+__global__ void __launch_bounds__(kSmallBlock *LANES, LANES == 1 ? 8 : 3) k_xsph_small(StepArgs a, uint32_t tile)
 {
     SMALL_LOOP_BEGIN
     const SceneDesc d = a.scenes[s];
@@ -2380,11 +2515,9 @@ __global__ void __launch_bounds__(kSmallBlock, 8) k_xsph_small(StepArgs a, uint3
     const float4 A = pa[i];
     const float2 B = pb[i];
     XsphSum o(A, make_float4(A.w, B.x, B.y, 0.f), d);
-    list_walk_wide(
-        d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nbr_rows, a.nnb[i], p_off, i,
-        [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; },
-        [&](const PhaseRec &r, bool on) { o.add(r.A, r.A.w, r.B.x, r.B.y, on); });
-    a.v[__float_as_uint(a.xold[i].w)] = o.result(d);
+    if (small_sum<LANES>(a, d.list16 != 0, i, p_off, o,
+                         [&](uint32_t q) -> PhaseRec { return PhaseRec{__ldg(pa + q), __ldg(pb + q)}; }))
+        a.v[__float_as_uint(a.xold[i].w)] = o.result(d);
     SMALL_LOOP_END
 }
 
@@ -2715,6 +2848,7 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
         if (hook) hook->launched(name);   \
     } while (0)
     const uint32_t gs = sh.small_tiles * (sh.tile / kSmallBlock);  // small steps: a block per part of a tile
+    const uint32_t ls = kSmallBlock * (sh.small_lanes ? kLanes : 1u);  // threads of their list passes' blocks
     const bool front = sh.front && !hook;  // (a profile gets the phases one by one)
     if (front) {
         launch_cluster(front_fn(sh.front, packed), sh.front_cluster, st, a, sh.tile_shift, sh.small_tiles);
@@ -2784,14 +2918,14 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
         const int last = it == iters - 1 ? 1 : 0;
         if (it > 0) {
             if (sh.small) {
-                k_lambda_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile, a.xa, a.xb);
+                (sh.small_lanes ? k_lambda_small<kLanes> : k_lambda_small<1>)<<<gs, ls, 0, st>>>(a, sh.tile, a.xa, a.xb);
             } else {
                 PBF_PASS_DISPATCH(sh.chunk, launch_lambda(a, sh, st));
             }
             PBF_LAUNCHED("k_lambda");
         }
         if (sh.small) {
-            k_dp_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile, a.xb, a.xa, last);
+            (sh.small_lanes ? k_dp_small<kLanes> : k_dp_small<1>)<<<gs, ls, 0, st>>>(a, sh.tile, a.xb, a.xa, last);
         } else {
             PBF_PASS_DISPATCH(sh.chunk, launch_dp(a, sh, last, st));
         }
@@ -2805,7 +2939,7 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
     const bool l16 = (post & kPostList16) != 0, l32 = (post & kPostList32) != 0;
 #define PBF_POST(kernel, grid)                                               \
     if (sh.small) {                                                          \
-        kernel##_small<<<gs, kSmallBlock, 0, st>>>(a, sh.tile);              \
+        (sh.small_lanes ? kernel##_small<kLanes> : kernel##_small<1>)<<<gs, ls, 0, st>>>(a, sh.tile); \
         PBF_LAUNCHED(#kernel);                                               \
     } else {                                                                 \
         if (l32) {                                                           \

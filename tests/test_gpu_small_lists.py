@@ -23,7 +23,8 @@ def _scenes():
 
 def _run(scs, params, filler, max_pair, capacity, steps=4):
     small = [(sc, H.resolved(params, sc)) for sc in scs]
-    fill = [scenes.dam_break(52, 52, 50, (4.0, 4.0, 4.0), scene_id=390)] if filler else []
+    side = {False: 0, True: 52, "mid": 32}[filler]
+    fill = [scenes.dam_break(side, side, side, (4.0, 4.0, 4.0), scene_id=390)] if side else []
     rest = [(sc, H.resolved(params, sc)) for sc in fill]
     cells = sum(int(np.prod(p["grid_size"])) + 1 for _, p in small + rest)
     b = api.Batch(len(small) + len(rest), sum(max(sc.n, capacity) for sc, _ in small + rest), cells, max_pair)
@@ -48,7 +49,20 @@ def test_small_step_lists_equal_large_steps(gpu, max_pair, capacity):
         assert np.array_equal(va.view(np.uint32), vb.view(np.uint32)), k
 
 
-@pytest.mark.parametrize("filler", [False, True], ids=["small", "large"])
+@pytest.mark.parametrize("capacity", [0, 70000], ids=["u16", "u32"])
+@pytest.mark.parametrize("max_pair", [9, 16, 18, 30, 34, 70])
+def test_lanes_and_one_lane_lists_equal(gpu, max_pair, capacity):
+    """Two lanes a particle (few particles) against one (32,768 more): sums
+    pass from lane to lane in list order."""
+    params = api.config_params(scorr_k=1e-4, max_pair_particle_num=max_pair)
+    scs = _scenes()[:3] if capacity else _scenes()
+    for k, ((xa, va), (xb, vb)) in enumerate(zip(_run(scs, params, False, max_pair, capacity),
+                                                 _run(scs, params, "mid", max_pair, capacity))):
+        assert np.array_equal(xa.view(np.uint32), xb.view(np.uint32)), k
+        assert np.array_equal(va.view(np.uint32), vb.view(np.uint32)), k
+
+
+@pytest.mark.parametrize("filler", [False, "mid", True], ids=["small", "mid", "large"])
 @pytest.mark.parametrize("capacity", [0, 70000], ids=["u16", "u32"])
 def test_infinite_velocities_count_listed_neighbours_only(gpu, capacity, filler):
     """Pairs far apart from each other whose confinement overflows to opposite
