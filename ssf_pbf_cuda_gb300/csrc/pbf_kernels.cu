@@ -1566,29 +1566,38 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
         auto src = [&](uint32_t k) { return rd[(k + (k >= selfat ? 1u : 0u)) * blockDim.x]; };
         // the list out in whole quads (u32) or octs (u16): one 16-byte store
         // per four or eight slots (slots past the count in the last one are
-        // padding, never read)
+        // padding, never read), and the same eight slots' pairs, four at a
+        // time (past the end: the particle itself, masked).  Written out
+        // first and read again for the pairs: 1,335 us at 5.95 M particles in
+        // 256 scenes, 1,300 so
         uint4 *wq = reinterpret_cast<uint4 *>(nl);
-        if (l16) {
-            for (uint32_t k0 = 0; k0 < cnt; k0 += 8) {
+        for (uint32_t k0 = 0; k0 < cnt; k0 += 8) {
+            uint32_t q[8];
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) q[k] = k0 + k < cnt ? src(k0 + k) : i;
+            if (l16) {
                 uint32_t w[4];
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) {
-                    const uint32_t lo = (k0 + 2 * j < cnt) ? src(k0 + 2 * j) - d.p_off : 0u;
-                    const uint32_t hi = (k0 + 2 * j + 1 < cnt) ? src(k0 + 2 * j + 1) - d.p_off : 0u;
-                    w[j] = (lo & 0xFFFFu) | (hi << 16);
-                }
+                for (uint32_t k = 0; k < 4; ++k) w[k] = __byte_perm(q[2 * k] - d.p_off, q[2 * k + 1] - d.p_off, 0x5410);
                 list_st(wq + (uint64_t)(k0 >> 3) * stride, make_uint4(w[0], w[1], w[2], w[3]));
+            } else {
+                list_st(wq + (uint64_t)(k0 >> 2) * stride, make_uint4(q[0], q[1], q[2], q[3]));
+                if (k0 + 4 < cnt) list_st(wq + (uint64_t)((k0 >> 2) + 1) * stride, make_uint4(q[4], q[5], q[6], q[7]));
             }
-        } else {
-            for (uint32_t k0 = 0; k0 < cnt; k0 += 4) {
-                uint32_t q4[4];
 #pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) q4[j] = (k0 + j < cnt) ? src(k0 + j) : 0u;
-                list_st(wq + (uint64_t)(k0 >> 2) * stride, make_uint4(q4[0], q4[1], q4[2], q4[3]));
+            for (uint32_t h = 0; h < 8; h += 4) {
+                if (h == 0 || k0 + h < cnt) {
+                    float4 x[4];
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) x[k] = __ldg(xa + q[h + k]);
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) {
+                        const PairGeo g = pair_geo(xp, x[k]);
+                        ls.add(g, masked(pair_ws(g.r2, pc), k0 + h + k < cnt));
+                    }
+                }
             }
         }
-#pragma unroll 4
-        for (uint32_t k = 0; k < cnt; ++k) lam_add(ls, xp, __ldg(xa + src(k)), pc);
     } else {
 #pragma unroll 4
         for (uint32_t k = 0; k < cnt; ++k) {
