@@ -510,7 +510,7 @@ def main():
     ap.add_argument("--preheat", type=float, default=3.0,
                     help="seconds of untimed steps before the warm-up: a GPU coming out of idle runs the first "
                          "seconds ~5%% slower")
-    ap.add_argument("--chunk", type=int, default=0, help="neighbour chunk of the lambda/dp passes (0 = autotune)")
+    ap.add_argument("--chunk", type=int, default=0, help="neighbour chunk of the lambda passes (0 = autotune)")
     ap.add_argument("--serve-seconds", type=float, default=5.0,
                     help="arrival window of each serving run of the rate ramp (0 = off)")
     ap.add_argument("--serve-rate", type=float, default=0.0,

@@ -264,8 +264,9 @@ pbf_status pbf_batch_get_all_async(pbf_batch *b, uint32_t *counts_dev, float *x_
  * Leaves particle state unchanged. */
 pbf_status pbf_batch_autotune(pbf_batch *b, int iters, void *stream, uint32_t *chosen_tile);
 pbf_status pbf_batch_set_tile(pbf_batch *b, uint32_t tile);
-/* Neighbour indices requested ahead per thread in the lambda / delta-p
- * passes (4 or 8; the autotuner also picks it).  Results do not depend on it.
+/* Neighbour indices requested ahead per thread in the lambda passes of large
+ * steps (4 or 8; the autotuner also picks it; scenes that expect at most 16
+ * neighbours a particle always use 4).  Results do not depend on it.
  * No reference counterpart. */
 pbf_status pbf_batch_set_chunk(pbf_batch *b, uint32_t chunk);
 /* Current tile (particles per block) and chunk. */

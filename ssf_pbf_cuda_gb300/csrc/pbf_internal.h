@@ -135,7 +135,7 @@ struct LaunchShape {
     uint32_t scan_grid;   // grid for the three scan kernels; 0 = one kernel
     uint32_t scan_cluster; // one kernel: blocks of its cluster, 0 = one block
     uint32_t scan_rounds; // one kernel: rounds of 1024 cells a block holds in registers
-    uint32_t chunk;       // neighbours per chunk in the lambda / delta-p passes (4 or 8)
+    uint32_t chunk;       // neighbours per chunk in the large steps' lambda pass (4 or 8)
     // persistent grids of the heavy kernels, each from its own occupancy
     uint32_t grid_nb, grid_lambda, grid_dp;
     uint32_t grid_omega[2], grid_apply[2], grid_xsph[2];  // list-form post passes: u32 lists, u16 lists

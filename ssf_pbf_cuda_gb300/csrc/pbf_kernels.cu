@@ -520,7 +520,7 @@ __device__ __forceinline__ void list_group(uint32_t left, uint32_t self, IDX &&i
 
 // Visit list slots [0, nn) of one particle in list order.  Indices are
 // requested CH at a time (CH / 4 quads), one chunk ahead of their use; the
-// chunk (loads in flight against registers) is picked by the autotuner.  The
+// chunk (loads in flight against registers) is each pass's choice.  The
 // last, partial chunk is taken in groups of four.
 template <int CH, class LD, class USE>
 __device__ __forceinline__ void list_walk(const uint32_t *__restrict__ nl, uint64_t stride, uint32_t nn, uint32_t self,
@@ -2114,8 +2114,9 @@ struct DpSum {
 };
 
 // delta-p with s_corr (calcPositionUpdateCUDA cached, pbf_position_update.cu:131-188),
-// in list order.
-template <int kChunk>
+// in list order.  Chunks of 4: 4 x 277 us at 5.95 M particles in 256 scenes
+// (290 in chunks of 8), 4 x 34 at 1 M of h = 1.4 spacings (38), the same at 1 M of
+// h = 2 spacings; the pair's longer arithmetic leaves fewer registers than lambda's.
 __global__ void __launch_bounds__(512, 2) k_dp(StepArgs a, const float4 *__restrict__ xc, float4 *__restrict__ xo,
                                                int last)
 {
@@ -2129,7 +2130,7 @@ __global__ void __launch_bounds__(512, 2) k_dp(StepArgs a, const float4 *__restr
     const float4 xp = xc[i];
     const float3 sum = by_scorr(d, [&](auto form) {
         DpSum<decltype(form)::value, true> o(d, xp);
-        list_walk_any<kChunk>(
+        list_walk_any<4>(
             d.list16 != 0, list_of(a.nbr, i), a.nbr_stride, a.nnb[i], d.p_off, i,
             [&](uint32_t q) -> float4 { return __ldg(xc + q); }, [&](const float4 &xq, bool on) { o.add(o.term(xq, on)); });
         return make_float3(o.s0, o.s1, o.s2);
@@ -2691,25 +2692,9 @@ __global__ void k_store_phase(const float4 *__restrict__ x, const float4 *__rest
 
 }  // namespace
 
-// The large steps' lambda / delta-p variants by neighbour chunk, selected at
-// run time.
-template <int CH>
-struct PassFns {
-    static const void *lambda() { return (const void *)k_lambda<CH>; }
-    static const void *dp() { return (const void *)k_dp<CH>; }
-    static void launch_lambda(const StepArgs &a, const LaunchShape &sh, cudaStream_t st)
-    {
-        k_lambda<CH><<<sh.grid_lambda, sh.tile, 0, st>>>(a, a.xa, a.xb);
-    }
-    static void launch_dp(const StepArgs &a, const LaunchShape &sh, int last, cudaStream_t st)
-    {
-        k_dp<CH><<<sh.grid_dp, sh.tile, 0, st>>>(a, a.xb, a.xa, last);
-    }
-};
-
-#define PBF_PASS_DISPATCH(chunk, CALL) \
-    if ((chunk) == 4) PassFns<4>::CALL; \
-    else PassFns<8>::CALL;
+// The large steps' lambda pass by neighbour chunk, selected at run time.
+using LambdaFn = void (*)(StepArgs, const float4 *, float4 *);
+static LambdaFn lambda_fn(uint32_t chunk) { return chunk == 4 ? k_lambda<4> : k_lambda<8>; }
 
 // Resident blocks per SM of each kernel at a tile size (cached per device,
 // tile and chunk: the step asks for its launch shape every time it runs).
@@ -2744,9 +2729,8 @@ Occupancy occupancy(uint32_t tile, uint32_t chunk)
                          (int)kNbSmemMax);
     cudaFuncSetAttribute((const void *)k_neighbors_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNbSmemMax);
     cudaFuncSetAttribute((const void *)k_neighbors_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNbSmemMax);
-    const bool c4 = chunk == 4;
-    o.lambda = occ(c4 ? PassFns<4>::lambda() : PassFns<8>::lambda());
-    o.dp = occ(c4 ? PassFns<4>::dp() : PassFns<8>::dp());
+    o.lambda = occ((const void *)lambda_fn(chunk));
+    o.dp = occ((const void *)k_dp);
     o.omega[0] = occ((const void *)k_vort_omega<false>);
     o.omega[1] = occ((const void *)k_vort_omega<true>);
     o.apply[0] = occ((const void *)k_vort_apply<false>);
@@ -2929,14 +2913,14 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
             if (sh.small) {
                 (sh.small_lanes ? k_lambda_small<kLanes> : k_lambda_small<1>)<<<gs, ls, 0, st>>>(a, sh.tile, a.xa, a.xb);
             } else {
-                PBF_PASS_DISPATCH(sh.chunk, launch_lambda(a, sh, st));
+                lambda_fn(sh.chunk)<<<sh.grid_lambda, b, 0, st>>>(a, a.xa, a.xb);
             }
             PBF_LAUNCHED("k_lambda");
         }
         if (sh.small) {
             (sh.small_lanes ? k_dp_small<kLanes> : k_dp_small<1>)<<<gs, ls, 0, st>>>(a, sh.tile, a.xb, a.xa, last);
         } else {
-            PBF_PASS_DISPATCH(sh.chunk, launch_dp(a, sh, last, st));
+            k_dp<<<sh.grid_dp, b, 0, st>>>(a, a.xb, a.xa, last);
         }
         PBF_LAUNCHED("k_dp");
     }
