@@ -141,15 +141,15 @@ struct LaunchShape {
     uint32_t grid_omega[2], grid_apply[2], grid_xsph[2];  // list-form post passes: u32 lists, u16 lists
     uint32_t grid_cells;  // grid of k_rank_cells: a block of cell_tile threads per cell tile
     uint32_t cell_tile;   // cells per cell tile = threads per k_rank_cells block (autotuned)
-    uint32_t small;       // latency-bound step (at most kSmallStep particle slots): split
-                          // neighbour walk, per-particle rank, wide list reads
+    uint32_t small;       // latency-bound step (at most kSmallStep particle slots): walk by shared
+                          // ranges, per-particle rank, wide list reads
     uint32_t front;       // small steps: k_front's rounds of 1024 cells a block, 0 = a kernel per phase
     uint32_t front_cluster; // blocks of its cluster
     uint32_t tile_shift;  // log2 of tile
-    uint32_t small_split; // small steps: their walk takes kSplit lanes a particle
+    uint32_t small_split; // small steps: their walk takes kSplit lanes a particle (k_neighbors_split)
     uint32_t small_lanes; // small steps: their list passes take kLanes lanes a particle
     uint32_t small_tiles; // small steps: tiles rounded up to a power of two, for which headers are written
-    uint32_t nb_smem;     // k_neighbors_lambda: bytes of shared memory for the block's lists (0 = stored directly)
+    uint32_t nb_smem;     // the walk's bytes of shared memory for the block's lists (large steps: 0 = stored directly)
     bool operator==(const LaunchShape &o) const
     {
         return tile == o.tile && grid == o.grid && scan_grid == o.scan_grid && scan_rounds == o.scan_rounds && scan_cluster == o.scan_cluster &&

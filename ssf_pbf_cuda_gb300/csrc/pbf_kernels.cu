@@ -1475,9 +1475,10 @@ __global__ void __launch_bounds__(1024) k_front(StepArgs a, uint32_t tile_shift,
 // the working positions are the sorted predicted positions, so the pair
 // terms can be summed while the list is built.
 // SMEM: the accepted indices are collected in shared memory ([slot][thread]
-// per block, conflict-free), then written to the list in whole quads (a
-// warp's 16-byte stores contiguous) instead of one scattered 4-byte store per
-// accepted candidate, and the lambda loop reads them back from shared memory.
+// per block, conflict-free), then written to the list in whole rows (a
+// warp's 16-byte stores contiguous) instead of one scattered store per
+// accepted candidate, and summed as they are read.  Otherwise (lists beyond
+// kNbSmemMax a block) they are stored directly and read back.
 template <bool SMEM>
 __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
 {
@@ -1556,11 +1557,11 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
     cnt -= selfat < cnt ? 1u : 0u;  // entries stored
     a.nnb[i] = (uint8_t)cnt;
     a.selfat[i] = (uint8_t)selfat;
-    // phase 2: lambda over the list just written (L2-resident; plain loads,
+    // phase 2: lambda over the list (direct stores: read back by plain loads,
     // the read-only path may not see this kernel's own stores)
     LamSum ls;
     if (selfat != kNotListed) ls.ks = 1.f;
-    if (SMEM) {  // the list from shared memory, written out slot by slot as it is summed
+    if (SMEM) {  // the list from shared memory, written out as it is summed
         // stored entry k is shared-memory entry k, or k + 1 from the
         // particle's own slot on
         auto src = [&](uint32_t k) { return rd[(k + (k >= selfat ? 1u : 0u)) * blockDim.x]; };
@@ -1830,9 +1831,8 @@ __global__ void __launch_bounds__(kSmallBlock, 8) k_neighbors_small(StepArgs a, 
 // takes a run of the near cells into its own part of shared memory, a prefix
 // over the group's counts lays the runs end to end up to the cap (the
 // reference's first cap accepted candidates in walk order), lane k writes
-// every fourth row of the list, and the lambda terms of slots k, k + kSplit,
-// ... reach the group by shuffles and are added in list order by each lane
-// (the one-lane sums, bit for bit).  The step of 4,096 particles 73 -> 68 us
+// every fourth row of the list, and the lambda sums go from lane to lane over
+// 8 slots each (lanes_sum; the one-lane sums, bit for bit).  The step of 4,096 particles 73 -> 68 us
 // against the split without shared ranges; a fourth block a SM (64 registers)
 // spills and takes 72.
 __global__ void __launch_bounds__(kSplitBlock, 3) k_neighbors_split(StepArgs a, uint32_t tile)
