@@ -45,3 +45,18 @@ def test_depth_by_tiles_at_sprite_sizes(gpu, mode, radius):
     r.render(x)
     inv, inc = r.frame_constants()
     assert np.array_equal(r.image("depth"), S.splat(S.frame(r.params, inv, inc), x))
+
+
+@pytest.mark.parametrize("radius", [5.5e-6, 2e-4, 0.05], ids=["inside", "edges", "outside"])
+@pytest.mark.parametrize("size", [(129, 66), (5, 3), (1, 1)], ids=lambda s: f"{s[0]}x{s[1]}")
+def test_blur_taps_inside_and_past_the_edges(gpu, size, radius):
+    """Taps within a texel, at the borders' texels and past every border,
+    against the oracle's blur (expf differs by a few ulps: 2e-6, as the other
+    passes' tests allow)."""
+    r = api.SsfRenderer(api.ssf_default_params(width=size[0], height=size[1], blur_passes=1, point_radius=1.5,
+                                               blur_radius=radius))
+    r.render(_cloud(r, 3000, 9, "mixed"))
+    inv, inc = r.frame_constants()
+    got, want = r.image("blurred"), S.blur(S.frame(r.params, inv, inc), r.image("blur_input"))
+    assert np.array_equal(got == 1, want == 1)
+    assert np.max(np.abs(got - want)) <= 2e-6
