@@ -1,0 +1,38 @@
+// Kernels of one call launched one by one on a stream, each set up while the
+// one before it still runs (programmatic dependent launch).
+#pragma once
+#include <cuda_runtime.h>
+
+namespace pbf103 {
+
+// Lets the launch after this one be set up; its blocks wait in after_previous
+// themselves.  (For a call's first kernel, which is launched as usual.)
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// First in every kernel launched by launch_after, before any access to memory:
+// waits until the launch before it is complete (its writes are visible from
+// here on, and so, in turn, are those of the launches before that).
+__device__ __forceinline__ void after_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    release_next();
+}
+
+// Launches fn, whose first act is after_previous().  The next launch that is
+// not a launch_after waits for all of them, as any launch does.
+template <class... K, class... A>
+void launch_after(void (*fn)(K...), dim3 blocks, dim3 threads, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = blocks;
+    cfg.blockDim = threads;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, fn, static_cast<K>(args)...);  // (errors: the caller's cudaGetLastError)
+}
+
+}  // namespace pbf103

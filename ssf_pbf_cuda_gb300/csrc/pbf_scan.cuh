@@ -4,6 +4,7 @@
 #include <cooperative_groups.h>
 #include <cstdint>
 
+#include "pbf_after.cuh"
 #include "pbf_internal.h"
 
 namespace pbf103 {
@@ -81,19 +82,22 @@ inline uint32_t cluster_scan_rounds(uint32_t n, uint32_t blocks)
 }
 
 // Launches fn (a kernel of 1024-thread blocks) as one cluster of `blocks`.
-template <class... A>
+// AFTER: as launch_after does.
+template <bool AFTER = false, class... A>
 cudaError_t launch_cluster(void (*fn)(A...), uint32_t blocks, cudaStream_t st, A... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(1024);
     cfg.stream = st;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = blocks;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = blocks;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = AFTER ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 
