@@ -5,18 +5,19 @@
 
 namespace pbf103 {
 
-// Lets the launch after this one be set up; its blocks wait in after_previous
-// themselves.  (For a call's first kernel, which is launched as usual.)
-__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // First in every kernel launched by launch_after, before any access to memory:
 // waits until the launch before it is complete (its writes are visible from
 // here on, and so, in turn, are those of the launches before that).
-__device__ __forceinline__ void after_previous()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    release_next();
-}
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the launch after this one be set up once every block of this one has
+// come here (otherwise once every block is done); its blocks wait in
+// after_previous themselves.  After after_previous, but for a call's first
+// kernel, which is launched as usual.  Not for grids of several waves: the
+// waiting blocks take their places (a frame of 524,288
+// particles at 1920 x 1080 184 us without it in the blurs and normals, 199 with,
+// 189 by plain launches).
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Launches fn, whose first act is after_previous().  The next launch that is
 // not a launch_after waits for all of them, as any launch does.

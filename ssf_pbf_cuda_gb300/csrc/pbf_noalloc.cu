@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(1024) na_scan_cluster(uint32_t C, Scratch s, u
                                                         uint32_t *__restrict__ ce)
 {
     pbf103::after_previous();
+    pbf103::release_next();
     if (blockIdx.x == 0 && threadIdx.x == 0) s.big[0] = 0;
     const uint32_t all = pbf103::cluster_scan<R>([&](uint32_t c) { return s.counts[c]; }, C, [&](uint32_t c, uint32_t offset, uint32_t count) {
         s.offsets[c] = offset;
@@ -196,6 +197,7 @@ __global__ void na_scan_tiles(uint32_t C, Scratch s, uint32_t *__restrict__ cs, 
 __global__ void na_scatter(uint32_t n, Scratch s)
 {
     pbf103::after_previous();
+    pbf103::release_next();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) s.tmp[s.offsets[s.keys[i]] + s.slots[i]] = i;
 }
@@ -206,6 +208,7 @@ __global__ void na_scatter(uint32_t n, Scratch s)
 __global__ void na_rank(uint32_t n, Scratch s, uint32_t *__restrict__ perm)
 {
     pbf103::after_previous();
+    pbf103::release_next();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t k = s.keys[i];
@@ -231,6 +234,7 @@ __global__ void __launch_bounds__(pbf103::kRadixThreads) na_big(uint32_t n, Scra
     __shared__ pbf103::RadixSmem sm;
     __shared__ uint32_t base[16], tot[16];
     pbf103::after_previous();
+    pbf103::release_next();
     const uint32_t nb = s.big[0];
     for (uint32_t q = blockIdx.x; q < nb; q += gridDim.x) {
         const uint32_t k = s.big[1 + q];

@@ -17,6 +17,7 @@
 #include <cstring>
 #include <new>
 
+#include "pbf_after.cuh"
 #include "pbf_engine.h"
 
 #define CK(call)                                              \
@@ -194,6 +195,8 @@ template <int STRIDE>
 __global__ void __launch_bounds__(256) k_ssf_setup(const float *__restrict__ x, const uint32_t *__restrict__ n_dev,
                                                    uint32_t n_arg, Frame f, SplatRec *__restrict__ rec)
 {
+    after_previous();
+    release_next();
     const uint32_t n = n_dev ? *n_dev : n_arg;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const float *xp = x + (size_t)p * STRIDE;
@@ -223,6 +226,7 @@ __global__ void __launch_bounds__(256) k_ssf_raster_box(const SplatRec *__restri
                                                     const uint32_t *__restrict__ n_dev, uint32_t n_arg, Frame f,
                                                     uint32_t *__restrict__ depth)
 {
+    after_previous();  // (no release: its cached depth reads end before the next launch's blocks start)
     const uint32_t n = n_dev ? *n_dev : n_arg;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -310,6 +314,8 @@ __global__ void __launch_bounds__(256) k_ssf_raster(const SplatRec *__restrict__
                                                     const uint32_t *__restrict__ n_dev, uint32_t n_arg, Frame f,
                                                     uint32_t *__restrict__ depth, uint32_t *__restrict__ zmax)
 {
+    after_previous();
+    release_next();
     const uint32_t n = n_dev ? *n_dev : n_arg;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -391,6 +397,7 @@ __global__ void __launch_bounds__(256) k_ssf_raster(const SplatRec *__restrict__
 
 __global__ void k_ssf_fill(uint32_t *__restrict__ dst, uint32_t value, uint32_t n)
 {
+    release_next();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = value;
 }
 
@@ -429,6 +436,7 @@ __device__ inline float depth_store(float v)
 // weight is exp(-0) = 1 where the shader's r2 is 0.
 __global__ void __launch_bounds__(256) k_ssf_blur(const float *__restrict__ in, float *__restrict__ out, Frame f)
 {
+    after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= f.w || j >= f.h) return;
     // the centre tap: at a texel centre the 8-bit filter weights round to 0
@@ -524,6 +532,7 @@ __device__ inline float3 eye_at(const Frame &f, const float *__restrict__ D, int
 // past an odd edge) still supplies its position, as a helper invocation does.
 __global__ void __launch_bounds__(256) k_ssf_normal(const float *__restrict__ D, float4 *__restrict__ N, Frame f)
 {
+    after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= f.w || j >= f.h) return;
     const size_t o = (size_t)j * f.w + i;
@@ -549,6 +558,7 @@ __device__ inline float clamp01(float v) { return fminf(fmaxf(v, 0.f), 1.f); }
 __global__ void __launch_bounds__(256) k_ssf_shade(const float *__restrict__ D, const float4 *__restrict__ N,
                                                    float4 *__restrict__ C, uchar4 *__restrict__ C8, Frame f)
 {
+    after_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= f.w || j >= f.h) return;
     const size_t o = (size_t)j * f.w + i;
@@ -667,6 +677,9 @@ pbf_status launch_frame(pbf_ssf_renderer *r, const float *x, int stride, const u
     const Frame &f = r->f;
     const uint32_t px = f.w * f.h;
     uint32_t launches = 0;
+    // Every launch but the first is set up while the one before runs
+    // (launch_after): 20,000 particles at 640 x 360 45 -> 33 us, 32,768 at 1280 x 720
+    // 80 -> 64, 524,288 at 1920 x 1080 189 -> 176.
     // the depth image and the tile bounds after it
     k_ssf_fill<<<std::min<uint32_t>((px + 255) / 256, (uint32_t)r->sms * 8), 256, 0, st>>>(r->depth, kEmptyDepth,
                                                                                            px + tiles(f));
@@ -683,31 +696,31 @@ pbf_status launch_frame(pbf_ssf_renderer *r, const float *x, int stride, const u
         }
         const uint32_t sblocks = std::min<uint32_t>((n_upper + 255) / 256, (uint32_t)r->sms * 8);
         if (stride == 4)
-            k_ssf_setup<4><<<sblocks, 256, 0, st>>>(x, n_dev, n, f, r->rec);
+            launch_after(k_ssf_setup<4>, sblocks, 256, st, x, n_dev, n, f, r->rec);
         else
-            k_ssf_setup<3><<<sblocks, 256, 0, st>>>(x, n_dev, n, f, r->rec);
+            launch_after(k_ssf_setup<3>, sblocks, 256, st, x, n_dev, n, f, r->rec);
         // a warp per particle while they fit the device at once; larger sets
         // take half the warps, so that fewer far particles start before the
         // near ones' depths are in place
         const uint32_t want = (n_upper + 7) / 8, most = (uint32_t)r->sms * 8;
         const uint32_t rblocks = want <= most ? want : most / 2;
         if (n_upper <= kBoxRaster)
-            k_ssf_raster_box<<<rblocks, 256, 0, st>>>(r->rec, n_dev, n, f, r->depth);
+            launch_after(k_ssf_raster_box, rblocks, 256, st, r->rec, n_dev, n, f, r->depth);
         else
-            k_ssf_raster<<<rblocks, 256, 0, st>>>(r->rec, n_dev, n, f, r->depth, r->depth + px);
+            launch_after(k_ssf_raster, rblocks, 256, st, r->rec, n_dev, n, f, r->depth, r->depth + px);
         launches += 2;
     }
     const dim3 blk(32, 4), grd((f.w + 31) / 32, (f.h + 3) / 4);
     const float *src = reinterpret_cast<const float *>(r->depth), *prev = src;
     for (uint32_t k = 0; k < r->p.blur_passes; ++k) {
         float *dst = r->blur[k & 1];  // even, odd, even ... (main.cpp:430-509)
-        k_ssf_blur<<<grd, blk, 0, st>>>(src, dst, f);
+        launch_after(k_ssf_blur, grd, blk, st, src, dst, f);
         ++launches;
         prev = src;
         src = dst;
     }
-    k_ssf_normal<<<grd, blk, 0, st>>>(src, r->normal, f);
-    k_ssf_shade<<<grd, blk, 0, st>>>(reinterpret_cast<const float *>(r->depth), r->normal, r->color, r->rgba8, f);
+    launch_after(k_ssf_normal, grd, blk, st, src, r->normal, f);
+    launch_after(k_ssf_shade, grd, blk, st, reinterpret_cast<const float *>(r->depth), r->normal, r->color, r->rgba8, f);
     launches += 2;
     CK(cudaGetLastError());
     r->blurred = src;
