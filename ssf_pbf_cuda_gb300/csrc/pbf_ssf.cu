@@ -488,11 +488,14 @@ __global__ void __launch_bounds__(256) k_ssf_blur(const float *__restrict__ in, 
                 }
             }
         };
-        // a tap's coordinate grows with k (each rounding keeps the order), so
-        // the first and the last one tell whether all texels are inside; most
-        // pixels' are, and need no clamps and one address a tap: a frame at
-        // 1600 x 900 110 -> 105 us, at 1920 x 1080 193 -> 188, no change at 1280 x 720
-        if ((at + -4.f * br) * (float)N - 0.5f >= 0.f && (at + 3.f * br) * (float)N - 0.5f < (float)(N - 1u))
+        // with a spacing br of at least 0 a tap's coordinate grows with k (each
+        // rounding keeps the order), so the first and the last one tell whether
+        // all texels are inside; most pixels' are, and need no clamps and one
+        // address a tap: a frame at 1600 x 900 110 -> 105 us, at 1920 x 1080 193 ->
+        // 188, no change at 1280 x 720.  A negative spacing (its sign is the
+        // product's of two parameters) or NaN takes the clamps.
+        if (br >= 0.f && (at + -4.f * br) * (float)N - 0.5f >= 0.f &&
+            (at + 3.f * br) * (float)N - 0.5f < (float)(N - 1u))
             texels(std::true_type());
         else
             texels(std::false_type());
