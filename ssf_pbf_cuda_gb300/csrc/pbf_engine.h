@@ -126,7 +126,7 @@ private:
     pbf_status run(int iters, cudaStream_t st, bool allow_graph, bool packed = false);
     // set the active scenes' counts (or keep them) and stage their pack offsets
     pbf_status stage_counts(const uint32_t *counts, const std::vector<uint32_t> &ids, cudaStream_t st);
-    LaunchShape shape_for(uint32_t tile) const;
+    LaunchShape shape_for(uint32_t tile, bool any_counts = false) const;
     uint32_t post_modes() const;  // kPost* bits of the active scenes
     void rebuild_tiles();
     StepArgs args() const;

@@ -141,8 +141,8 @@ struct LaunchShape {
     uint32_t grid_omega[2], grid_apply[2], grid_xsph[2];  // list-form post passes: u32 lists, u16 lists
     uint32_t grid_cells;  // grid of k_rank_cells: a block of cell_tile threads per cell tile
     uint32_t cell_tile;   // cells per cell tile = threads per k_rank_cells block (autotuned)
-    uint32_t small;       // latency-bound step (at most kSmallStep particle slots): walk by shared
-                          // ranges, per-particle rank, wide list reads
+    uint32_t rank_each;   // few particle slots (at most kSmallStep): per-particle rank
+    uint32_t small;       // latency-bound step (as few): walk by shared ranges, wide list reads
     uint32_t front;       // small steps: k_front's rounds of 1024 cells a block, 0 = a kernel per phase
     uint32_t front_cluster; // blocks of its cluster
     uint32_t tile_shift;  // log2 of tile
@@ -154,7 +154,7 @@ struct LaunchShape {
     {
         return tile == o.tile && grid == o.grid && scan_grid == o.scan_grid && scan_rounds == o.scan_rounds && scan_cluster == o.scan_cluster &&
                chunk == o.chunk &&
-               grid_cells == o.grid_cells && cell_tile == o.cell_tile && small == o.small && small_tiles == o.small_tiles && small_split == o.small_split && small_lanes == o.small_lanes && nb_smem == o.nb_smem &&
+               grid_cells == o.grid_cells && cell_tile == o.cell_tile && rank_each == o.rank_each && small == o.small && small_tiles == o.small_tiles && small_split == o.small_split && small_lanes == o.small_lanes && nb_smem == o.nb_smem &&
                front == o.front && front_cluster == o.front_cluster &&
                grid_nb == o.grid_nb && grid_lambda == o.grid_lambda && grid_dp == o.grid_dp &&
                grid_omega[0] == o.grid_omega[0] && grid_omega[1] == o.grid_omega[1] && grid_apply[0] == o.grid_apply[0] &&

@@ -2875,7 +2875,7 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
         }
         k_scatter<<<g, b, 0, st>>>(a);
         PBF_LAUNCHED("k_scatter");
-        if (sh.small) {
+        if (sh.rank_each) {
             k_rank_reorder<<<g, b, 0, st>>>(a);
             PBF_LAUNCHED("k_rank_reorder");
         } else {
