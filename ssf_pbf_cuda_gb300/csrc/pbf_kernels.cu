@@ -1425,7 +1425,7 @@ __global__ void __launch_bounds__(1024) k_front(StepArgs a, uint32_t tile_shift,
     cluster.barrier_wait(std::move(zeroed));
     if (live) slot = atomicAdd(cluster.map_shared_rank(counts + (gk & kMask), gk >> kShift), 1u);
     cluster.sync();
-    const uint32_t all = cluster_scan<R>([&](uint32_t c) { return counts[c & kMask]; }, n_cells,
+    const uint32_t all = cluster_scan<R, true>([&](uint32_t c) { return counts[c & kMask]; }, n_cells,
                                          [&](uint32_t c, uint32_t offset, uint32_t) {
                                              cells[c & kMask] = offset;
                                              a.offsets[c] = offset;

@@ -25,8 +25,11 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
 // the cluster's barrier each block adds the totals before it.
 // count(index) gives a count, out(index, offset, count) is called for every
 // index below n, both by the thread of the block that holds the index; returns
-// the sum of all counts.
-template <uint32_t R, class COUNT, class OUT>
+// the sum of all counts.  A block's shared memory may be written from outside
+// once the block runs, so the totals go out after a barrier of the cluster:
+// the caller's (MET), or one that is arrived at here before the counts are
+// requested and waited for after their warp scans.
+template <uint32_t R, bool MET = false, class COUNT, class OUT>
 __device__ __forceinline__ uint32_t cluster_scan(COUNT &&count, uint32_t n, OUT &&out)
 {
     namespace cg = cooperative_groups;
@@ -34,6 +37,7 @@ __device__ __forceinline__ uint32_t cluster_scan(COUNT &&count, uint32_t n, OUT 
     __shared__ uint32_t ws[R][32], tot[32];
     const uint32_t rank = cluster.block_rank(), blocks = cluster.num_blocks();
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, base = rank * (1024u * R);
+    if (!MET) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     uint32_t v[R], inc[R];
 #pragma unroll
     for (uint32_t k = 0; k < R; ++k) {
@@ -46,6 +50,7 @@ __device__ __forceinline__ uint32_t cluster_scan(COUNT &&count, uint32_t n, OUT 
         if (lane == 31) ws[k][warp] = inc[k];
     }
     __syncthreads();
+    if (!MET) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     if (warp == 0) {  // exclusive prefix of every (round, warp) total, rounds in order
         uint32_t carry = 0;
 #pragma unroll
