@@ -7,7 +7,12 @@ namespace pbf103 {
 
 // First in every kernel launched by launch_after, before any access to memory:
 // waits until the launch before it is complete (its writes are visible from
-// here on, and so, in turn, are those of the launches before that).
+// here on, and so, in turn, are those of the launches before that).  The
+// kernel may be running while the launch before still writes, so what launches
+// of the same call write is read by plain loads, __ldca or __ldcg: __ldg and const
+// __restrict__ say that nobody writes the data while the kernel runs, and such
+// a load may be moved above the wait.  (The caller's own input may be read so:
+// the call's first launch starts when it is complete.)
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Lets the launch after this one be set up once every block of this one has

@@ -33,3 +33,29 @@ def test_cluster_scan_meets_before_it_writes_other_blocks():
         for m in re.finditer(r"cluster_scan<R, true>", src):
             kernel = src[src.rindex("__global__", 0, m.start()):m.start()]
             assert "cluster.sync()" in kernel or "barrier_wait" in kernel
+
+
+def test_kernels_set_up_early_read_plainly_what_launches_before_them_write():
+    """__ldg and const __restrict__ promise data that nobody writes while the
+    kernel runs; a kernel that waits in after_previous runs while the launch
+    before it writes.  The caller's own input may be read so."""
+    inputs = {"x", "n_dev", "xp"}
+    seen = 0
+    for name in ("pbf_ssf.cu", "pbf_noalloc.cu"):
+        src = _source(name)
+        helpers = {m.group(1): m for m in re.finditer(r"__device__ [^;{}]*?\b(\w+)\(([^{};]*)\)\s*\{", src)}
+        for m in re.finditer(r"__global__[^;{}]*?\b(\w+)\((?=[^()]*\b[A-Z]\w*\b|[^()]*\*)([^{};]*)\)\s*\{", src):
+            body = _body(src, m.end() - 1)
+            if "after_previous" not in body:
+                continue
+            seen += 1
+            parts = [(m.group(2), body)]
+            for h, hm in helpers.items():
+                if re.search(r"\b%s\(" % h, body):
+                    parts.append((hm.group(2), _body(src, hm.end() - 1)))
+            for args, text in parts:
+                for q in re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", args):
+                    assert q in inputs, (name, m.group(1), q)
+                for q in re.findall(r"__ldg\(\s*(\w+)", text):
+                    assert q in inputs, (name, m.group(1), q)
+    assert seen >= 10  # set-up, two rasters, blur, normal, shade; scan, scatter, rank, big
