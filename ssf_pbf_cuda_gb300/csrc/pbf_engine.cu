@@ -1067,7 +1067,9 @@ pbf_status Batch::get_num(uint32_t id, uint32_t *num, cudaStream_t st)
 // the copy (all before it is done, the copy itself may be in flight) and
 // takes over the count.  The copy is enqueued before the wait, bounded by the
 // host's upper bound and by the count on the device, and its first block
-// writes the count to pinned memory, which the host polls.  A 4-byte copy to
+// writes the count to pinned memory, which the host polls by acquire loads (so
+// that its later reads of pinned memory see what earlier work of the stream
+// wrote there, as after a wait for the stream).  A 4-byte copy to
 // the host, its wait and only then the launch left the GPU idle meanwhile:
 // set, step and get of 4,096 particles 97 us so, 87 us now (91 with a stream
 // synchronisation in place of the poll); 32,768 particles 122 and 108.
@@ -1077,16 +1079,17 @@ pbf_status Batch::store_device(uint32_t id, float *x, float *v, uint32_t *num, c
     CK(cudaSetDevice(device_));
     SceneHost &s = scenes_[id];
     uint32_t n = 0;
-    volatile uint32_t *slot = h_small_ + 2ull * max_scenes_ + id;
+    uint32_t *slot = h_small_ + 2ull * max_scenes_ + id;
     if (s.num_upper) {
         constexpr uint32_t kUnset = 0xFFFFFFFFu;  // no count: capacities lie below
         *slot = kUnset;
         launch_store_phase(d_x_ + s.desc.p_off, d_v_ + s.desc.p_off, x, v, s.num_upper, st, d_scene_num_ + id, slot);
         CK(cudaGetLastError());
+        auto count = [&] { return n = __atomic_load_n(slot, __ATOMIC_ACQUIRE); };
         uint32_t polls = 0;
-        while ((n = *slot) == kUnset)
+        while (count() == kUnset)
             if ((++polls & 1023u) == 0 && cudaStreamQuery(st) != cudaErrorNotReady) break;
-        if (n != kUnset || (n = *slot) != kUnset) {
+        if (n != kUnset || count() != kUnset) {
             if (n != s.num_upper) {
                 s.num_upper = n;
                 dirty_tiles_ = true;

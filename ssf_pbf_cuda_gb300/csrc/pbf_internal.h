@@ -202,7 +202,7 @@ void launch_aos3_to_f4(const float *src, float4 *dst, uint32_t n, cudaStream_t s
 void launch_load_phase(const float *sx, const float *sv, float4 *x, float4 *v, uint32_t *id, uint32_t *next_id,
                        uint32_t *scene_num, uint32_t n, uint32_t total, bool append, cudaStream_t st);
 void launch_store_phase(const float4 *x, const float4 *v, float *dx, float *dv, uint32_t n, cudaStream_t st,
-                        const uint32_t *num = nullptr, volatile uint32_t *num_out = nullptr);
+                        const uint32_t *num = nullptr, uint32_t *num_out = nullptr);
 void launch_set_u32(uint32_t *dst, uint32_t value, cudaStream_t st);
 // pack_off[active[k]] = sum of the live counts of active[0..k), counts[k] =
 // the live count of active[k], computed on the device (one block)

@@ -59,3 +59,12 @@ def test_kernels_set_up_early_read_plainly_what_launches_before_them_write():
                 for q in re.findall(r"__ldg\(\s*(\w+)", text):
                     assert q in inputs, (name, m.group(1), q)
     assert seen >= 10  # set-up, two rasters, blur, normal, shade; scan, scatter, rank, big
+
+
+def test_the_polled_count_is_a_release_read_by_acquire():
+    engine, kernels = _source("pbf_engine.cu"), _source("pbf_kernels.cu")
+    body = _body(engine, engine.index("Batch::store_device"))
+    assert "volatile" not in body and "__atomic_load_n(slot, __ATOMIC_ACQUIRE)" in body
+    assert not re.search(r"=\s*\*slot|\*slot\s*[!=]=", body)
+    body = _body(kernels, kernels.index("void k_store_phase"))
+    assert 0 <= body.find("fence.acq_rel.sys") < body.find("st.relaxed.sys")
