@@ -167,19 +167,25 @@ __device__ inline float splat_fragment(const Frame &f, const Splat &s, int i, in
     return fminf(fmaxf(d, 0.f), 1.f) + 0.f;  // clamped to the depth range; + 0 turns -0 into +0
 }
 
-// Early depth rejection, exact: no fragment of the particle is nearer than
-// its front point (nz = 1) by more than the rounding of the depth formula,
-// so a pixel already holding a depth at or below the bound keeps it.
+// Early depth rejection, exact: a fragment's view z lies between the centre's
+// and the front point's (nz = 0 .. 1), and the depth formula is monotone there
+// unless its denominator changes sign, so no fragment is nearer than the nearer
+// of the two by more than the formula's rounding: a pixel already holding a
+// depth at or below the bound keeps it.  A sphere that reaches past the eye
+// plane has fragments at any depth: bound 0.
+__device__ inline float depth_bound(const Frame &f, float pz)
+{
+    const float num = f.proj[10] * pz + f.proj[14], den = f.proj[11] * pz + f.proj[15];
+    if (!(den > 0.f)) return 0.f;
+    // |float - exact| <= 2^-22 (|P22 pz| + |P32|) / den + ulp / 2; four times that
+    return num / den - 4.f * (2.3841858e-7f * (fabsf(f.proj[10] * pz) + fabsf(f.proj[14])) / den + 6e-8f);
+}
+
 __device__ inline uint32_t front_bound(const Frame &f, float ez)
 {
-    const float pz = ez + f.radius;
-    const float num = f.proj[10] * pz + f.proj[14], den = f.proj[11] * pz + f.proj[15];
-    const float d = num / den;
-    // |float - exact| <= 2^-22 (|P22 pz| + |P32|) / |den| + ulp / 2; four times that
-    const float err = 4.f * (2.3841858e-7f * (fabsf(f.proj[10] * pz) + fabsf(f.proj[14])) / fabsf(den) + 6e-8f);
-    const float b = d - err;
-    if (!(b > 0.f)) return 0u;  // also NaN
-    return __float_as_uint(fminf(b, 1.f));
+    const float b0 = depth_bound(f, ez), b1 = depth_bound(f, ez + f.radius);
+    if (!(b0 > 0.f && b1 > 0.f)) return 0u;  // also NaN
+    return __float_as_uint(fminf(fminf(b0, b1), 1.f));
 }
 
 // A particle's splat as the raster kernel reads it (32 B): (x0, y0, rx, ry)
