@@ -192,10 +192,18 @@ private:
             return iters == o.iters && modes == o.modes && shape == o.shape;
         }
     };
-    // one captured step per input form: [0] the phase, [1] packed input
-    cudaGraphExec_t exec_[2] = {nullptr, nullptr};
-    GraphKey key_[2];
-    uint32_t graph_launches_[2] = {0, 0};
+    // The last few captured steps of each input form, [0] the phase, [1] packed
+    // input: a batch whose scenes come and go passes back and forth over the
+    // sizes and neighbour counts at which launch shapes change (see run()).
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        GraphKey key;
+        uint32_t launches = 0;
+        uint64_t used = 0;  // when it was last launched
+    };
+    static constexpr int kStepGraphs = 4;
+    StepGraph graphs_[2][kStepGraphs];
+    uint64_t graph_use_ = 0;
     uint32_t last_launches_ = 0;
     PackedIn *d_pin_ = nullptr;  // input buffers of the current packed-input step
 };
