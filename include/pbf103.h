@@ -265,11 +265,13 @@ pbf_status pbf_batch_get_all_async(pbf_batch *b, uint32_t *counts_dev, float *x_
 pbf_status pbf_batch_autotune(pbf_batch *b, int iters, void *stream, uint32_t *chosen_tile);
 pbf_status pbf_batch_set_tile(pbf_batch *b, uint32_t tile);
 /* Neighbour indices requested ahead per thread in the lambda passes of large
- * steps (4 or 8; the autotuner also picks it; scenes that expect at most 16
- * neighbours a particle always use 4).  Results do not depend on it.
- * No reference counterpart. */
+ * steps (4 or 8; the autotuner also picks it).  Used when some scene of the
+ * batch expects more than 16 neighbours a particle within h at rest density;
+ * a batch of shorter lists alone is stepped with 4 whatever is set here, and
+ * the autotuner leaves the setting.  Results do not depend on it.  No
+ * reference counterpart. */
 pbf_status pbf_batch_set_chunk(pbf_batch *b, uint32_t chunk);
-/* Current tile (particles per block) and chunk. */
+/* Current tile (particles per block) and chunk, as set or tuned. */
 pbf_status pbf_batch_get_launch_shape(pbf_batch *b, uint32_t *tile, uint32_t *chunk);
 /* Cells per CTA of the per-cell stable rank of large steps (64, 128, 256 or
  * 512; the autotuner also picks it).  Results do not depend on it.  No

@@ -581,7 +581,8 @@ class Batch:
         check(load().pbf_batch_set_tile(self.handle, int(tile)), "pbf_batch_set_tile")
 
     def set_chunk(self, chunk: int):
-        """Neighbour indices requested ahead per thread in large steps' lambda passes (4 or 8)."""
+        """Neighbour indices requested ahead per thread in large steps' lambda passes (4 or 8; a batch whose scenes
+        all expect at most 16 neighbours a particle is stepped with 4)."""
         check(load().pbf_batch_set_chunk(self.handle, int(chunk)), "pbf_batch_set_chunk")
 
     def set_cell_tile(self, cells: int):

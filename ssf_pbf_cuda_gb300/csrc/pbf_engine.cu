@@ -1310,15 +1310,18 @@ pbf_status Batch::autotune(int iters, cudaStream_t st, uint32_t *chosen)
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     const uint32_t cands[] = {128, 256, 512, 64};
-    const uint32_t chunks[] = {8, 4};
+    const uint32_t set_chunk = chunk_, chunks[] = {set_chunk, 12u - set_chunk};
     uint32_t best = tile_, best_chunk = chunk_;
     float best_ms = 1e30f;
     for (uint32_t t : cands)
     for (uint32_t ch : chunks) {
         set_tile(t);
-        chunk_ = ch;
+        chunk_ = set_chunk;
         rc = upload(st);
         if (rc != PBF_SUCCESS) break;
+        // small steps, and batches of short lists, run the same for either chunk
+        if (ch != set_chunk && (!long_lists_ || shape_for(t).small)) continue;
+        chunk_ = ch;
         for (int r = 0; r < 2; ++r) run(iters, st, false);  // warm-up
         CK(cudaEventRecord(e0, st));
         for (int r = 0; r < 8; ++r) run(iters, st, false);
