@@ -284,7 +284,14 @@ pbf_status pbf_batch_last_launches(pbf_batch *b, uint32_t *launches);
 pbf_status pbf_last_launches(pbf_handle *h, uint32_t *launches);
 /* Advance one step without a CUDA graph, timing every kernel with CUDA
  * events on the stream: ms[k] and names[64 * k] (NUL-terminated) for the
- * k-th launch, at most max entries, *n written. */
+ * k-th launch, at most max entries, *n written.  The names are the phases':
+ * k_scan_single is the scan in one launch (of a block or a cluster),
+ * k_neighbors_split a small step's walk (one or four lanes a particle), k_dp
+ * and the other passes either step size's kernel.  The smallest steps (up to
+ * 16,384 particle slots) run everything before the walk as one kernel; a
+ * profile times these phases as kernels of their own, with the same results,
+ * so its launches are more than pbf_last_launches gives after a step and the
+ * sum of its times more than the step's. */
 pbf_status pbf_batch_profile_step(pbf_batch *b, int iters, void *stream, float *ms, char *names, uint32_t max,
                                   uint32_t *n);
 pbf_status pbf_profile_step(pbf_handle *h, const pbf_boundary_t *boundary, const float area_min[3],

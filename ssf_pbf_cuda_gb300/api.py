@@ -381,8 +381,9 @@ def one_step(simulatee: PbfParticle, boundary: Boundary | None, simulation_area,
 
 def profile_step(simulatee: PbfParticle, boundary: Boundary | None, simulation_area, num_solver_iteration: int,
                  stream=None) -> list:
-    """one_step without a CUDA graph, timing each kernel with CUDA events:
-    returns [(kernel name, milliseconds)] in launch order."""
+    """one_step without a CUDA graph, timing each phase's kernel with CUDA
+    events: returns [(name, milliseconds)] in launch order.  The smallest
+    steps run the phases before the neighbour walk as one kernel otherwise."""
     amin, amax = simulation_area
     names = (ctypes.c_char * (64 * 64))()
     ms = (ctypes.c_float * 64)()
@@ -561,8 +562,9 @@ class Batch:
                                              _stream(stream)), "pbf_batch_get_all_async")
 
     def profile_step(self, iters: int, stream=None) -> list:
-        """One step without a graph, with CUDA events between kernels; returns
-        [(kernel name, milliseconds)] in launch order."""
+        """One step without a graph, with CUDA events between the phases'
+        kernels; returns [(name, milliseconds)] in launch order (see
+        profile_step)."""
         names = (ctypes.c_char * (64 * 64))()
         ms = (ctypes.c_float * 64)()
         n = ctypes.c_uint32()

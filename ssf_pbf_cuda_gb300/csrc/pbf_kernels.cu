@@ -2902,7 +2902,7 @@ uint32_t enqueue_step(const StepArgs &a, const LaunchShape &sh, int iters, uint3
             k_neighbors_split<<<gs, kSplitBlock, sh.nb_smem, st>>>(a, sh.tile);
         else
             k_neighbors_small<<<gs, kSmallBlock, sh.nb_smem, st>>>(a, sh.tile);
-        PBF_LAUNCHED("k_neighbors_split");
+        PBF_LAUNCHED("k_neighbors_split");  // the profile's name for a small step's walk
     } else {
         if (sh.nb_smem)
             k_neighbors_lambda<true><<<sh.grid_nb, b, sh.nb_smem, st>>>(a);
