@@ -361,19 +361,18 @@ __device__ __forceinline__ void walk27_ranges(const SceneDesc &d, const uint32_t
 // reference visits wrapped cells twice) are visited whole, in sorted order.
 // r(st, en) gets the range of working slots.
 //
-// PRUNE restricts the walk to cells that can hold a particle within h of xp
+// The walk is restricted to cells that can hold a particle within h of xp
 // (the binned position): a cell whose nearest point is farther than h holds
 // no accepted candidate, so skipping it leaves the visited sequence of
 // accepted candidates unchanged.  A 1e-3 relative margin covers the rounding
 // of the cell assignment.  It applies only when every axis has at least 4
 // cells (with fewer, the reference visits wrapped cells more than once).
-template <bool PRUNE, class R>
+template <class R>
 __device__ __forceinline__ void walk27_cells(const SceneDesc &d, const uint32_t *__restrict__ offsets,
-                                             const uint64_t *__restrict__ chist, uint32_t shift, float4 xp, R &&r,
-                                             int rr0 = 0, int rr1 = 9)
+                                             const uint64_t *__restrict__ chist, uint32_t shift, float4 xp, R &&r)
 {
     const int32_t icx = cell_coord(xp.x, d.cw), icy = cell_coord(xp.y, d.cw), icz = cell_coord(xp.z, d.cw);
-    const bool prune = PRUNE && d.gx >= 4 && d.gy >= 4 && d.gz >= 4;
+    const bool prune = d.gx >= 4 && d.gy >= 4 && d.gz >= 4;
     float lx = 0.f, ly = 0.f, lz = 0.f, rx = 0.f, ry = 0.f, rz = 0.f;
     if (prune) {
         lx = xp.x - (float)icx * d.cw;
@@ -395,7 +394,7 @@ __device__ __forceinline__ void walk27_cells(const SceneDesc &d, const uint32_t 
     // byte selections instead of counts and a byte sum, 1,405 -> 1,376.
     bool go = true;
 #pragma unroll 1
-    for (int rr = rr0; rr < rr1 && go; ++rr) {  // rows (dz, dy), z outermost: the reference's walk order
+    for (int rr = 0; rr < 9 && go; ++rr) {  // rows (dz, dy), z outermost: the reference's walk order
         const int dz = rr / 3 - 1, dy = rr % 3 - 1;
         bool mid = true, left = true, right = true;
         if (prune) {
@@ -1518,7 +1517,7 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
     // carries no extra state; otherwise the walk skips it as it stores.
     constexpr uint32_t kNbFetch = 4;
     uint32_t cnt = 0, selfat = kNotListed;
-    walk27_cells<true>(d, a.offsets, a.chist, shift, xp, [&](uint32_t st, uint32_t en) -> bool {
+    walk27_cells(d, a.offsets, a.chist, shift, xp, [&](uint32_t st, uint32_t en) -> bool {
         for (uint32_t q0 = st; q0 < en; q0 += kNbFetch) {
             float4 c[kNbFetch];
             const float4 *pq = xa + q0;
