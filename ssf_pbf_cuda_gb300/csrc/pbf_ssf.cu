@@ -678,6 +678,14 @@ void cross3(const float a[3], const float b[3], float out[3])
     out[2] = a[0] * b[1] - b[0] * a[1];
 }
 
+// Pixels between which the screen passes' blocks take 32 x 8 pixels, not
+// 32 x 4: mostly empty frames are bound by their blocks' start, covered ones by
+// the pixels' arithmetic.  A frame of one particle and of 32,768 in us, by 4
+// rows and by 8: 1280 x 720 35 and 64, 33 and 64; 1600 x 900 45 and 81, 39 and
+// 81; 1920 x 1080 58 and 105, 48 and 104; 3840 x 2160 197 and 341, 170 and 332;
+// 4096 x 2400 229 and 399, 202 and 393; 5120 x 2880 353 and 604, 350 and 615.
+constexpr uint32_t kTallFrom = 1500000, kTallTo = 10000000;
+
 // 8 x 4 pixel tiles of the image (their depth bounds follow the depth image)
 inline uint32_t tiles(const Frame &f) { return ((f.w + 7u) / 8u) * ((f.h + 3u) / 4u); }
 
@@ -721,7 +729,8 @@ pbf_status launch_frame(pbf_ssf_renderer *r, const float *x, int stride, const u
             launch_after(k_ssf_raster, rblocks, 256, st, r->rec, n_dev, n, f, r->depth, r->depth + px);
         launches += 2;
     }
-    const dim3 blk(32, 4), grd((f.w + 31) / 32, (f.h + 3) / 4);
+    const uint32_t rows = px >= kTallFrom && px <= kTallTo ? 8u : 4u;
+    const dim3 blk(32, rows), grd((f.w + 31) / 32, (f.h + rows - 1) / rows);
     const float *src = reinterpret_cast<const float *>(r->depth), *prev = src;
     for (uint32_t k = 0; k < r->p.blur_passes; ++k) {
         float *dst = r->blur[k & 1];  // even, odd, even ... (main.cpp:430-509)
