@@ -225,6 +225,14 @@ __global__ void __launch_bounds__(256) k_ssf_setup(const float *__restrict__ x, 
 // by boxes and by tiles: 12,000 particles at 640 x 360 49.5 and 51.6 us, 20,000 at
 // 1280 x 720 75.1 and 75.4, 32,768 82.2 and 80.1, 100,000 at 1001 x 563 96 and 83.
 constexpr uint32_t kBoxRaster = 20000;
+// Small images are drawn by boxes too: their depths stay in L1, which the box
+// raster reads through, where tiles go to L2 for theirs (96 KB at the larger
+// bound, which very many particles, less often near the front, do not gain
+// from).  Frames by tiles and by boxes, 60,000 and 200,000 particles near the
+// eye: 64 x 36 80 -> 35 and 177 -> 61 us, 128 x 72 60 -> 39 and 148 -> 66, 192 x 108
+// 71 -> 46 and 128 -> 80, 320 x 180 78 -> 72 and 123 -> 133; 1,000,000 before the
+// camera: 128 x 72 260 -> 209, 192 x 108 178 -> 210.
+constexpr uint32_t kBoxPixels = 16384, kBoxPixelsFew = 24576, kBoxFew = 262144;
 
 // One warp per particle, lanes over its pixel box (stepped without
 // division): every pixel tests its own depth alone.
@@ -719,14 +727,14 @@ pbf_status launch_frame(pbf_ssf_renderer *r, const float *x, int stride, const u
         else
             launch_after(k_ssf_setup<3>, sblocks, 256, st, x, n_dev, n, f, r->rec);
         // a warp per particle while they fit the device at once; larger sets
-        // take half the warps, so that fewer far particles start before the
-        // near ones' depths are in place
+        // by tiles take half the warps, so that fewer far particles start
+        // before the near ones' depths are in place
         const uint32_t want = (n_upper + 7) / 8, most = (uint32_t)r->sms * 8;
-        const uint32_t rblocks = want <= most ? want : most / 2;
-        if (n_upper <= kBoxRaster)
-            launch_after(k_ssf_raster_box, rblocks, 256, st, r->rec, n_dev, n, f, r->depth);
+        if (n_upper <= kBoxRaster || px <= kBoxPixels || (px <= kBoxPixelsFew && n_upper <= kBoxFew))
+            launch_after(k_ssf_raster_box, std::min(want, most), 256, st, r->rec, n_dev, n, f, r->depth);
         else
-            launch_after(k_ssf_raster, rblocks, 256, st, r->rec, n_dev, n, f, r->depth, r->depth + px);
+            launch_after(k_ssf_raster, want <= most ? want : most / 2, 256, st, r->rec, n_dev, n, f, r->depth,
+                         r->depth + px);
         launches += 2;
     }
     const uint32_t rows = px >= kTallFrom && px <= kTallTo ? 8u : 4u;
