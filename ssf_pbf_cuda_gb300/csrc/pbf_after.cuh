@@ -19,9 +19,9 @@ __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.
 // come here (otherwise once every block is done); its blocks wait in
 // after_previous themselves.  After after_previous, but for a call's first
 // kernel, which is launched as usual.  Not for grids of several waves: the
-// waiting blocks take their places (a frame of 524,288
-// particles at 1920 x 1080 184 us without it in the blurs and normals, 199 with,
-// 189 by plain launches).
+// waiting blocks take their places (a frame of 32,768 particles at 1600 x 900
+// 81 us without it in the blurs and normals, 91 with, 94 by plain launches; at
+// 1280 x 720 63, 70 and 79).
 __device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Launches fn, whose first act is after_previous().  The next launch that is

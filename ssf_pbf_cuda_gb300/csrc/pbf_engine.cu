@@ -826,9 +826,9 @@ LaunchShape Batch::shape_for(uint32_t tile, bool any_counts) const
         sh.scan_cluster = lim;
         sh.scan_rounds = r;
     }
-    // everything before the walk in one cluster, a particle a thread (16,384
-    // slots: 84 against 88 us for 4,096 particles; more would need two a thread,
-    // which loses)
+    // everything before the walk in one cluster, a particle a thread (up to
+    // 16,384 slots: set, step and get of 4,096 particles 74 us against 79, of
+    // 16,384 84 against 86; more would need two a thread, which loses)
     sh.front = sh.front_cluster = 0;
     sh.tile_shift = 0;
     while ((1u << sh.tile_shift) < tile) ++sh.tile_shift;
@@ -922,7 +922,7 @@ pbf_status Batch::run(int iters, cudaStream_t st, bool allow_graph, bool packed)
         k.shape = sh;
         // the graph of this shape, else the place of the one not used for longest.
         // One graph alone was captured anew whenever the shape changed: two
-        // scene sets in turn, of 20,000 and 30,000 particles, 384 us for the
+        // scene sets in turn, of 20,000 and 30,000 particles, 378 us for the
         // pair of steps, 239 so.
         StepGraph *g0 = graphs_[f];
         for (StepGraph &c : graphs_[f]) {

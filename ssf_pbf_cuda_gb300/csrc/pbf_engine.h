@@ -159,7 +159,7 @@ private:
     uint32_t *d_id_ = nullptr, *d_id_tmp_ = nullptr;  // particle ids, phase order / sorted scratch
     uint32_t *d_next_id_ = nullptr;                   // per scene: next id to hand out
     uint8_t *d_cls_ = nullptr;                        // alias class per particle (input order)
-    uint64_t *d_chist_ = nullptr;                     // per cell: class counts of its bucket
+    uint64_t *d_chist_ = nullptr;                     // per cell: class ends of its bucket
     uint32_t *d_wpos_ = nullptr;                      // sorted slot -> working slot
     uint32_t *d_dense_ = nullptr;                     // dense-bucket queue
     uint32_t *d_mid_ = nullptr;                       // medium-bucket queue

@@ -1372,11 +1372,12 @@ __global__ void __launch_bounds__(kSmallBlock) k_gather_small(StepArgs a, uint32
 // cluster of 1024-thread blocks, a particle a thread, R rounds of 1024 cells a
 // block.  Sorted and working orders are the separate kernels'.
 //
-// Bound by latency: four cluster barriers (850 cycles each with nothing to
-// drain, 1,500 with stores) and the loads between them, 12,000 cycles in all,
-// against six launches and the reload in each of what the phase before knew:
-// set, step and get of 4,096 particles 87 -> 82 us, of 10,648 at h = 1.4
-// spacings 67 -> 62.  A particle keeps its prediction, bucket and slot in
+// Bound by latency: five cluster barriers (counts cleared, counted, block
+// totals, offsets, scattered; 850 cycles each with nothing to drain, 1,500 with
+// stores; a sixth where buckets are dense) and the loads between them, 12,000
+// cycles in all, against six launches and the reload in each of what the phase
+// before knew: set, step and get of 4,096 particles 79 -> 74 us, of 10,000 at
+// h = 1.4 spacings 68 -> 63.  A particle keeps its prediction, bucket and slot in
 // registers through the phases and writes its records into its working slot
 // itself; counts and offsets are the blocks' shared memory.  Two particles a
 // thread took 32,768 particles' step from 88.2 to 90.1 us, so such steps keep

@@ -705,8 +705,8 @@ pbf_status launch_frame(pbf_ssf_renderer *r, const float *x, int stride, const u
     const uint32_t px = f.w * f.h;
     uint32_t launches = 0;
     // Every launch but the first is set up while the one before runs
-    // (launch_after): 20,000 particles at 640 x 360 45 -> 33 us, 32,768 at 1280 x 720
-    // 80 -> 64, 524,288 at 1920 x 1080 189 -> 176.
+    // (launch_after): 20,000 particles at 640 x 360 45 -> 31 us, 32,768 at 1280 x 720
+    // 79 -> 63, 524,288 at 1920 x 1080 188 -> 175.
     // the depth image and the tile bounds after it
     k_ssf_fill<<<std::min<uint32_t>((px + 255) / 256, (uint32_t)r->sms * 8), 256, 0, st>>>(r->depth, kEmptyDepth,
                                                                                            px + tiles(f));
