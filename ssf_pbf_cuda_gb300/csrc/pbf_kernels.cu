@@ -1535,9 +1535,23 @@ __global__ void __launch_bounds__(512, 2) k_neighbors_lambda(StepArgs a)
                         s_list[cnt * blockDim.x + threadIdx.x] = q;
                     } else {
                         const uint32_t ks = cnt - (selfat < cnt ? 1u : 0u);  // stored entries before this one
-                        if (q == i)
+                        if (q == i) {
+                            // met again (an axis of one cell is visited three times): the last
+                            // place is the one left out, so the earlier one is stored after all
+                            if (selfat != kNotListed) {
+                                for (uint32_t e = ks; e > selfat; --e) {
+                                    if (l16)
+                                        nl16[list16_slot(e, stride)] = nl16[list16_slot(e - 1u, stride)];
+                                    else
+                                        nl[list_slot(e, stride)] = nl[list_slot(e - 1u, stride)];
+                                }
+                                if (l16)
+                                    nl16[list16_slot(selfat, stride)] = (uint16_t)(i - d.p_off);
+                                else
+                                    nl[list_slot(selfat, stride)] = i;
+                            }
                             selfat = cnt;
-                        else if (l16)
+                        } else if (l16)
                             nl16[list16_slot(ks, stride)] = (uint16_t)(q - d.p_off);
                         else
                             nl[list_slot(ks, stride)] = q;
