@@ -278,6 +278,10 @@ pbf_status pbf_batch_get_launch_shape(pbf_batch *b, uint32_t *tile, uint32_t *ch
  * reference counterpart. */
 pbf_status pbf_batch_set_cell_tile(pbf_batch *b, uint32_t cells);
 pbf_status pbf_batch_get_cell_tile(pbf_batch *b, uint32_t *cells);
+/* Steps as CUDA graphs of the library's own (the default) or as launches on
+ * the stream.  With launches a step may be recorded in a caller's graph (after
+ * one step, so that nothing is left to upload): a replay steps whatever
+ * particles the batch holds then, as long as its set of scenes stays. */
 pbf_status pbf_batch_set_graph_mode(pbf_batch *b, int enable);
 /* Kernels launched by the last pbf_batch_step / pbf_one_step call. */
 pbf_status pbf_batch_last_launches(pbf_batch *b, uint32_t *launches);
