@@ -1288,21 +1288,28 @@ pbf_status Batch::autotune(int iters, cudaStream_t st, uint32_t *chosen)
     }
     const uint64_t hw = palloc_.high_water();
     float4 *sx = nullptr, *sv = nullptr;
-    uint32_t *sn = nullptr, *sf = nullptr;
+    uint32_t *sn = nullptr, *sf = nullptr, *si = nullptr, *sp = nullptr;
     CK(cudaMalloc(&sx, 16 * std::max<uint64_t>(hw, 1)));
     CK(cudaMalloc(&sv, 16 * std::max<uint64_t>(hw, 1)));
     CK(cudaMalloc(&sn, 4ull * max_scenes_));
     CK(cudaMalloc(&sf, 4ull * max_scenes_));
+    // ids follow the particles, and the last step's permutation serves restore_order
+    CK(cudaMalloc(&si, 4 * std::max<uint64_t>(hw, 1)));
+    CK(cudaMalloc(&sp, 4 * std::max<uint64_t>(hw, 1)));
     auto save = [&]() -> cudaError_t {
         cudaMemcpyAsync(sx, d_x_, 16 * hw, cudaMemcpyDeviceToDevice, st);
         cudaMemcpyAsync(sv, d_v_, 16 * hw, cudaMemcpyDeviceToDevice, st);
         cudaMemcpyAsync(sn, d_scene_num_, 4ull * max_scenes_, cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(si, d_id_, 4 * hw, cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(sp, d_perm_, 4 * hw, cudaMemcpyDeviceToDevice, st);
         return cudaMemcpyAsync(sf, d_flags_, 4ull * max_scenes_, cudaMemcpyDeviceToDevice, st);
     };
     auto restore = [&]() -> cudaError_t {
         cudaMemcpyAsync(d_x_, sx, 16 * hw, cudaMemcpyDeviceToDevice, st);
         cudaMemcpyAsync(d_v_, sv, 16 * hw, cudaMemcpyDeviceToDevice, st);
         cudaMemcpyAsync(d_scene_num_, sn, 4ull * max_scenes_, cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(d_id_, si, 4 * hw, cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(d_perm_, sp, 4 * hw, cudaMemcpyDeviceToDevice, st);
         return cudaMemcpyAsync(d_flags_, sf, 4ull * max_scenes_, cudaMemcpyDeviceToDevice, st);
     };
     CK(save());
@@ -1369,6 +1376,8 @@ pbf_status Batch::autotune(int iters, cudaStream_t st, uint32_t *chosen)
     cudaFree(sv);
     cudaFree(sn);
     cudaFree(sf);
+    cudaFree(si);
+    cudaFree(sp);
     if (chosen) *chosen = best;
     return rc;
 }
